@@ -7,13 +7,11 @@
 // `idbits` = ceil(log2 n) bits carry order.
 //
 //   slice <= kTinyCap ids   one warp bucket-sorts it in shared memory (256
-//                           buckets, a few ids each, insertion-sorted);
-//   slice <= kSmallCap ids  one CTA bucket-sorts it in shared memory: ids
-//                           are counted into 2048 buckets by their top bits
-//                           (the atomic's return value is the id's slot in
-//                           its bucket), a block scan gives bucket bases,
-//                           each bucket (a few ids) is insertion-sorted and
-//                           the order leaves in coalesced stores.
+//                           buckets over the slice's own id range, a few ids
+//                           each, insertion-sorted);
+//   slice <= kSmallCap ids  one CTA bucket-sorts it the same way (2048
+//                           buckets).  In both, a slice whose ids crowd into
+//                           few buckets is radix-sorted instead.
 //   larger slices           1. window partition: ids are split by
 //                              id >> wbits (wbits = min(idbits, 18)) into
 //                              G = 2^(idbits - wbits) windows: tile
@@ -83,55 +81,136 @@ using Job = SortJob;
 // ============================================================================
 // Small slices: bucket sort
 // ============================================================================
+// Ids are often not spread over [0, n): objects loaded region by region give
+// a box a few short id ranges.  Buckets over all of [0, n) then hold hundreds
+// of ids each and their insertion sorts dominate (5,000 boxes over 2,000,003
+// points in 64 id-contiguous clusters: k_sort_small 21.5 ms, k_sort_tiny 2.7
+// ms, k_win_sort_warp 1.3 ms).  So a slice with a bucket of more than
+// kCrowded ids is counted again into buckets over its own range [min, max],
+// and one that is crowded all the same (several ranges far apart) takes
+// stable 8-bit radix passes over the bits of max - min.  kCrowded: a bucket
+// of 32 ids costs its lane about 256 insertion steps, what three radix passes
+// cost the warp.  The batch above: 29.3 -> 2.9 ms (0.18, 0.10 and 0.05 ms in
+// the three kernels).
+constexpr uint32_t kCrowded = 32;
 struct BucketSmem {
   uint32_t stage[kSmallCap];
-  uint32_t cnt[kBuckets];
-  uint32_t base[kBuckets];
-  uint16_t slot[kSmallCap];
-  uint32_t wtot[kSmallWarps];
+  uint32_t cnt[kBuckets];   // bucket counts, then next slots; radix: [warp][digit]
+  uint32_t red[3 * kSmallWarps];
 };
 
 // Slices of at most kTinyCap ids, one warp each (no CTA barriers): the ids
 // are loaded into registers (32 per lane, all loads in flight together) and
-// counted into kTinyBuckets buckets by their top bits, a warp scan gives the
-// bucket bases, every id takes the next slot of its bucket, each lane insertion-sorts its 8 buckets (a few ids each) and the
-// slice leaves in coalesced stores.  Jobs of more ids are k_sort_small's.
+// counted into kTinyBuckets buckets, a warp scan gives the bucket bases,
+// every id takes the next slot of its bucket, each lane insertion-sorts its 8
+// buckets (a few ids each) and the slice leaves in coalesced stores.  Jobs of
+// more ids are k_sort_small's.
+// CTAs per SM (registers and shared memory): 4 for slices (3 cost their sort
+// a second wave: 356 -> 540 us on 100,000 slices of 640 ids), 6 for windows.
+constexpr uint32_t kTinyBlocks = 4;
+constexpr uint32_t kWinWarpBlocks = 6;
+template <uint32_t CAP>
 struct TinySmem {
-  uint32_t stage[kTinyWarps][kTinyCap];
+  uint32_t stage[kTinyWarps][CAP];
   uint32_t cnt[kTinyWarps][kTinyBuckets];
   uint32_t base[kTinyWarps][kTinyBuckets];
 };
 
-// One warp sorts the size <= CAP (<= kTinyCap) distinct ids at src into dst
-// (src may equal dst): buckets by (id - lo) >> bshift (every id's bucket
-// below kTinyBuckets), then the steps above.  The warp's counters are zero
-// on entry and on return.
-template <uint32_t CAP>
-__device__ __forceinline__ void warp_bucket_sort(const int32_t* src, int32_t* dst, uint32_t size, uint32_t lo,
-                                                 uint32_t bshift, uint32_t* stage, uint32_t* cnt, uint32_t* base,
-                                                 uint32_t lane) {
-  constexpr uint32_t kPer = kTinyBuckets / 32;  // buckets per lane
-  // 1. the slice into registers (all loads in flight at once), bucket counts
-  static_assert(CAP % 32 == 0 && CAP <= kTinyCap, "one warp's stage holds kTinyCap ids");
-  constexpr uint32_t kPerLane = CAP / 32;
-  uint32_t v[kPerLane];
+// Bits needed for values 0..range.
+__device__ __forceinline__ uint32_t bits_of(uint32_t range) { return 32u - (uint32_t)__clz((int)range); }
+
+// Position mask of the active lanes that hold the same 8-bit digit as this
+// one (one ballot per bit).
+__device__ __forceinline__ uint32_t digit_peers(uint32_t active, uint32_t d) {
+  uint32_t peers = active;
 #pragma unroll
-  for (uint32_t k = 0; k < kPerLane; ++k) {
+  for (int b = 0; b < 8; ++b) {
+    const uint32_t bit = (d >> b) & 1u;
+    const uint32_t bal = __ballot_sync(active, bit);
+    peers &= bit ? bal : ~bal;
+  }
+  return peers;
+}
+
+// Stable placement of this warp's ids (v[k] at position 32 k + lane of the
+// warp's run, kNone past its end) by their digit: next[d] is the next free
+// slot of digit d and advances in position order.
+template <uint32_t K>
+__device__ __forceinline__ void place_by_digit(const uint32_t (&v)[K], uint32_t lo, uint32_t shift, uint32_t* next,
+                                               uint32_t* stage, uint32_t lane) {
+  const uint32_t lt = lane_lt_mask();
+#pragma unroll
+  for (uint32_t k = 0; k < K; ++k) {
+    const bool valid = v[k] != kNone;
+    const uint32_t active = __ballot_sync(0xffffffffu, valid);
+    if (valid) {
+      const uint32_t d = ((v[k] - lo) >> shift) & 255u;
+      const uint32_t peers = digit_peers(active, d);
+      const uint32_t at = next[d] + __popc(peers & lt);
+      __syncwarp(active);
+      if (lane == (uint32_t)(__ffs(peers) - 1)) next[d] = at + __popc(peers);
+      stage[at] = v[k];
+      __syncwarp(active);
+    }
+  }
+}
+
+// Lowest and highest id of v over the warp (kNone: empty, the least as a
+// signed value).
+template <uint32_t K>
+__device__ __forceinline__ void warp_range(const uint32_t (&v)[K], uint32_t* lo, uint32_t* hi) {
+  uint32_t a = kNone;
+  int32_t b = -1;
+#pragma unroll
+  for (uint32_t k = 0; k < K; ++k) {
+    a = min(a, v[k]);
+    b = max(b, (int32_t)v[k]);
+  }
+  *lo = __reduce_min_sync(0xffffffffu, a);
+  *hi = (uint32_t)__reduce_max_sync(0xffffffffu, b);
+}
+
+// The warp's ids into registers, all loads in flight at once (position 32 k
+// + lane in v[k]).
+template <uint32_t K>
+__device__ __forceinline__ void load_slice(uint32_t (&v)[K], const int32_t* src, uint32_t size, uint32_t lane) {
+#pragma unroll
+  for (uint32_t k = 0; k < K; ++k) {
     const uint32_t i = lane + 32 * k;
     v[k] = (i < size) ? (uint32_t)__ldg(src + i) : kNone;
   }
+}
+
+// Buckets of (id - lo) >> bshift: c[] = the counts of this lane's buckets,
+// *most = the largest of all.  The counters are zero on entry and on return.
+template <uint32_t K>
+__device__ __forceinline__ void count_buckets(const uint32_t (&v)[K], uint32_t lo, uint32_t bshift, uint32_t* cnt,
+                                              uint32_t (&c)[kTinyBuckets / 32], uint32_t* most, uint32_t lane) {
+  constexpr uint32_t kPer = kTinyBuckets / 32;
 #pragma unroll
-  for (uint32_t k = 0; k < kPerLane; ++k)
+  for (uint32_t k = 0; k < K; ++k)
     if (v[k] != kNone) atomicAdd(&cnt[(v[k] - lo) >> bshift], 1u);
   __syncwarp();
-  // 2. bucket bases: each lane owns kPer consecutive buckets
-  uint32_t c[kPer];
-  uint32_t t = 0;
+  uint32_t m = 0;
 #pragma unroll
   for (uint32_t k = 0; k < kPer; ++k) {
     c[k] = cnt[lane * kPer + k];
-    t += c[k];
+    m = max(m, c[k]);
+    cnt[lane * kPer + k] = 0;
   }
+  *most = __reduce_max_sync(0xffffffffu, m);
+}
+
+// The counted slice into stage, in order: bucket bases, every id to the next
+// slot of its bucket, an insertion sort of each lane's buckets.
+template <uint32_t K>
+__device__ __forceinline__ void sort_buckets(const uint32_t (&v)[K], uint32_t lo, uint32_t bshift,
+                                             const uint32_t (&c)[kTinyBuckets / 32], uint32_t* stage, uint32_t* base,
+                                             uint32_t lane) {
+  constexpr uint32_t kPer = kTinyBuckets / 32;
+  uint32_t t = 0;
+#pragma unroll
+  for (uint32_t k = 0; k < kPer; ++k) t += c[k];
   uint32_t tot;
   uint32_t run = warp_excl_sum(t, &tot);
 #pragma unroll
@@ -140,13 +219,10 @@ __device__ __forceinline__ void warp_bucket_sort(const int32_t* src, int32_t* ds
     run += c[k];
   }
   __syncwarp();
-  // 3. every id to the next slot of its bucket (order inside a bucket is
-  //    settled below)
 #pragma unroll
-  for (uint32_t k = 0; k < kPerLane; ++k)
+  for (uint32_t k = 0; k < K; ++k)
     if (v[k] != kNone) stage[atomicAdd(&base[(v[k] - lo) >> bshift], 1u)] = v[k];
   __syncwarp();
-  // 4. insertion sort of each bucket [base - count, base); counts cleared
 #pragma unroll
   for (uint32_t k = 0; k < kPer; ++k) {
     const uint32_t n = c[k];
@@ -160,19 +236,84 @@ __device__ __forceinline__ void warp_bucket_sort(const int32_t* src, int32_t* ds
       }
       stage[b0 + jj] = key;
     }
-    cnt[lane * kPer + k] = 0;
   }
   __syncwarp();
+}
+
+// A slice whose buckets are crowded, into stage: buckets over its own range,
+// or radix passes (least significant digit first) where those are crowded
+// too.  Kept out of line so that the spread slices' code stays within the
+// registers of kTinyBlocks CTAs per SM.
+template <uint32_t CAP>
+__device__ __noinline__ void warp_sort_crowded(const int32_t* src, uint32_t size, uint32_t* stage, uint32_t* cnt,
+                                               uint32_t* base, uint32_t lane) {
+  constexpr uint32_t kPer = kTinyBuckets / 32;
+  constexpr uint32_t kPerLane = CAP / 32;
+  uint32_t v[kPerLane], c[kPer];
+  uint32_t lo, hi, most;
+  load_slice(v, src, size, lane);
+  warp_range(v, &lo, &hi);
+  const uint32_t rbits = bits_of(hi - lo);
+  const uint32_t bshift = rbits > 8 ? rbits - 8 : 0;
+  __syncwarp();
+  count_buckets(v, lo, bshift, cnt, c, &most, lane);
+  if (most <= kCrowded) {
+    sort_buckets(v, lo, bshift, c, stage, base, lane);
+    return;
+  }
+  for (uint32_t shift = 0; shift < rbits; shift += 8) {  // warp-uniform
+#pragma unroll
+    for (uint32_t k = 0; k < kPer; ++k) base[lane * kPer + k] = 0;
+    __syncwarp();
+#pragma unroll
+    for (uint32_t k = 0; k < kPerLane; ++k)
+      if (v[k] != kNone) atomicAdd(&base[((v[k] - lo) >> shift) & 255u], 1u);
+    __syncwarp();
+    uint32_t t = 0;
+#pragma unroll
+    for (uint32_t k = 0; k < kPer; ++k) t += base[lane * kPer + k];
+    uint32_t tot;
+    uint32_t run = warp_excl_sum(t, &tot);
+#pragma unroll
+    for (uint32_t k = 0; k < kPer; ++k) {
+      const uint32_t b = base[lane * kPer + k];
+      base[lane * kPer + k] = run;
+      run += b;
+    }
+    __syncwarp();
+    place_by_digit<kPerLane>(v, lo, shift, base, stage, lane);
+    __syncwarp();
+#pragma unroll
+    for (uint32_t k = 0; k < kPerLane; ++k)
+      if (lane + 32 * k < size) v[k] = stage[lane + 32 * k];
+    __syncwarp();
+  }
+}
+
+// One warp sorts the size <= CAP (<= kTinyCap) distinct ids at src into dst
+// (src may equal dst), as described above; bucket of id: (id - lo) >>
+// bshift.  The warp's counters are zero on entry and on return.
+template <uint32_t CAP>
+__device__ __forceinline__ void warp_bucket_sort(const int32_t* src, int32_t* dst, uint32_t size, uint32_t lo,
+                                                 uint32_t bshift, uint32_t* stage, uint32_t* cnt, uint32_t* base,
+                                                 uint32_t lane) {
+  static_assert(CAP % 32 == 0 && CAP <= kTinyCap, "one warp's stage holds kTinyCap ids");
+  uint32_t v[CAP / 32], c[kTinyBuckets / 32];
+  uint32_t most;
+  load_slice(v, src, size, lane);
+  count_buckets(v, lo, bshift, cnt, c, &most, lane);
+  if (most <= kCrowded) sort_buckets(v, lo, bshift, c, stage, base, lane);
+  else warp_sort_crowded<CAP>(src, size, stage, cnt, base, lane);
   for (uint32_t i = lane; i < size; i += 32) __stcs(dst + i, (int32_t)stage[i]);
   __syncwarp();
 }
 
-__global__ void __launch_bounds__(kTinyWarps * 32, 3) k_sort_tiny(const Job* __restrict__ jobs,
+__global__ void __launch_bounds__(kTinyWarps * 32, kTinyBlocks) k_sort_tiny(const Job* __restrict__ jobs,
                                                                const uint32_t* __restrict__ njobs_p,
                                                                int32_t* out, uint32_t idbits) {
   const uint32_t njobs = *njobs_p;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  TinySmem& sm = *reinterpret_cast<TinySmem*>(smem_raw);
+  auto& sm = *reinterpret_cast<TinySmem<kTinyCap>*>(smem_raw);
   const uint32_t lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
   constexpr uint32_t kPer = kTinyBuckets / 32;
   const uint32_t bshift = idbits > 8 ? idbits - 8 : 0;
@@ -190,15 +331,15 @@ __global__ void __launch_bounds__(kTinyWarps * 32, 3) k_sort_tiny(const Job* __r
 
 // Windows of at most kWinWarpMax ids (listed by k_win_split), one warp
 // each: the window's ids at src + wbase[g] in ascending order to
-// dst + wbase[g], bucketed on their low wbits bits.
-__global__ void __launch_bounds__(kTinyWarps * 32, 3) k_win_sort_warp(const uint32_t* __restrict__ list,
+// dst + wbase[g].
+__global__ void __launch_bounds__(kTinyWarps * 32, kWinWarpBlocks) k_win_sort_warp(const uint32_t* __restrict__ list,
                                                                    const uint32_t* __restrict__ nlist_p, uint32_t G,
                                                                    uint32_t wbits, const uint32_t* __restrict__ whist,
                                                                    const unsigned long long* __restrict__ wbase,
                                                                    const int32_t* __restrict__ src, int32_t* dst) {
   const uint32_t nlist = *nlist_p;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  TinySmem& sm = *reinterpret_cast<TinySmem*>(smem_raw);
+  auto& sm = *reinterpret_cast<TinySmem<kWinWarpMax>*>(smem_raw);
   const uint32_t lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
   constexpr uint32_t kPer = kTinyBuckets / 32;
   const uint32_t bshift = wbits > 8 ? wbits - 8 : 0;
@@ -246,93 +387,147 @@ __global__ void k_win_split(const uint32_t* __restrict__ njobs_p, uint32_t G, co
   }
 }
 
-// jobs_end: one past the last job; job j is jobs_end[-1 - j].
-__global__ void __launch_bounds__(kSmallThreads) k_sort_small(const Job* __restrict__ jobs_end,
-                                                              const uint32_t* __restrict__ njobs_p,
-                                                              int32_t* out, uint32_t idbits) {
+// One CTA per slice of kTinyCap < size <= kSmallCap ids: as warp_bucket_sort,
+// with the CTA's kSmallWarps warps and kBuckets buckets.  The ids stay in
+// registers (warp w holds positions [w * kWarpRun, (w + 1) * kWarpRun) of
+// the slice), so every slice is read once.  jobs_end: one past the last job;
+// job j is jobs_end[-1 - j].
+constexpr uint32_t kWarpRun = kSmallCap / kSmallWarps;
+__global__ void __launch_bounds__(kSmallThreads, 4) k_sort_small(const Job* __restrict__ jobs_end,
+                                                                 const uint32_t* __restrict__ njobs_p,
+                                                                 int32_t* out, uint32_t idbits) {
   const uint32_t njobs = *njobs_p;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   BucketSmem& s = *reinterpret_cast<BucketSmem*>(smem_raw);
   const uint32_t tid = threadIdx.x, lane = tid & 31, wp = tid >> 5;
-  const uint32_t bshift = idbits > kBucketBits ? idbits - kBucketBits : 0;
   constexpr uint32_t kPer = kBuckets / kSmallThreads;  // buckets per thread
-  for (uint32_t i = tid; i < kBuckets; i += kSmallThreads) s.cnt[i] = 0;
-  __syncthreads();
+  constexpr uint32_t kPerLane = kWarpRun / 32;
+  static_assert(kBuckets == kSmallWarps * 256, "the radix counters reuse the bucket counters");
+  // exclusive sum of one value per thread over the CTA (red[0..kSmallWarps))
+  auto excl_sum = [&](uint32_t t) -> uint32_t {
+    uint32_t wtot;
+    const uint32_t ex = warp_excl_sum(t, &wtot);
+    if (lane == 0) s.red[wp] = wtot;
+    __syncthreads();
+    uint32_t run = ex;
+    for (uint32_t k = 0; k < wp; ++k) run += s.red[k];
+    return run;
+  };
   for (uint32_t j = blockIdx.x; j < njobs; j += gridDim.x) {
     const Job jb = jobs_end[-1 - (long long)j];
     const uint32_t size = jb.size;
-    // 1. count into buckets; each id's slot in its bucket is kept by index
-    for (uint32_t i0 = 0; i0 < size; i0 += kSmallThreads * 8) {
-      uint32_t v[8];
+    int32_t* slice = out + jb.off;
+    // 1. the slice into registers, bucket counts
+    uint32_t v[kPerLane];
 #pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        const uint32_t i = i0 + k * kSmallThreads + tid;
-        v[k] = (i < size) ? (uint32_t)out[jb.off + i] : 0xffffffffu;
-      }
-#pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        const uint32_t i = i0 + k * kSmallThreads + tid;
-        if (v[k] != 0xffffffffu) s.slot[i] = (uint16_t)atomicAdd(&s.cnt[v[k] >> bshift], 1u);
-      }
+    for (uint32_t k = 0; k < kPerLane; ++k) {
+      const uint32_t i = wp * kWarpRun + k * 32 + lane;
+      v[k] = (i < size) ? (uint32_t)slice[i] : kNone;
     }
-    __syncthreads();
+    uint32_t c[kPer];  // each thread owns kPer consecutive buckets
+    uint32_t lo = 0, rbits = idbits;
+    uint32_t t, bshift;
+    auto count = [&]() -> bool {
+      bshift = rbits > kBucketBits ? rbits - kBucketBits : 0;
+#pragma unroll
+      for (uint32_t k = 0; k < kPer; ++k) s.cnt[k * kSmallThreads + tid] = 0;
+      __syncthreads();
+#pragma unroll
+      for (uint32_t k = 0; k < kPerLane; ++k)
+        if (v[k] != kNone) atomicAdd(&s.cnt[(v[k] - lo) >> bshift], 1u);
+      __syncthreads();
+      uint32_t most = 0;
+      t = 0;
+#pragma unroll
+      for (uint32_t k = 0; k < kPer; ++k) {
+        c[k] = s.cnt[tid * kPer + k];
+        t += c[k];
+        most = max(most, c[k]);
+      }
+      return __syncthreads_or(most > kCrowded);
+    };
+    bool crowded = count();
+    if (crowded) {
+      uint32_t hi;
+      warp_range(v, &lo, &hi);
+      if (lane == 0) {
+        s.red[kSmallWarps + wp] = lo;
+        s.red[2 * kSmallWarps + wp] = hi;
+      }
+      __syncthreads();
+      // (a warp without ids: lo = hi = kNone)
+#pragma unroll
+      for (uint32_t k = 0; k < kSmallWarps; ++k) {
+        lo = min(lo, s.red[kSmallWarps + k]);
+        hi = (uint32_t)max((int32_t)hi, (int32_t)s.red[2 * kSmallWarps + k]);
+      }
+      rbits = bits_of(hi - lo);
+      crowded = count();
+    }
     // 2. bucket bases
-    uint32_t c[kPer];
-    uint32_t t = 0;
+    if (!crowded) {
+      uint32_t run = excl_sum(t);
 #pragma unroll
-    for (uint32_t k = 0; k < kPer; ++k) {
-      c[k] = s.cnt[tid * kPer + k];
-      t += c[k];
-    }
-    uint32_t x = t;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-      if (lane >= (uint32_t)o) x += y;
-    }
-    if (lane == 31) s.wtot[wp] = x;
-    __syncthreads();
-    uint32_t run = x - t;
-    for (uint32_t k = 0; k < wp; ++k) run += s.wtot[k];
-#pragma unroll
-    for (uint32_t k = 0; k < kPer; ++k) {
-      s.base[tid * kPer + k] = run;
-      run += c[k];
-    }
-    __syncthreads();
-    // 3. place (ids read again, from L2); every id is read before any write
-    for (uint32_t i0 = 0; i0 < size; i0 += kSmallThreads * 8) {
-      uint32_t v[8];
-#pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        const uint32_t i = i0 + k * kSmallThreads + tid;
-        v[k] = (i < size) ? (uint32_t)out[jb.off + i] : 0xffffffffu;
+      for (uint32_t k = 0; k < kPer; ++k) {
+        s.cnt[tid * kPer + k] = run;
+        run += c[k];
       }
+      __syncthreads();
+      // 3. every id to the next slot of its bucket
 #pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        const uint32_t i = i0 + k * kSmallThreads + tid;
-        if (v[k] != 0xffffffffu) s.stage[s.base[v[k] >> bshift] + s.slot[i]] = v[k];
-      }
-    }
-    __syncthreads();
-    // 4. insertion sort inside each bucket, clear the counts
+      for (uint32_t k = 0; k < kPerLane; ++k)
+        if (v[k] != kNone) s.stage[atomicAdd(&s.cnt[(v[k] - lo) >> bshift], 1u)] = v[k];
+      __syncthreads();
+      // 4. insertion sort of each bucket [slot - count, slot)
 #pragma unroll
-    for (uint32_t k = 0; k < kPer; ++k) {
-      const uint32_t b0 = s.base[tid * kPer + k];
-      const uint32_t n = c[k];
-      for (uint32_t i = 1; i < n; ++i) {
-        const uint32_t key = s.stage[b0 + i];
-        uint32_t jj = i;
-        while (jj > 0 && s.stage[b0 + jj - 1] > key) {
-          s.stage[b0 + jj] = s.stage[b0 + jj - 1];
-          --jj;
+      for (uint32_t k = 0; k < kPer; ++k) {
+        const uint32_t n = c[k];
+        const uint32_t b0 = s.cnt[tid * kPer + k] - n;
+        for (uint32_t i = 1; i < n; ++i) {
+          const uint32_t key = s.stage[b0 + i];
+          uint32_t jj = i;
+          while (jj > 0 && s.stage[b0 + jj - 1] > key) {
+            s.stage[b0 + jj] = s.stage[b0 + jj - 1];
+            --jj;
+          }
+          s.stage[b0 + jj] = key;
         }
-        s.stage[b0 + jj] = key;
       }
-      s.cnt[tid * kPer + k] = 0;
+      __syncthreads();
+    } else {
+      // crowded: radix passes, least significant digit first; counters per
+      // (warp, digit), slots in (digit, warp) order
+      for (uint32_t shift = 0; shift < rbits; shift += 8) {  // CTA-uniform
+        uint32_t* next = s.cnt + wp * 256;
+#pragma unroll
+        for (uint32_t k = 0; k < kPer; ++k) s.cnt[k * kSmallThreads + tid] = 0;
+        __syncthreads();
+#pragma unroll
+        for (uint32_t k = 0; k < kPerLane; ++k)
+          if (v[k] != kNone) atomicAdd(&next[((v[k] - lo) >> shift) & 255u], 1u);
+        __syncthreads();
+        t = 0;
+#pragma unroll
+        for (uint32_t w = 0; w < kSmallWarps; ++w) t += s.cnt[w * 256 + tid];
+        uint32_t run = excl_sum(t);
+#pragma unroll
+        for (uint32_t w = 0; w < kSmallWarps; ++w) {
+          const uint32_t n = s.cnt[w * 256 + tid];
+          s.cnt[w * 256 + tid] = run;
+          run += n;
+        }
+        __syncthreads();
+        place_by_digit<kPerLane>(v, lo, shift, next, s.stage, lane);
+        __syncthreads();
+#pragma unroll
+        for (uint32_t k = 0; k < kPerLane; ++k) {
+          const uint32_t i = wp * kWarpRun + k * 32 + lane;
+          if (i < size) v[k] = s.stage[i];
+        }
+        __syncthreads();
+      }
     }
-    __syncthreads();
-    for (uint32_t i = tid; i < size; i += kSmallThreads) __stcs(out + jb.off + i, (int32_t)s.stage[i]);
+    for (uint32_t i = tid; i < size; i += kSmallThreads) __stcs(slice + i, (int32_t)s.stage[i]);
     __syncthreads();
   }
 }
@@ -898,8 +1093,9 @@ static void launch_win_sort(Workspace* ws, uint64_t max_pairs, uint32_t sms, con
   else launch_win_sort_t<16>(max_pairs, sms, big, ctr + kCtrWinBig, G, wbits, whist, wbase, src, out, err, s);
   if (stats) mark(ws, kEvSortBitmap, s);
   const uint64_t warp_blocks = (max_pairs + kTinyWarps - 1) / kTinyWarps;
-  k_win_sort_warp<<<(uint32_t)(warp_blocks < (uint64_t)sms * 4 ? warp_blocks : (uint64_t)sms * 4), kTinyWarps * 32,
-                    sizeof(TinySmem), s>>>(small, ctr + kCtrWinSmall, G, wbits, whist, wbase, src, out);
+  const uint64_t warp_cap = (uint64_t)sms * kWinWarpBlocks;
+  k_win_sort_warp<<<(uint32_t)(warp_blocks < warp_cap ? warp_blocks : warp_cap), kTinyWarps * 32,
+                    sizeof(TinySmem<kWinWarpMax>), s>>>(small, ctr + kCtrWinSmall, G, wbits, whist, wbase, src, out);
 }
 
 static qcp_status set_sort_attrs(const qcp_index* ix, size_t scatter_max) {
@@ -908,9 +1104,9 @@ static qcp_status set_sort_attrs(const qcp_index* ix, size_t scatter_max) {
     QCP_CUDA(cudaFuncSetAttribute(k_sort_small, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)sizeof(BucketSmem)));
     QCP_CUDA(cudaFuncSetAttribute(k_sort_tiny, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)sizeof(TinySmem)));
+                                  (int)sizeof(TinySmem<kTinyCap>)));
     QCP_CUDA(cudaFuncSetAttribute(k_win_sort_warp, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)sizeof(TinySmem)));
+                                  (int)sizeof(TinySmem<kWinWarpMax>)));
     QCP_CUDA(cudaFuncSetAttribute(k_win_sort<16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)sizeof(RankSmem<16>)));
     QCP_CUDA(cudaFuncSetAttribute(k_win_sort<17>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -951,13 +1147,14 @@ qcp_status sort_small_slices(qcp_index* ix, Workspace* ws, uint32_t q, cudaStrea
   ws->sort_small_jobs = ntiny + nsmall;
   ws->sort_msd_jobs = nbig;
   if (ntiny) {
-    k_sort_tiny<<<min((ntiny + kTinyWarps - 1) / kTinyWarps, sms * 4), kTinyWarps * 32, sizeof(TinySmem), s>>>(
+    k_sort_tiny<<<min((ntiny + kTinyWarps - 1) / kTinyWarps, sms * kTinyBlocks), kTinyWarps * 32,
+                  sizeof(TinySmem<kTinyCap>), s>>>(
         small, ctr + kCtrJobs0, ws->out_ids, idbits);
     note_launch();
     QCP_TRY(check_launch("k_sort_tiny"));
   }
   if (nsmall) {
-    k_sort_small<<<min(nsmall, sms * 3), kSmallThreads, sizeof(BucketSmem), s>>>(small + ws->jobs_cap,
+    k_sort_small<<<min(nsmall, sms * 4), kSmallThreads, sizeof(BucketSmem), s>>>(small + ws->jobs_cap,
                                                                                   ctr + kCtrSmall, ws->out_ids,
                                                                                   idbits);
     note_launch();
@@ -1108,8 +1305,8 @@ qcp_status segmented_sort_device(qcp_index* ix, Workspace* ws, uint32_t q, void*
   k_classify<<<(q + 255) / 256, 256, 0, s>>>((const unsigned long long*)ws->offsets, q, small, ctr + kCtrJobs0,
                                              ctr + kCtrSmall, ws->jobs_cap,
                                              big, ctr + kCtrJobs1, nullptr);
-  k_sort_tiny<<<sms * 4, kTinyWarps * 32, sizeof(TinySmem), s>>>(small, ctr + kCtrJobs0, ws->out_ids, idbits);
-  k_sort_small<<<sms * 3, kSmallThreads, sizeof(BucketSmem), s>>>(small + ws->jobs_cap, ctr + kCtrSmall,
+  k_sort_tiny<<<sms * kTinyBlocks, kTinyWarps * 32, sizeof(TinySmem<kTinyCap>), s>>>(small, ctr + kCtrJobs0, ws->out_ids, idbits);
+  k_sort_small<<<sms * 4, kSmallThreads, sizeof(BucketSmem), s>>>(small + ws->jobs_cap, ctr + kCtrSmall,
                                                                   ws->out_ids, idbits);
   note_launch();
   k_tiles_per_job<<<(q + 255) / 256, 256, 0, s>>>(big, ctr + kCtrJobs1, q, tiles);
