@@ -132,22 +132,18 @@ typedef struct qcp_query_opts {
    * the root's level = everything on the GPU). */
   uint32_t cpu_threads;
   uint32_t handoff_level;
-  /* Leaf prefetch of the batched traversal (0 = default): partially covered
-   * leaves are copied into a per-warp shared-memory ring by bulk copies
-   * (cp.async.bulk on the TMA unit) this many leaves ahead of the one being
-   * tested; 0 = 2 buffers, 1 = no ring (every lane loads its coordinates
-   * itself), 2..4 = that many buffers (fewer where shared memory is short).
-   * qcp_autotune picks it. */
+  /* 0..4, accepted and without effect: it was the depth of a shared-memory
+   * ring of partially covered leaves, which the count pass now reads once per
+   * run of queries and the write pass replays from recorded hit bits. */
   uint32_t leaf_prefetch;
   /* Queries per warp of the batched traversal's level expansion: lanes
    * that share one (query, node) item, 32 (default, 0), 16 or 8 (two or
    * four items per warp at once).  qcp_autotune picks it. */
   uint32_t lanes_per_item;
   /* Hit cache between the two leaf passes of a call that writes ids: the
-   * count pass records which leaves overlap and which objects of partially
-   * covered leaves hit, and the write pass replays that instead of testing
-   * again.  0 = on (default), 1 = off (the count pass runs leaner, the write
-   * pass tests again).  qcp_autotune picks it. */
+   * count pass records which objects of partially covered leaves hit, and the
+   * write pass replays that instead of testing again.  0 = on (default), 1 =
+   * off (the write pass tests again).  qcp_autotune picks it. */
   uint32_t hit_cache;
 } qcp_query_opts;
 

@@ -308,6 +308,32 @@ __global__ void k_scan_apply(const T* __restrict__ in, T* __restrict__ out, uint
   }
 }
 
+// The whole scan in one CTA: up to SC_ONE values, 16 consecutive ones per
+// thread.  Short scans are launch-bound: three kernels of 2 us each and their
+// gaps against one of 3.
+constexpr uint64_t SC_ONE = 1024 * SC_ITEMS;
+template <class T>
+__global__ void __launch_bounds__(1024) k_scan_one(const T* __restrict__ in, T* __restrict__ out, uint32_t n,
+                                                   T* grand_total) {
+  __shared__ T wt[32];
+  const uint32_t base = threadIdx.x * SC_ITEMS;
+  T vals[SC_ITEMS];
+  T s = 0;
+#pragma unroll
+  for (int r = 0; r < SC_ITEMS; ++r) {
+    vals[r] = base + r < n ? in[base + r] : (T)0;
+    s += vals[r];
+  }
+  T total;
+  T ex = block_excl_scan(s, wt, &total);
+#pragma unroll
+  for (int r = 0; r < SC_ITEMS; ++r) {
+    if (base + r < n) out[base + r] = ex;
+    ex += vals[r];
+  }
+  if (threadIdx.x == 0 && grand_total) *grand_total = total;
+}
+
 // objs -> sorted SoA arrays; flags non-finite coordinates in *bad.
 __global__ void k_pack(const float* __restrict__ objs, const uint32_t* __restrict__ perm, uint64_t n,
                        uint64_t npad, uint32_t ncoord, float* __restrict__ coords,
@@ -469,6 +495,13 @@ template <class T>
 qcp_status exclusive_scan(const T* in, T* out, uint64_t n, T* grand_total, DevPool& pool,
                           cudaStream_t s, void* scratch, size_t scratch_bytes) {
   (void)pool;
+  if (n && n <= SC_ONE) {
+    // no more threads than hold a value, in whole warps
+    const uint32_t threads = (uint32_t)(((n + SC_ITEMS - 1) / SC_ITEMS + 31) & ~31ull);
+    k_scan_one<T><<<1, threads, 0, s>>>(in, out, (uint32_t)n, grand_total);
+    note_launch();
+    return check_launch("exclusive_scan");
+  }
   const uint32_t nblk = (uint32_t)((n + SC_CHUNK - 1) / SC_CHUNK);
   void* sums = scratch;
   if (scratch) {

@@ -199,14 +199,11 @@ qcp_status ws_reserve_items(qcp_index* ix, Workspace* ws, size_t items) {
   size_t n = items + (items >> 2) + 1024;
   cudaFree(ws->items[0]);
   cudaFree(ws->items[1]);
-  cudaFree(ws->item_hits);
   ws->items[0] = ws->items[1] = nullptr;
-  ws->item_hits = nullptr;
-  ws->items_cap = ws->item_hits_cap = 0;
+  ws->items_cap = 0;
   QCP_CUDA(cudaMalloc(&ws->items[0], sizeof(uint2) * n));
   QCP_CUDA(cudaMalloc(&ws->items[1], sizeof(uint2) * n));
-  QCP_CUDA(cudaMalloc(&ws->item_hits, sizeof(uint32_t) * n));
-  ws->items_cap = ws->item_hits_cap = n;
+  ws->items_cap = n;
   return QCP_OK;
 }
 
@@ -290,15 +287,15 @@ qcp_status ws_reserve_sort(qcp_index* ix, Workspace* ws, size_t jobs, size_t til
   return QCP_OK;
 }
 
-// The count pass's hit cache: group records for `items` items and
-// `mask_words` words of partial-leaf hit masks (each grown on its own).
-qcp_status ws_reserve_hitcache(Workspace* ws, size_t items, size_t mask_words) {
-  if (items && (!ws->item_grp || ws->item_grp_cap < items)) {
+// What the count pass keeps for the write pass: `recs` group records and
+// `mask_words` words of partial-leaf hit bits (each grown on its own).
+qcp_status ws_reserve_hitcache(Workspace* ws, size_t recs, size_t mask_words) {
+  if (recs && (!ws->item_grp || ws->item_grp_cap < recs)) {
     cudaFree(ws->item_grp);
     ws->item_grp = nullptr;
     ws->item_grp_cap = 0;
-    QCP_CUDA(cudaMalloc(&ws->item_grp, sizeof(uint32_t) * kMaxGroups * kGrpWords * items));
-    ws->item_grp_cap = items;
+    QCP_CUDA(cudaMalloc(&ws->item_grp, sizeof(uint4) * recs));
+    ws->item_grp_cap = recs;
   }
   if (mask_words && (!ws->hmask || ws->hmask_cap < mask_words)) {
     cudaFree(ws->hmask);
@@ -318,13 +315,27 @@ qcp_status ws_reserve_qwhist(Workspace* ws, size_t n) {
   return QCP_OK;
 }
 
+// Counts and cursors per level-1 node and the scratch of their scan.
+qcp_status ws_reserve_nodes(Workspace* ws, size_t nodes) {
+  QCP_TRY(grow(&ws->node_hist, &ws->node_hist_cap, 2 * nodes, 1024));
+  const size_t need = scan_scratch_bytes(nodes);
+  if (!ws->scan_tmp || ws->scan_tmp_cap < need) {
+    cudaFree(ws->scan_tmp);
+    ws->scan_tmp = nullptr;
+    ws->scan_tmp_cap = 0;
+    QCP_CUDA(cudaMalloc(&ws->scan_tmp, need));
+    ws->scan_tmp_cap = need;
+  }
+  return QCP_OK;
+}
+
 void ws_destroy(Workspace* ws, qcp_index* ix) {
+  cudaFree(ws->node_hist);
   cudaFree(ws->qwhist);
   cudaFree(ws->scan_tmp);
   cudaFree(ws->boxes);
   cudaFree(ws->items[0]);
   cudaFree(ws->items[1]);
-  cudaFree(ws->item_hits);
   cudaFree(ws->item_grp);
   cudaFree(ws->hmask);
   cudaFree(ws->qcount);
@@ -578,7 +589,6 @@ static qcp_status run_query(qcp_index* ix, const float* boxes, uint32_t q, const
   ws->timing = (o.flags & QCP_QUERY_TIMING) != 0;
   ws->blocks_per_sm = o.blocks_per_sm ? (o.blocks_per_sm > 32 ? 32u : o.blocks_per_sm) : 8u;
   ws->win_bits = o.win_bits ? (o.win_bits < 12 ? 12u : o.win_bits) : kDefaultWinBits;
-  ws->leaf_ring = leaf_ring_of(o.leaf_prefetch);
   ws->lanes_per_item = lanes_per_item_of(o.lanes_per_item);
   ws->hit_cache_on = o.hit_cache != 1;
   ws->sort_small_jobs = ws->sort_msd_jobs = 0;

@@ -82,8 +82,6 @@ struct Workspace {
   size_t boxes_cap = 0;          // floats
   uint2* items[2] = {nullptr, nullptr};
   size_t items_cap = 0;          // (query, node) items per buffer
-  uint32_t* item_hits = nullptr; // per level-1 item hit counts
-  size_t item_hits_cap = 0;
   uint64_t* qcount = nullptr;    // per-query counts, q
   uint64_t* qcursor = nullptr;   // per-query write cursors, q
   uint64_t* offsets = nullptr;   // q + 1, from the index's pool
@@ -115,15 +113,16 @@ struct Workspace {
   uint32_t hist_G = 0, hist_bits = 0;
   uint32_t blocks_per_sm = 8;    // traversal grid = SMs x this, this call
   uint32_t win_bits = 18;        // sort window, this call
-  uint32_t leaf_ring = 2;        // leaf prefetch buffers per warp, this call (< 2: none)
-  // hit cache of the count pass for the write pass: per item and 32-leaf
-  // group {overlap mask, covered mask, word offset of the group's partial
-  // leaves' hit masks in hmask}; per partially covered leaf its hit bits
-  uint32_t* item_grp = nullptr;
-  size_t item_grp_cap = 0;       // items
+  // what the count pass keeps for the write pass: per item and 32-leaf group
+  // {overlap mask, covered mask, word offset of the group's partial leaves'
+  // hit bits in hmask, hits}; per partially covered leaf its hit bits
+  uint4* item_grp = nullptr;
+  size_t item_grp_cap = 0;       // records
   uint32_t* hmask = nullptr;
   size_t hmask_cap = 0;          // words
-  bool use_hit_cache = false;    // this call's count pass fills the cache
+  bool use_hit_cache = false;    // this call's count pass records hit bits
+  uint32_t* node_hist = nullptr; // items per level-1 node, then the nodes' cursors
+  size_t node_hist_cap = 0;
   bool hit_cache_on = true;      // qcp_query_opts.hit_cache of this call
   uint32_t lanes_per_item = 32;  // lanes of k_expand per (query, node) item, this call
   // CPU + GPU co-processing (QCP_ALGO_HYBRID) of this call
@@ -164,9 +163,9 @@ enum CtrSlot : uint32_t {
   kCtrSmall = 7,      // small-segment job count
   kCtrWork2 = 8,
   kCtrTimeout = 9,    // nonzero: a bounded device wait ran out (results invalid)
-  kCtrMaskWords = 10, // hit-cache words the count pass asked for (may exceed the capacity)
   kCtrWinBig = 11,    // windows listed for the bitmap sort
   kCtrWinSmall = 12,  // windows listed for the one-warp sort
+  kCtrMaskWords = 14, // (64 bits) hit-bit words the count pass asked for (may exceed the capacity)
   kCtrCount = 16
 };
 
@@ -425,13 +424,8 @@ qcp_status run_batched(qcp_index* ix, Workspace* ws, uint32_t q, bool counts_onl
                        cudaStream_t s);
 qcp_status run_plain(qcp_index* ix, Workspace* ws, uint32_t q, bool counts_only, bool sort,
                      cudaStream_t s);
-// Steps of the batched pipeline (qcp_search.cu): root items of every query
-// into items[0]; (query, node) items of level l in items[cur] -> items of
-// level l - 1 in items[cur ^ 1]; unsorted write of the level-1 items in
-// items[cur] whose item_hits are nonzero.
+// Root items of every query into items[0].
 qcp_status init_items(Workspace* ws, uint32_t q, cudaStream_t s);
-qcp_status expand_level(qcp_index* ix, Workspace* ws, uint32_t l, int cur, cudaStream_t s);
-qcp_status write_items(qcp_index* ix, Workspace* ws, int cur, cudaStream_t s);
 // Host walk of the internal levels for QCP_ALGO_HYBRID: the (query, node)
 // items of `level` for every query into items[0] and its counter.
 qcp_status host_frontier(qcp_index* ix, Workspace* ws, uint32_t q, uint32_t level, cudaStream_t s);
@@ -442,15 +436,6 @@ qcp_status segmented_sort_device(qcp_index* ix, Workspace* ws, uint32_t q, void*
 size_t sort_tables_bytes(const qcp_index* ix, const Workspace* ws, uint32_t q);
 // Window bits and window count of the per-query sort for this call.
 void sort_window_shape(const qcp_index* ix, const Workspace* ws, uint32_t* wbits, uint32_t* G);
-// Leaf prefetch buffers per warp of the traversal's leaf passes for a
-// qcp_query_opts.leaf_prefetch value: 0 = the default (2), 1 = none (direct
-// loads), 2..4 = that many.
-constexpr uint32_t kDefaultLeafRing = 2;
-inline uint32_t leaf_ring_of(uint32_t knob) {
-  if (knob == 0) return kDefaultLeafRing;
-  if (knob == 1) return 0;
-  return knob > 4 ? 4u : knob;
-}
 // Lanes per (query, node) item of the level expansion for a
 // qcp_query_opts.lanes_per_item value (0 = 32; 8, 16 or 32).
 inline uint32_t lanes_per_item_of(uint32_t knob) { return (knob == 8 || knob == 16) ? knob : 32u; }
@@ -459,11 +444,11 @@ constexpr uint32_t kHistMaxG = 256;
 // Default log2 of the per-query sort's id windows (qcp_query_opts.win_bits).
 constexpr uint32_t kDefaultWinBits = 17;
 qcp_status ws_reserve_qwhist(Workspace* ws, size_t n);
-// Words per (item, group) record of the hit cache and groups per item.
-constexpr uint32_t kGrpWords = 3;
-constexpr uint32_t kMaxGroups = 8;                    // fan-out <= 256
+constexpr uint32_t kMaxGroups = 8;                    // 32-leaf groups per item (fan-out <= 256)
 constexpr uint32_t kNoMask = 0xffffffffu;            // group without cached hit masks
-qcp_status ws_reserve_hitcache(Workspace* ws, size_t items, size_t mask_words);
+constexpr size_t kMaxMaskWords = 0xc0000000u;        // hit-bit words (32-bit offsets)
+qcp_status ws_reserve_hitcache(Workspace* ws, size_t recs, size_t mask_words);
+qcp_status ws_reserve_nodes(Workspace* ws, size_t nodes);
 // Workspace construction and buffer reservation (qcp_capi.cu).
 qcp_status ws_reserve_queries(qcp_index* ix, Workspace* ws, uint32_t q);
 qcp_status ws_reserve_items(qcp_index* ix, Workspace* ws, size_t items);
@@ -477,8 +462,7 @@ qcp_status sort_small_slices(qcp_index* ix, Workspace* ws, uint32_t q, cudaStrea
                              const SortJob** big, uint32_t* nbig);
 
 qcp_status run_batched_counts_into(qcp_index* ix, const float* boxes, uint32_t q, uint64_t* counts,
-                                   uint2* items0, uint2* items1, uint32_t* item_hits, size_t item_cap,
-                                   uint32_t* ctr, unsigned long long* stats, cudaStream_t s);
+                                   uint2* items0, uint2* items1, size_t item_cap, uint32_t* ctr, cudaStream_t s);
 qcp_status exclusive_scan_counts(const uint64_t* counts, uint64_t* offsets, uint32_t q,
                                  DevPool& pool, cudaStream_t s, void* scratch = nullptr,
                                  size_t scratch_bytes = 0);

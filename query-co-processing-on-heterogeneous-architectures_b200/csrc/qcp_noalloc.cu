@@ -29,9 +29,7 @@ constexpr uint32_t kNoAllocMaxQueries = 1u << 18;         // queries per call
 
 struct NoAllocScratch {
   uint2 items[2][kNoAllocMaxItems];
-  uint32_t item_hits[kNoAllocMaxItems];
   uint32_t ctr[kCtrCount];
-  unsigned long long stats[kStatCount];
 };
 
 constexpr size_t kNoAllocScratchBytes = sizeof(NoAllocScratch);
@@ -108,6 +106,6 @@ extern "C" qcp_status qcp_query_counts_noalloc(qcp_index* index, const float* d_
   }
   NoAllocScratch* sc = nullptr;
   QCP_TRY(scratch_on_current_device(&sc));
-  return run_batched_counts_into(index, d_boxes, q, d_counts, sc->items[0], sc->items[1], sc->item_hits,
-                                 kNoAllocMaxItems, sc->ctr, sc->stats, (cudaStream_t)stream);
+  return run_batched_counts_into(index, d_boxes, q, d_counts, sc->items[0], sc->items[1],
+                                 kNoAllocMaxItems, sc->ctr, (cudaStream_t)stream);
 }

@@ -79,7 +79,6 @@ extern "C" qcp_status qcp_plan_create(qcp_index* ix, uint32_t max_queries, uint6
   Workspace* ws = p->ws;
   ws->blocks_per_sm = (opts && opts->blocks_per_sm) ? (opts->blocks_per_sm > 32 ? 32u : opts->blocks_per_sm) : 8u;
   ws->win_bits = (opts && opts->win_bits) ? (opts->win_bits < 12 ? 12u : opts->win_bits) : kDefaultWinBits;
-  ws->leaf_ring = leaf_ring_of(opts ? opts->leaf_prefetch : 0u);
   ws->lanes_per_item = lanes_per_item_of(opts ? opts->lanes_per_item : 0u);
   qcp_status st = QCP_OK;
   do {
@@ -88,6 +87,13 @@ extern "C" qcp_status qcp_plan_create(qcp_index* ix, uint32_t max_queries, uint6
     // (query, node) items per frontier: 64 per query plus one per 1024 hits
     if ((st = ws_reserve_items(ix, ws, (size_t)max_queries * 64 + (size_t)(max_hits >> 10) + (1u << 16))) != QCP_OK)
       break;
+    // the write pass's records, hit bits for sixteen partially covered leaves
+    // per query and one per 512 hits (the write pass tests those that find no room)
+    if ((st = ws_reserve_hitcache(ws, ws->items_cap * (ix->fanout / 32),
+                                  ((size_t)max_queries * 16 + (size_t)(max_hits >> 9)) * ((ix->fanout + 127) / 128) *
+                                      8)) != QCP_OK)
+      break;
+    if (ix->levels > 1 && (st = ws_reserve_nodes(ws, ix->level_nodes[1])) != QCP_OK) break;
     if ((st = ws_reserve_out(ix, ws, (size_t)max_hits)) != QCP_OK) break;
     if ((st = ws_reserve_sort(ix, ws, (size_t)max_queries + 256, (size_t)(max_hits / kSortTile) + max_queries + 1)) !=
         QCP_OK)
@@ -102,8 +108,13 @@ extern "C" qcp_status qcp_plan_create(qcp_index* ix, uint32_t max_queries, uint6
       }
     }
     // scan scratch owned by the workspace: no stream-ordered temporaries in the graph
-    ws->scan_tmp_cap = scan_scratch_bytes((uint64_t)max_queries + 1);
-    if (cudaMalloc(&ws->scan_tmp, ws->scan_tmp_cap) != cudaSuccess ||
+    const size_t scan_need = scan_scratch_bytes((uint64_t)max_queries + 1);
+    if (ws->scan_tmp_cap < scan_need) {
+      cudaFree(ws->scan_tmp);
+      ws->scan_tmp = nullptr;
+      ws->scan_tmp_cap = scan_need;
+    }
+    if ((!ws->scan_tmp && cudaMalloc(&ws->scan_tmp, ws->scan_tmp_cap) != cudaSuccess) ||
         cudaMalloc(&p->tables, sort_tables_bytes(ix, ws, max_queries)) != cudaSuccess ||
         cudaMalloc(&p->empty, sizeof(float) * row * max_queries) != cudaSuccess) {
       st = cuda_status(cudaGetLastError(), "qcp_plan_create");

@@ -4,16 +4,17 @@
 //   1. k_expand, once per level above the leaves' parents: every
 //      (query, node) item of level l becomes the (query, child) items of the
 //      children whose MBR overlaps the query (warp per item, ballot
-//      compaction, one atomic per warp).
-//   2. k_leafscan<COUNT>: every (query, level-1 node) item is fetched
-//      dynamically by a warp from a device work counter; the warp tests the
-//      node's leaf MBRs, counts leaves whose MBR lies inside the query box
-//      without touching their objects, and tests the objects of the other
-//      overlapping leaves with 128-bit coalesced loads.
+//      compaction, one atomic per 32 items written).
+//   2. k_join: the (query, level-1 node) items, in large batches ordered by
+//      node (k_node_hist, a scan, k_node_scatter), are counted by one CTA per
+//      run of items: the node's leaf MBRs and the queries' boxes are staged in
+//      shared memory, leaves whose MBR lies inside a box are counted without
+//      touching their objects, and each other leaf that some box of the run
+//      overlaps is loaded once and tested against all of them.
 //   3. exclusive scan of the per-query counts -> CSR offsets.
-//   4. k_leafscan<WRITE>: the same items again; each warp reserves its
-//      item's slice of the query's output with one atomic and writes ids
-//      (whole id runs for covered leaves, ballot-compacted ids otherwise).
+//   4. k_leafwrite: a warp per item reserves its item's slice of the query's
+//      output with one atomic and writes ids (whole id runs for covered
+//      leaves, the hit bits k_join recorded, or a test of the leaf's objects).
 //   5. per-query sort of the ids (qcp_segsort.cu).
 //
 // Plain traversal (QCP_ALGO_PLAIN): k_mprs, one query per CUDA block,
@@ -25,6 +26,7 @@
 // (src/node/node_soa.cpp:94-113).
 #include <algorithm>
 #include <cfloat>
+#include <cstring>
 #include <thread>
 
 #include "qcp_internal.cuh"
@@ -44,25 +46,48 @@ __global__ void k_init_items(uint2* items, uint32_t q, uint32_t node, uint32_t* 
 }
 
 // LPI lanes per (query, node) item (32, 16 or 8: 1, 2 or 4 items per warp
-// at once); each group tests its item's children LPI at a time, compacts the
-// overlapping ones with the group's part of one warp ballot and reserves
-// their slots with one atomic per group and round.
+// at once); each group tests its item's children LPI at a time and the
+// overlapping ones are compacted with one warp ballot into the warp's stage in
+// shared memory, which leaves 32 items at a time.  One atomic per round on
+// the output counter bound the kernel (100,000 queries over 64 M points: 250,000
+// atomics on one address, 152 us); one per 32 items takes 63 us.
+// in == nullptr: the root level, item i is (i, node 0).
 template <int D, int LPI>
 __global__ void __launch_bounds__(256) k_expand(const float* __restrict__ boxes,
                                                 const uint2* __restrict__ in,
-                                                const uint32_t* __restrict__ in_count,
+                                                const uint32_t* __restrict__ in_count, uint32_t nroot,
                                                 uint2* __restrict__ out, uint32_t* out_count,
                                                 uint64_t out_cap, const float* __restrict__ child_mbr,
                                                 uint64_t nchild, uint64_t child_pad, uint32_t fanout,
                                                 uint32_t* overflow, uint32_t* need) {
   constexpr uint32_t kGroups = 32 / LPI;
-  constexpr uint32_t kGroupMask = LPI == 32 ? 0xffffffffu : ((1u << LPI) - 1u);
+  __shared__ uint2 stage_all[8][64];
   const uint32_t lane = threadIdx.x & 31;
+  uint2* stage = stage_all[threadIdx.x >> 5];
   const uint32_t grp = lane / LPI, gl = lane % LPI;
   // the counter keeps counting past the capacity when a level overflowed
-  const uint32_t nin = (uint32_t)min((uint64_t)*in_count, out_cap);
+  const uint32_t nin = in ? (uint32_t)min((uint64_t)*in_count, out_cap) : nroot;
   const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
   const uint32_t rounds = (fanout + LPI - 1) / LPI;  // warp-uniform
+  uint32_t held = 0;                                 // staged items (warp-uniform)
+  auto flush = [&](uint32_t k) {                     // the first k <= 32 staged items out
+    __syncwarp();
+    uint32_t base = 0;
+    if (lane == 0) base = atomicAdd(out_count, k);
+    base = __shfl_sync(0xffffffffu, base, 0);
+    if (lane < k) {
+      const uint64_t pos = (uint64_t)base + lane;
+      if (pos < out_cap) out[pos] = stage[lane];
+      else atomicOr(overflow, 1u);
+    }
+    if (lane == 0 && (uint64_t)base + k > out_cap) atomicMax(need, base + k);
+    // the rest (fewer than 32) to the front
+    const uint2 rest = stage[32 + lane];
+    __syncwarp();
+    stage[lane] = rest;
+    held -= k;
+    __syncwarp();
+  };
   for (uint32_t i0 = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * kGroups; i0 < nin; i0 += warps * kGroups) {
     const uint32_t i = i0 + grp;
     const bool have = i < nin;
@@ -70,7 +95,7 @@ __global__ void __launch_bounds__(256) k_expand(const float* __restrict__ boxes,
     Box<D> b;
     uint64_t c0 = 0, c1 = 0;
     if (have) {
-      it = in[i];
+      it = in ? in[i] : make_uint2(i, 0);
       b = load_box<D>(boxes, it.x);
       c0 = (uint64_t)it.y * fanout;
       c1 = (c0 + fanout < nchild) ? c0 + fanout : nchild;
@@ -81,399 +106,624 @@ __global__ void __launch_bounds__(256) k_expand(const float* __restrict__ boxes,
       if (have && c < c1) test_node<D>(b, child_mbr, child_pad, c, ov, in_);
       const uint32_t wm = __ballot_sync(0xffffffffu, ov);
       if (!wm) continue;  // warp-uniform
-      const uint32_t m = (wm >> (grp * LPI)) & kGroupMask;
-      uint32_t base = 0;
-      if (gl == 0 && m) base = atomicAdd(out_count, (uint32_t)__popc(m));
-      base = __shfl_sync(0xffffffffu, base, grp * LPI);
-      if (ov) {
-        const uint64_t pos = (uint64_t)base + __popc(m & ((1u << gl) - 1u));
-        if (pos < out_cap) {
-          out[pos] = make_uint2(it.x, (uint32_t)c);
-        } else {
-          atomicOr(overflow, 1u);
-        }
-      }
-      if (gl == 0 && m && (uint64_t)base + __popc(m) > out_cap) atomicMax(need, base + __popc(m));
+      if (ov) stage[held + __popc(wm & lane_lt_mask())] = make_uint2(it.x, (uint32_t)c);
+      held += __popc(wm);
+      if (held >= 32) flush(32);
     }
+  }
+  if (held) flush(held);
+}
+
+// Items per node (of `nodes`) from which node order and k_join pay: the host
+// knows only the queries, so the kernels decide from the item count whether
+// the batch is ordered.  Below it a node's leaves are shared by too few items
+// to pay for k_join's staging (4.8 M points, 2,400 boxes of four ids, 2 items
+// per node: k_join 34 us, k_count 12); 16 M points, 1,900 boxes, 29 per node:
+// 110 against 143, and 32 M 8-D rectangles, 3,000 boxes, 13 per node: 154
+// against 202.
+constexpr uint32_t kNodeOrderItems = 12;
+__device__ __forceinline__ bool is_ordered(uint32_t nitems, uint64_t nodes) {
+  return nodes && nitems >= nodes * kNodeOrderItems;
+}
+
+// Items per level-1 node, and the items in node order (cursor: the exclusive
+// sums of the counts, advanced in place) or, in a batch that is not ordered,
+// as they are.
+__global__ void k_node_hist(const uint2* __restrict__ items, const uint32_t* __restrict__ count, uint64_t cap,
+                            uint64_t nodes, uint32_t* hist) {
+  const uint32_t n = (uint32_t)min((uint64_t)*count, cap);
+  if (!is_ordered(n, nodes)) return;
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+    atomicAdd(hist + items[i].y, 1u);
+}
+
+__global__ void k_node_scatter(const uint2* __restrict__ items, const uint32_t* __restrict__ count, uint64_t cap,
+                               uint64_t nodes, uint32_t* cursor, uint2* __restrict__ out, uint32_t* out_count) {
+  const uint32_t n = (uint32_t)min((uint64_t)*count, cap);
+  const bool ordered = is_ordered(n, nodes);
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const uint2 it = items[i];
+    out[ordered ? atomicAdd(cursor + it.y, 1u) : i] = it;
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) *out_count = n;
+}
+
+enum { kCount = 0, kWrite = 1 };  // modes of the plain traversal
+
+// What the count pass hands to the write pass.  Per item and 32-leaf group,
+// rec = {overlapping leaves, covered leaves, word offset of the hit bits of
+// its partially covered leaves, hits}; per partially covered leaf and
+// 128-object chunk 32 bytes in mask, bit k of byte l = object 4l + k is a hit.  The write pass then copies ids without testing a leaf MBR or a
+// coordinate again.  A group whose hit bits did not fit (words past
+// mask_cap), or that records none (mask == nullptr), is marked kNoMask and
+// the write pass tests its partially covered leaves.  rec == nullptr: counts
+// only.
+struct HitCache {
+  uint4* rec;                  // [item][F / 32]
+  uint32_t* mask;              // hit bits
+  uint32_t mask_cap;           // words
+  unsigned long long* cursor;  // words asked for so far (may pass mask_cap)
+};
+
+constexpr uint32_t kChunkWords = 8;  // hit words of a 128-object chunk
+
+// Four consecutive objects per lane in registers: a warp holds 128 objects of
+// a leaf.
+template <int D, bool RECT>
+struct Quad {
+  float lo[D][4], hi[RECT ? D : 1][4];
+};
+__device__ __forceinline__ void load_four(float (&v)[4], const float* p) {
+  const float4 x = __ldg(reinterpret_cast<const float4*>(p));
+  v[0] = x.x, v[1] = x.y, v[2] = x.z, v[3] = x.w;
+}
+template <int D, bool RECT>
+__device__ __forceinline__ void load_quad(Quad<D, RECT>& c, const float* coords, uint64_t npad, uint64_t p) {
+#pragma unroll
+  for (int d = 0; d < D; ++d) {
+    load_four(c.lo[d], coords + (uint64_t)d * npad + p);
+    if constexpr (RECT) load_four(c.hi[d], coords + (uint64_t)(D + d) * npad + p);
   }
 }
 
-enum { kCount = 0, kWrite = 1 };
-
-// Shared memory of one warp's leaf prefetch ring: kRingHeader bytes of
-// mbarriers (one per buffer) and the list of the current item's partially
-// covered leaves (offsets in the item), then `nbuf` leaf buffers of NR runs
-// of F floats (the leaf's coordinate runs; in the write pass its ids too).
-constexpr uint32_t kRingHeader = 384;
-constexpr uint32_t kRingMaxBuf = 4;
-
-__host__ __device__ constexpr uint32_t leaf_runs(int D, bool rect, int mode) {
-  return (rect ? 2u * D : (uint32_t)D) + (mode == kWrite ? 1u : 0u);
+// The closed-interval test on sign bits: an object is a hit iff neither
+// e.hi - q.lo nor q.hi - e.lo is negative in any dimension.  The rounded
+// difference of two floats has the sign of the exact one (subnormals are not
+// flushed); a difference of zeros is -0 only if both operands allow it, so a
+// zero box bound is passed as +0 in -q.lo and q.hi; a NaN bound gives the
+// canonical NaN, sign clear, and passes as the negated comparison does;
+// objects are finite.  So this is overlaps1 exactly.  The differences go to
+// the FMA pipe and one three-input logic operation per object and dimension
+// collects the signs; comparisons would all be issued to the ALU pipe.
+// s[v] |= (sign bit) object v misses in dimension d.
+template <int D, bool RECT>
+__device__ __forceinline__ void miss_dim(const Quad<D, RECT>& c, int d, float nlo, float hi, uint32_t (&s)[4]) {
+#pragma unroll
+  for (int v = 0; v < 4; ++v)
+    s[v] |= __float_as_uint(__fadd_rn(RECT ? c.hi[RECT ? d : 0][v] : c.lo[d][v], nlo)) |
+            __float_as_uint(__fsub_rn(hi, c.lo[d][v]));
 }
-__host__ __device__ inline uint32_t ring_warp_bytes(uint32_t runs, uint32_t F, uint32_t nbuf) {
-  return kRingHeader + nbuf * runs * F * 4u;
+// The signs of a and b as bytes 0 and 1 (0xff or 0; selector bit 3 replicates
+// the selected byte's sign).
+__device__ __forceinline__ uint32_t sign_bytes(uint32_t a, uint32_t b) {
+  uint32_t r;
+  asm("prmt.b32 %0, %1, %2, 0x00fb;" : "=r"(r) : "r"(a), "r"(b));
+  return r;
+}
+// Hit bits of four objects (bit v: the sign of s[v] is clear): the four signs
+// as bytes, masked to 1, 2, 4, 8 and summed.
+__device__ __forceinline__ uint32_t hit_bits(const uint32_t (&s)[4]) {
+  const uint32_t m = __byte_perm(sign_bytes(s[0], s[1]), sign_bytes(s[2], s[3]), 0x5410);
+  return __dp4a(~m & 0x08040201u, 0x01010101u, 0u);
 }
 
-// Hit cache handed from the count pass to the write pass of one call.  The
-// count pass records, per item and 32-leaf group, the overlap and covered
-// masks of the group's leaves and where the hit bits of its partially
-// covered leaves start; per partially covered leaf and 128-object chunk it
-// records four words, bit l of word k = object 4l + k is a hit.  The write
-// pass then copies ids without testing a leaf MBR or a coordinate again.
-// grp == nullptr: no cache.  A group whose hit bits did not fit (mask words
-// past mask_cap) is marked kNoMask and the write pass tests its leaves.
-struct HitCache {
-  uint32_t* grp;       // [item][kMaxGroups][kGrpWords]
-  uint32_t* mask;      // hit bits
-  uint32_t mask_cap;   // words
-  uint32_t* cursor;    // words asked for so far (may pass mask_cap)
+// A box in shared memory: {-lo, hi} per dimension, zeros as +0.
+template <int D>
+struct BoxRow {
+  float v[2 * D];  // -lo0, hi0, -lo1, hi1, ..
+  __device__ __forceinline__ void load(const float* row) {
+    if constexpr (D % 2 == 0) {
+#pragma unroll
+      for (int e = 0; e < 2 * D; e += 4)
+        *reinterpret_cast<float4*>(v + e) = *reinterpret_cast<const float4*>(row + e);
+    } else {
+#pragma unroll
+      for (int e = 0; e < 2 * D; e += 2)
+        *reinterpret_cast<float2*>(v + e) = *reinterpret_cast<const float2*>(row + e);
+    }
+  }
 };
 
-__device__ __forceinline__ uint32_t words_per_leaf(uint32_t F) { return ((F + 127u) / 128u) * 4u; }
-constexpr uint32_t kMaskChunk = 1024;  // hit-cache words a warp takes at a time
+// Items of one CTA's run at most: one per thread.
+constexpr uint32_t kJoinItems = 128;
+constexpr uint32_t kJoinThreads = 128;
+constexpr uint32_t kJoinWarps = kJoinThreads / 32;
+constexpr uint32_t kJoinTasks = 8;  // tasks per CTA in large batches
+constexpr uint32_t kPairs = 8;      // (leaf, box) pairs counted and stored together
 
-// Warp per (query, level-1 node) item.  COUNT: item_hits[i] and qcount[q].
-// WRITE: ids at out[offsets[q] + reserved slice].
-// PF: the partially covered leaves of an item are fetched into the warp's
-// shared-memory ring by bulk copies (cp.async.bulk on the TMA unit, nbuf
-// leaves ahead, completion on one mbarrier per buffer) while the warp tests
-// the leaf before; without PF every lane loads its float4s from global
-// memory.  A bulk-copy wait that runs out sets err[0] and the warp stops.
-template <int D, bool RECT, int MODE, bool PF, bool CACHE>
-__global__ void __launch_bounds__(256) k_leafscan(TreeView t, const float* __restrict__ boxes,
-                                                  const uint2* __restrict__ items,
-                                                  const uint32_t* __restrict__ item_count,
-                                                  uint32_t* work, uint32_t* __restrict__ item_hits,
-                                                  unsigned long long* qcount,
-                                                  const unsigned long long* __restrict__ offsets,
-                                                  unsigned long long* qcursor,
-                                                  int32_t* __restrict__ out, uint64_t item_cap,
-                                                  unsigned long long* stats, uint32_t* qwhist, uint32_t hist_G,
-                                                  uint32_t hist_bits, uint32_t nbuf, uint32_t* err,
-                                                  HitCache hc) {
-  // write pass of the sorted path: per-(query, window) id counts in per-warp
-  // shared counters, flushed once per item
-  __shared__ uint32_t wcount[8][MODE == kWrite ? kHistMaxG : 1];
-  extern __shared__ __align__(128) unsigned char ring_raw[];
-  constexpr uint32_t NC = RECT ? 2 * D : D;       // coordinate runs of a leaf
-  constexpr uint32_t NR = leaf_runs(D, RECT, MODE);
+// Counts: qcount[q] of every query, and the records of hc.  A task is a run of
+// consecutive items and one 32-leaf group of their nodes; the items of one
+// node are treated together: the leaves' coordinates, which one warp per item
+// read again for every item, are read once per run.  That read bounded the
+// pass: 32 M 8-D rectangles, 50,000 boxes (426,542 items, 1.7 M partially
+// covered leaves of 8 KB) 2.53 -> 0.82 ms; 16 M 3-D points, 10,000 boxes 0.68 ->
+// 0.30 ms; 64 M 2-D points, 100,000 boxes 0.50 -> 0.25 ms.  The run length
+// follows from the item count: kJoinTasks tasks per CTA (the tail of the last
+// ones is short), at most kJoinItems items; small batches get one item per
+// task, its leaves spread over the warps.
+// What remains is bound by issue and by what shared memory can broadcast (a
+// box of 2 D floats takes 2 D cycles of an SM whatever the width of the
+// loads), so a (leaf, box) pair is kept short: four objects per lane, sign
+// bits instead of comparisons, the leaf's boxes from a list, a byte of hit
+// bits per lane instead of ballots, and the bytes of kPairs pairs are counted
+// and stored together.  (Prefetching the next leaf, into registers or L2,
+// measured 15 % slower; packed f32x2 differences need every bound twice and
+// were slower too.)
+template <int D, bool RECT>
+__global__ void __launch_bounds__(kJoinThreads, (RECT ? 2 * D : D) > 8 ? 4 : ((RECT ? 2 * D : D) > 4 ? 6 : 8))
+    k_join(TreeView t, const float* __restrict__ boxes, const uint2* __restrict__ items,
+           const uint32_t* __restrict__ item_count, uint32_t* work, unsigned long long* qcount, uint64_t item_cap,
+           uint64_t nodes, unsigned long long* stats, HitCache hc) {
+  __shared__ __align__(16) float bx[kJoinItems * 2 * D];
+  __shared__ uint2 item[kJoinItems];
+  __shared__ uint32_t part[kJoinItems], cov[kJoinItems];    // partially covered and covered leaves
+  __shared__ uint32_t hits[kJoinItems], moff[kJoinItems];   // moff kNoMask: no hit bits kept
+  __shared__ uint16_t s_list[kJoinWarps][kJoinItems];       // the warp's leaf: items that overlap it
+  __shared__ __align__(16) uint8_t s_hit[kJoinWarps][kPairs * 32];  // hit bits of kPairs pairs
+  __shared__ uint32_t s_pair[kJoinWarps][kPairs];           // their item | leaf << 16 | chunk << 24
+  __shared__ uint32_t s_task, s_any, s_wsum[kJoinWarps];
+  __shared__ unsigned long long s_base;
+  const uint32_t F = t.fanout, G = F >> 5;
+  const uint32_t tid = threadIdx.x, lane = tid & 31, wp = tid >> 5;
+  const uint32_t nitems = (uint32_t)min((uint64_t)*item_count, item_cap);
+  if (!is_ordered(nitems, nodes)) return;  // k_count's
+  const float* lmbr = t.mbr[0];
+  const uint64_t lpad = t.pad[0], nleaves = t.nodes[0];
+  const uint32_t chunks = (F + 127u) >> 7;  // 128-object chunks of a leaf
+  const uint32_t wpl = chunks * kChunkWords;
+  uint64_t want = (uint64_t)nitems * G / (gridDim.x * kJoinTasks);
+  const uint32_t runlen = want < 1 ? 1u : (want > kJoinItems ? kJoinItems : (uint32_t)want);
+  uint32_t n_cov = 0, n_part = 0;  // work counters of this thread's items
+  unsigned long long o_cov = 0;
+  uint16_t* list = s_list[wp];
+  uint8_t* bytes = s_hit[wp];
+  uint32_t* pairs = s_pair[wp];
+  uint32_t fetched = 0;  // thread 0: the task after the current one
+  if (tid == 0) s_task = atomicAdd(work, 1u);
+  for (;;) {
+    __syncthreads();  // the task is known, the previous one finished with the shared memory
+    const uint32_t g = s_task % G;
+    const uint64_t i0 = (uint64_t)(s_task / G) * runlen;
+    if (i0 >= nitems) break;
+    const uint32_t rn = (uint32_t)min((uint64_t)runlen, nitems - i0);
+    if (tid < rn) item[tid] = items[i0 + tid];
+    __syncthreads();
+    if (tid == 0) fetched = atomicAdd(work, 1u);
+    for (uint32_t a = 0; a < rn;) {
+      // the run's next node and its items [a, a + m)
+      const uint32_t node = item[a].y;
+      uint32_t m = 0;
+      for (uint32_t j = a; j < rn; j += 32) {
+        const uint32_t diff = __ballot_sync(0xffffffffu, j + lane >= rn || item[j + lane].y != node);
+        m += diff ? __ffs(diff) - 1 : 32;
+        if (diff) break;
+      }
+      const uint64_t l0 = (uint64_t)node * F + g * 32;  // the group's first leaf
+      const uint32_t nl = l0 < nleaves ? (uint32_t)min((uint64_t)32, nleaves - l0) : 0u;
+      for (uint32_t e = tid; e < m * 2 * D; e += kJoinThreads) {
+        const uint32_t j = e / (2 * D), c = e % (2 * D);
+        const float v = __ldg(boxes + (uint64_t)item[a + j].x * (2 * D) + c);
+        bx[j * 2 * D + (c < D ? 2 * c : 2 * (c - D) + 1)] = v == 0.f ? 0.f : (c < D ? -v : v);
+      }
+      if (tid == 0) s_any = 0;
+      __syncthreads();
+      // A. every item's masks: a leaf's MBR per lane in registers (level_pad is
+      // a multiple of F, so whole groups exist)
+      if (wp < m) {
+        float lo[D], hi[D];
+#pragma unroll
+        for (int d = 0; d < D; ++d) {
+          lo[d] = __ldg(lmbr + d * lpad + l0 + lane);
+          hi[d] = __ldg(lmbr + (D + d) * lpad + l0 + lane);
+        }
+        uint32_t any = 0;
+        for (uint32_t j = wp; j < m; j += kJoinWarps) {
+          BoxRow<D> b;
+          b.load(bx + j * 2 * D);
+          bool ov = lane < nl;
+#pragma unroll
+          for (int d = 0; d < D; ++d) ov &= overlaps1(-b.v[2 * d], b.v[2 * d + 1], lo[d], hi[d]);
+          const uint32_t mov = __ballot_sync(0xffffffffu, ov);
+          uint32_t mcov = 0, h = 0;
+          if (mov) {  // warp-uniform
+            bool in = ov;
+#pragma unroll
+            for (int d = 0; d < D; ++d) in &= inside1(-b.v[2 * d], b.v[2 * d + 1], lo[d], hi[d]);
+            mcov = __ballot_sync(0xffffffffu, in);
+            if (mcov) {
+              h = __popc(mcov) * F;
+              // the tree's last leaf may hold fewer than F objects
+              const uint64_t last = nleaves - 1 - l0;
+              if (last < 32 && ((mcov >> last) & 1u)) h -= (uint32_t)(nleaves * F - t.n);
+            }
+          }
+          any |= mov & ~mcov;
+          if (lane == 0) {
+            part[j] = mov & ~mcov;
+            cov[j] = mcov;
+            hits[j] = h;
+          }
+        }
+        if (lane == 0 && any) atomicOr(&s_any, any);
+      }
+      __syncthreads();
+      // room for the items' hit bits (one atomic) and where each one's start
+      const uint32_t any = s_any;
+      uint32_t off = kNoMask;
+      if (hc.mask && any) {  // CTA-uniform
+        const uint32_t words = tid < m ? __popc(part[tid]) * wpl : 0u;
+        uint32_t wtot;
+        const uint32_t ex = warp_excl_sum(words, &wtot);
+        if (lane == 0) s_wsum[wp] = wtot;
+        __syncthreads();
+        uint32_t before = 0, total = 0;
+#pragma unroll
+        for (uint32_t w = 0; w < kJoinWarps; ++w) {
+          const uint32_t c = s_wsum[w];
+          before += w < wp ? c : 0u;
+          total += c;
+        }
+        if (tid == 0) s_base = atomicAdd(hc.cursor, (unsigned long long)total);
+        __syncthreads();
+        if (words && s_base + total <= hc.mask_cap) off = (uint32_t)s_base + before + ex;
+      }
+      if (tid < m) moff[tid] = off;
+      __syncthreads();
+      // B. partially covered leaves: a warp per leaf, against every box that
+      // overlaps it
+      uint32_t held = 0;  // pairs whose hit bits are held
+      auto flush = [&]() {
+        __syncwarp();
+        // eight bytes per lane, four lanes per pair
+        const bool mine = lane / 4 < held;
+        const uint32_t pr = mine ? pairs[lane / 4] : 0u;
+        const uint2 w = mine ? reinterpret_cast<const uint2*>(bytes)[lane] : make_uint2(0, 0);
+        const uint32_t j = pr & 0xffffu, k = (pr >> 16) & 0xffu, x = pr >> 24;
+        uint32_t cnt = __popc(w.x) + __popc(w.y);
+        cnt += __shfl_xor_sync(0xffffffffu, cnt, 1);
+        cnt += __shfl_xor_sync(0xffffffffu, cnt, 2);
+        if (mine) {
+          if ((lane & 3) == 0 && cnt) atomicAdd(&hits[j], cnt);
+          const uint32_t at = moff[j];
+          // by the leaf's place among the item's partially covered ones
+          if (at != kNoMask)
+            *reinterpret_cast<uint2*>(hc.mask + at + __popc(part[j] & ((1u << k) - 1u)) * wpl + x * kChunkWords +
+                                      (lane & 3) * 2) = w;
+        }
+        held = 0;
+        __syncwarp();
+      };
+      for (uint32_t k = wp; k < 32; k += kJoinWarps) {
+        if (!((any >> k) & 1u)) continue;  // warp-uniform
+        uint32_t np = 0;                   // pairs of this leaf
+        for (uint32_t j0 = 0; j0 < m; j0 += 32) {
+          const bool on = j0 + lane < m && ((part[j0 + lane] >> k) & 1u);
+          const uint32_t sel = __ballot_sync(0xffffffffu, on);
+          if (on) list[np + __popc(sel & lane_lt_mask())] = (uint16_t)(j0 + lane);
+          np += __popc(sel);
+        }
+        __syncwarp();
+        const uint64_t e0 = (l0 + k) * F;
+        for (uint32_t x = 0; x < chunks; ++x) {
+          const uint32_t o = x * 128 + lane * 4;
+          Quad<D, RECT> c;
+          if (o < F) load_quad<D, RECT>(c, t.coords, t.npad, e0 + o);
+          // lanes past the leaf's end, objects past n (padding of the last leaf)
+          uint32_t live = 0xfu;
+          if (o >= F || e0 + o >= t.n) live = 0;
+          else if (e0 + o + 4 > t.n) live = (1u << (t.n - e0 - o)) - 1u;
+          for (uint32_t i = 0; i < np; ++i) {
+            const uint32_t j = list[i];
+            BoxRow<D> b;
+            b.load(bx + j * 2 * D);
+            uint32_t s[4] = {0, 0, 0, 0};
+#pragma unroll
+            for (int d = 0; d < D; ++d) miss_dim<D, RECT>(c, d, b.v[2 * d], b.v[2 * d + 1], s);
+            bytes[held * 32 + lane] = (uint8_t)(hit_bits(s) & live);
+            if (lane == 0) pairs[held] = j | (k << 16) | (x << 24);
+            if (++held == kPairs) flush();
+          }
+        }
+        __syncwarp();
+      }
+      if (held) flush();
+      __syncthreads();
+      if (tid < m) {
+        const uint32_t cm = cov[tid], pm = part[tid], h = hits[tid];
+        if (hc.rec) hc.rec[(i0 + a + tid) * G + g] = make_uint4(pm | cm, cm, moff[tid], h);
+        if (h) atomicAdd(qcount + item[a + tid].x, (unsigned long long)h);
+        if (stats) {
+          n_cov += __popc(cm);
+          n_part += __popc(pm);
+          o_cov += __popc(cm) * F;
+          const uint64_t last = nleaves - 1 - l0;
+          if (last < 32 && ((cm >> last) & 1u)) o_cov -= nleaves * F - t.n;
+        }
+      }
+      a += m;
+      __syncthreads();  // the masks and boxes are free for the next node
+    }
+    if (tid == 0) s_task = fetched;
+  }
+  if (stats) {
+    if (n_cov) atomicAdd(stats + kStatCovered, (unsigned long long)n_cov);
+    if (n_part) atomicAdd(stats + kStatPartial, (unsigned long long)n_part);
+    if (o_cov) atomicAdd(stats + kStatObjCovered, o_cov);
+  }
+}
+
+// Counts of batches that are not in node order: a warp per item, or per
+// 32-leaf group of one where there are too few items to keep the warps busy;
+// no barriers.  Few items share a node, so nothing is staged: the box sits in
+// registers, a group's MBRs are tested one per lane, and the partially covered
+// leaves one after the other.  Bound by the latency of its dependent reads
+// (item, box and MBRs, objects).  1,000 boxes over 1 M points: 18.9 (a warp
+// per item) -> 12.4 us; 64 boxes over 16 M points 36.7 -> 14.8 us.
+template <int D, bool RECT>
+__global__ void __launch_bounds__(256, (RECT ? 2 * D : D) > 8 ? 2 : 4)
+    k_count(TreeView t, const float* __restrict__ boxes, const uint2* __restrict__ items,
+            const uint32_t* __restrict__ item_count, unsigned long long* qcount, uint64_t item_cap,
+            uint64_t nodes, unsigned long long* stats, HitCache hc) {
   const uint32_t lane = threadIdx.x & 31;
-  const uint32_t wib = (threadIdx.x >> 5) & 7;
-  uint32_t* wc = wcount[wib];
-  const bool hist = MODE == kWrite && qwhist != nullptr;
+  const uint32_t F = t.fanout, G = F >> 5;
+  const uint32_t nitems = (uint32_t)min((uint64_t)*item_count, item_cap);
+  if (is_ordered(nitems, nodes)) return;  // k_join's
+  const uint64_t nleaves = t.nodes[0], lpad = t.pad[0];
+  const float* lmbr = t.mbr[0];
+  const uint32_t chunks = (F + 127u) >> 7, wpl = chunks * kChunkWords;
+  const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
+  const bool whole = nitems >= warps * 2u;
+  const uint64_t units = whole ? nitems : (uint64_t)nitems * G;
+  uint64_t u = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  uint2 next = u < units ? items[whole ? u : u / G] : make_uint2(0, 0);
+  for (; u < units; u += warps) {
+    const uint2 it = next;
+    if (u + warps < units) next = items[whole ? u + warps : (u + warps) / G];
+    float b[2 * D];  // -lo, hi per dimension, zeros as +0
+    const float* q = boxes + (uint64_t)it.x * 2 * D;
+#pragma unroll
+    for (int d = 0; d < D; ++d) {
+      const float lo = __ldg(q + d), hi = __ldg(q + D + d);
+      b[2 * d] = lo == 0.f ? 0.f : -lo;
+      b[2 * d + 1] = hi == 0.f ? 0.f : hi;
+    }
+    uint32_t total = 0;  // hits of the unit
+    const uint32_t ga = whole ? 0u : (uint32_t)(u % G), gb = whole ? G : ga + 1;
+    for (uint32_t g = ga; g < gb; ++g) {
+      const uint64_t l0 = (uint64_t)it.y * F + g * 32;  // the group's first leaf
+      bool ov = l0 + lane < nleaves, in = true;
+#pragma unroll
+      for (int d = 0; d < D; ++d) {
+        const float lo = __ldg(lmbr + d * lpad + l0 + lane), hi = __ldg(lmbr + (D + d) * lpad + l0 + lane);
+        ov &= overlaps1(-b[2 * d], b[2 * d + 1], lo, hi);
+        in &= inside1(-b[2 * d], b[2 * d + 1], lo, hi);
+      }
+      const uint32_t mov = __ballot_sync(0xffffffffu, ov), mcov = __ballot_sync(0xffffffffu, ov && in);
+      const uint32_t part = mov & ~mcov;
+      // room for the hit bits; the objects' reads do not wait for it
+      uint32_t off = kNoMask;
+      const uint32_t words = __popc(part) * wpl;
+      unsigned long long base = 0;
+      if (hc.mask && words && lane == 0) base = atomicAdd(hc.cursor, (unsigned long long)words);
+      uint32_t hits = 0;  // of this lane
+      // the partially covered leaves' 128-object chunks, kAhead at a time
+      constexpr uint32_t kAhead = (RECT ? 2 * D : D) <= 4 ? 2 : 1;
+      const uint32_t nchunk = __popc(part) * chunks;
+      uint32_t mp = part, x = 0;
+      for (uint32_t c0 = 0; c0 < nchunk; c0 += kAhead) {
+        Quad<D, RECT> c[kAhead];
+        uint64_t p[kAhead];  // first object of the lane's four, t.n: none
+#pragma unroll
+        for (uint32_t v = 0; v < kAhead; ++v) {
+          p[v] = t.n;
+          if (c0 + v >= nchunk) continue;  // warp-uniform
+          const uint32_t o = x * 128 + lane * 4;
+          if (o < F) {
+            p[v] = (l0 + __ffs(mp) - 1) * F + o;
+            load_quad<D, RECT>(c[v], t.coords, t.npad, p[v]);
+          }
+          if (++x == chunks) {
+            x = 0;
+            mp &= mp - 1;
+          }
+        }
+        if (hc.mask && c0 == 0) {
+          base = __shfl_sync(0xffffffffu, base, 0);
+          if (base + words <= hc.mask_cap) off = (uint32_t)base;
+        }
+#pragma unroll
+        for (uint32_t v = 0; v < kAhead; ++v) {
+          if (c0 + v >= nchunk) continue;
+          uint32_t s[4] = {0, 0, 0, 0};
+#pragma unroll
+          for (int d = 0; d < D; ++d) miss_dim<D, RECT>(c[v], d, b[2 * d], b[2 * d + 1], s);
+          uint32_t hm = hit_bits(s);
+          // objects past n (padding of the last leaf) never hit
+          if (p[v] + 4 > t.n) hm &= p[v] < t.n ? (1u << (t.n - p[v])) - 1u : 0u;
+          hits += __popc(hm);
+          if (off != kNoMask)
+            reinterpret_cast<uint8_t*>(hc.mask + off + (c0 + v) * kChunkWords)[lane] = (uint8_t)hm;
+        }
+      }
+      hits = __reduce_add_sync(0xffffffffu, hits);
+      uint32_t chits = __popc(mcov) * F;
+      // the tree's last leaf may hold fewer than F objects
+      const uint64_t last = nleaves - 1 - l0;
+      if (last < 32 && ((mcov >> last) & 1u)) chits -= (uint32_t)(nleaves * F - t.n);
+      hits += chits;
+      if (lane == 0) {
+        if (hc.rec) hc.rec[whole ? u * G + g : u] = make_uint4(mov, mcov, off, hits);
+        if (stats) {
+          if (mcov) atomicAdd(stats + kStatCovered, (unsigned long long)__popc(mcov));
+          if (part) atomicAdd(stats + kStatPartial, (unsigned long long)__popc(part));
+          if (chits) atomicAdd(stats + kStatObjCovered, (unsigned long long)chits);
+        }
+      }
+      total += hits;
+    }
+    if (lane == 0 && total) atomicAdd(qcount + it.x, (unsigned long long)total);
+  }
+}
+
+// A warp per (query, level-1 node) item, or per 32-leaf group of one where the
+// batch has too few items to keep the warps busy (64 boxes over 16 M points:
+// 72 -> 22 us, the chain of one warp copying an item's up to 16,384 ids):
+// the group's slot in the query's slice is reserved by its hit count, ids of
+// covered leaves are copied as whole runs, ids of partially covered ones by
+// their hit bits.  Bound by the writes of the ids and the latency in front of
+// them: the records and slots of an item's groups are taken at once (one
+// lane each), the hit bits of a group's leaves by one load, and four leaves'
+// ids are in flight together.  qwhist: per-(query, window) id counts for the
+// sort, gathered in per-warp shared counters and flushed once per fetch.
+constexpr uint32_t kWriteUnroll = 4;
+template <int D, bool RECT>
+__global__ void __launch_bounds__(256) k_leafwrite(TreeView t, const float* __restrict__ boxes,
+                                                   const uint2* __restrict__ items,
+                                                   const uint32_t* __restrict__ item_count, uint32_t* work,
+                                                   const uint4* __restrict__ rec, const uint32_t* __restrict__ hmask,
+                                                   const unsigned long long* __restrict__ offsets,
+                                                   unsigned long long* qcursor, int32_t* __restrict__ out,
+                                                   uint64_t item_cap, uint32_t* qwhist, uint32_t hist_G,
+                                                   uint32_t hist_bits) {
+  __shared__ uint32_t wcount[8][kHistMaxG];
+  const uint32_t lane = threadIdx.x & 31, lt = lane_lt_mask();
+  uint32_t* wc = wcount[(threadIdx.x >> 5) & 7];
+  const bool hist = qwhist != nullptr;
   if (hist) {
     for (uint32_t w = lane; w < hist_G; w += 32) wc[w] = 0;
     __syncwarp();
   }
-  const uint32_t F = t.fanout;
-  unsigned char* ring = ring_raw + (size_t)wib * (PF ? ring_warp_bytes(NR, F, nbuf) : 0u);
-  uint64_t* bars = reinterpret_cast<uint64_t*>(ring);
-  uint8_t* plist = ring + 64;
-  float* bufs = reinterpret_cast<float*>(ring + kRingHeader);
-  const uint32_t buf_floats = NR * F;
-  uint32_t phase = 0;     // bit b: parity of buffer b's next completion
-  uint32_t pending = 0;   // bit b: a copy into buffer b has not been waited for
-  bool dead = false;      // a bulk-copy wait ran out
-  if (PF) {
-    if (lane == 0) {
-      for (uint32_t b = 0; b < nbuf; ++b) mbar_init(&bars[b], 1);
-      mbar_fence_init();
-    }
-    __syncwarp();
-  }
-  // hit-bit room in per-warp chunks of the global cursor (one atomic per
-  // chunk, not per group); kNoMask once the cache's capacity is used up
-  // (the warp's chunk is kept in shared memory, not in registers: the count
-  // pass is latency-bound and its occupancy is set by its registers)
-  __shared__ uint32_t chunk[8][2];  // per warp: next word, end (end = kNoMask: no room left)
-  if (CACHE) {
-    if (lane == 0) chunk[wib][0] = chunk[wib][1] = 0;
-    __syncwarp();
-  }
-  auto mask_alloc = [&](uint32_t want) -> uint32_t {
-    uint32_t r = 0;
-    if (lane == 0) {
-      uint32_t pos = chunk[wib][0], end = chunk[wib][1];
-      if (end == kNoMask) {
-        r = kNoMask;
-      } else {
-        if (pos + want > end) {
-          const uint32_t grab = want > kMaskChunk ? want : kMaskChunk;
-          pos = atomicAdd(hc.cursor, grab);
-          end = ((uint64_t)pos + grab > hc.mask_cap) ? kNoMask : pos + grab;
-        }
-        r = (end == kNoMask) ? kNoMask : pos;
-        chunk[wib][0] = pos + want;
-        chunk[wib][1] = end;
-      }
-    }
-    return __shfl_sync(0xffffffffu, r, 0);
-  };
+  const uint32_t F = t.fanout, G = F >> 5;
+  const uint32_t cpl = (F + 127u) >> 7;  // 128-object chunks per leaf
   const uint32_t nitems = (uint32_t)min((uint64_t)*item_count, item_cap);
-  const float* lmbr = t.mbr[0];
-  const uint64_t lpad = t.pad[0];
-  const uint64_t nleaves = t.nodes[0];
+  const uint32_t warps = gridDim.x * (blockDim.x >> 5);
+  // groups per fetch: a whole item, or one group in small batches
+  const bool whole = nitems >= warps * 4u;
+  const uint32_t per = whole ? G : 1u;
+  const uint32_t nfetch = whole ? nitems : nitems * G;
   for (;;) {
-    uint32_t i = 0;
-    if (lane == 0) i = atomicAdd(work, 1u);
-    i = __shfl_sync(0xffffffffu, i, 0);
-    if (i >= nitems) break;
+    uint32_t f = 0;
+    if (lane == 0) f = atomicAdd(work, 1u);
+    f = __shfl_sync(0xffffffffu, f, 0);
+    if (f >= nfetch) break;
+    const uint32_t i = whole ? f : f / G, gbase = whole ? 0u : f % G;
     const uint2 it = items[i];
-    const Box<D> b = load_box<D>(boxes, it.x);
-    uint64_t wpos = 0;
-    if (MODE == kWrite) {
-      const uint32_t mine = item_hits[i];
-      if (mine == 0) continue;
-      if (lane == 0) wpos = offsets[it.x] + atomicAdd(qcursor + it.x, (unsigned long long)mine);
-      wpos = __shfl_sync(0xffffffffu, wpos, 0);
+    uint4 r = make_uint4(0, 0, kNoMask, 0);
+    unsigned long long at = 0;
+    if (lane < per) {
+      r = rec[(size_t)i * G + gbase + lane];
+      if (r.w) at = offsets[it.x] + atomicAdd(qcursor + it.x, (unsigned long long)r.w);
     }
-    uint32_t hits = 0;  // per lane (count mode)
-    uint32_t n_cov = 0, n_part = 0, o_cov = 0;  // per lane work counters (count mode)
-    uint32_t npart = 0;  // PF: partially covered leaves listed for the ring
-    const uint64_t l0 = (uint64_t)it.y * F;
-    const uint64_t l1 = (l0 + F < nleaves) ? l0 + F : nleaves;
-    const bool cache = CACHE && hc.grp != nullptr;
-    const uint32_t wpl = words_per_leaf(F);
-    uint32_t* grec = cache ? hc.grp + (size_t)i * (kMaxGroups * kGrpWords) : nullptr;
-    uint32_t g_mov = 0, g_min = 0;  // ring path: lane g holds group g's masks
-    for (uint64_t lb = l0; lb < l1; lb += 32) {
-      const uint32_t gi = (uint32_t)((lb - l0) >> 5);
-      const uint64_t leaf = lb + lane;
-      bool ov = false, in_ = false;
-      uint32_t mov, min_, moff = kNoMask;
-      if (MODE == kWrite && cache) {
-        // the count pass's masks of this group
-        mov = grec[gi * kGrpWords + 0];
-        min_ = grec[gi * kGrpWords + 1];
-        moff = grec[gi * kGrpWords + 2];
-      } else {
-        if (leaf < l1) test_node<D>(b, lmbr, lpad, leaf, ov, in_);
-        mov = __ballot_sync(0xffffffffu, ov);
-        min_ = __ballot_sync(0xffffffffu, in_ && ov);
-        if (MODE == kCount && cache) {
-          if (PF) {
-            // recorded after the loop, with room for the whole item
-            if (lane == gi) {
-              g_mov = mov;
-              g_min = min_;
-            }
-          } else {
-            // record the group with room for its partial leaves' hit bits
-            const uint32_t np = __popc(mov & ~min_);
-            if (np) moff = mask_alloc(np * wpl);
-            if (lane == 0) {
-              grec[gi * kGrpWords + 0] = mov;
-              grec[gi * kGrpWords + 1] = min_;
-              grec[gi * kGrpWords + 2] = moff;
-            }
-          }
-        }
-      }
-      if (!mov) continue;
-      // leaves whose MBR lies inside the query: every object is a hit
-      if (MODE == kCount) {
-        if (in_ && ov) {
-          const uint64_t e0 = leaf * F;
-          const uint64_t e1 = (e0 + F < t.n) ? e0 + F : t.n;
-          hits += (uint32_t)(e1 - e0);
-          o_cov += (uint32_t)(e1 - e0);
-          ++n_cov;
-        } else if (ov) {
-          ++n_part;
-        }
-      } else {
-        uint32_t m = min_;
-        while (m) {
-          // a run of consecutive covered leaves is one contiguous id range
-          const int s = __ffs(m) - 1;
-          const uint32_t shifted = ~(m >> s);
-          const int len = shifted ? (__ffs(shifted) - 1) : (32 - s);
-          m &= ~((len >= 32 ? 0xffffffffu : ((1u << len) - 1u)) << s);
-          const uint64_t e0 = (lb + s) * F;
-          uint64_t e1 = (lb + s + len) * F;
-          if (e1 > t.n) e1 = t.n;
-          const int32_t* src = t.ids + e0;
-          const uint64_t cnt = e1 - e0;
-          // eight loads in flight per lane before their stores
-          uint64_t j = lane;
-          for (; j + 224 < cnt; j += 256) {
-            int32_t v[8];
-#pragma unroll
-            for (int k = 0; k < 8; ++k) v[k] = __ldg(src + j + 32 * k);
-#pragma unroll
-            for (int k = 0; k < 8; ++k) out[wpos + j + 32 * k] = v[k];
-            if (hist) {
-#pragma unroll
-              for (int k = 0; k < 8; ++k) atomicAdd(wc + ((uint32_t)v[k] >> hist_bits), 1u);
-            }
-          }
-          for (; j + 96 < cnt; j += 128) {
-            const int32_t a = __ldg(src + j), b = __ldg(src + j + 32);
-            const int32_t c = __ldg(src + j + 64), d = __ldg(src + j + 96);
-            out[wpos + j] = a;
-            out[wpos + j + 32] = b;
-            out[wpos + j + 64] = c;
-            out[wpos + j + 96] = d;
-            if (hist) {
-              atomicAdd(wc + ((uint32_t)a >> hist_bits), 1u);
-              atomicAdd(wc + ((uint32_t)b >> hist_bits), 1u);
-              atomicAdd(wc + ((uint32_t)c >> hist_bits), 1u);
-              atomicAdd(wc + ((uint32_t)d >> hist_bits), 1u);
-            }
-          }
-          for (; j < cnt; j += 32) {
-            const int32_t a = __ldg(src + j);
-            out[wpos + j] = a;
-            if (hist) atomicAdd(wc + ((uint32_t)a >> hist_bits), 1u);
-          }
-          wpos += cnt;
-        }
-      }
-      uint32_t mp = mov & ~min_;
-      const bool replay = MODE == kWrite && moff != kNoMask;  // hit bits cached by the count pass
-      if constexpr (PF) {
-        if (!replay) {
-          // listed for the prefetch ring below
-          if ((mp >> lane) & 1u) plist[npart + __popc(mp & lane_lt_mask())] = (uint8_t)(lb - l0 + lane);
-          npart += __popc(mp);
-          mp = 0;
-        }
-      }
-      // partially covered leaves: test every object, or replay its hit bits
-      uint32_t jl = 0;  // index of the leaf among the group's partial leaves
-      while (mp) {
-        const int s = __ffs(mp) - 1;
-        mp &= mp - 1;
+    uint32_t todo = __ballot_sync(0xffffffffu, r.w != 0);
+    if (!todo) continue;
+    do {
+      const uint32_t sl = __ffs(todo) - 1;
+      todo &= todo - 1;
+      const uint32_t mov = __shfl_sync(0xffffffffu, r.x, sl), mcov = __shfl_sync(0xffffffffu, r.y, sl);
+      const uint32_t moff = __shfl_sync(0xffffffffu, r.z, sl);
+      uint64_t wpos = __shfl_sync(0xffffffffu, at, sl);
+      const uint64_t lb = (uint64_t)it.y * F + (gbase + sl) * 32;  // the group's first leaf
+      uint32_t m = mcov;
+      while (m) {
+        // a run of consecutive covered leaves is one contiguous id range
+        const int s = __ffs(m) - 1;
+        const uint32_t shifted = ~(m >> s);
+        const int len = shifted ? (__ffs(shifted) - 1) : (32 - s);
+        m &= ~((len >= 32 ? 0xffffffffu : ((1u << len) - 1u)) << s);
         const uint64_t e0 = (lb + s) * F;
-        const uint32_t* mw = (moff != kNoMask) ? hc.mask + moff + jl * wpl : nullptr;
-        ++jl;
-        for (uint32_t g0 = 0; g0 < F; g0 += 128) {  // warp-uniform trip count
-          const uint32_t g = g0 + lane * 4;
-          const uint64_t p = e0 + g;
-          uint32_t hm;
-          if (replay) {
-            const uint4 w = *reinterpret_cast<const uint4*>(mw + (g0 >> 5));
-            hm = ((w.x >> lane) & 1u) | (((w.y >> lane) & 1u) << 1) | (((w.z >> lane) & 1u) << 2) |
-                 (((w.w >> lane) & 1u) << 3);
-          } else {
-            hm = (g < F) ? test4<D, RECT>(b, t.coords, t.npad, p, t.n) : 0u;
-          }
-          if (MODE == kCount) {
-            hits += __popc(hm);
-            if (mw) {
-              const uint32_t b0 = __ballot_sync(0xffffffffu, hm & 1u), b1 = __ballot_sync(0xffffffffu, hm & 2u);
-              const uint32_t b2 = __ballot_sync(0xffffffffu, hm & 4u), b3 = __ballot_sync(0xffffffffu, hm & 8u);
-              if (lane == 0) *reinterpret_cast<uint4*>(const_cast<uint32_t*>(mw) + (g0 >> 5)) = make_uint4(b0, b1, b2, b3);
-            }
-          } else {
-            uint32_t tot;
-            const uint32_t ex = warp_excl_sum(__popc(hm), &tot);
-            if (hm) {
-              const int4 idv = __ldg(reinterpret_cast<const int4*>(t.ids + p));
-              uint64_t o = wpos + ex;
-              if (hm & 1u) out[o++] = idv.x;
-              if (hm & 2u) out[o++] = idv.y;
-              if (hm & 4u) out[o++] = idv.z;
-              if (hm & 8u) out[o++] = idv.w;
-              if (hist) {
-                if (hm & 1u) atomicAdd(wc + ((uint32_t)idv.x >> hist_bits), 1u);
-                if (hm & 2u) atomicAdd(wc + ((uint32_t)idv.y >> hist_bits), 1u);
-                if (hm & 4u) atomicAdd(wc + ((uint32_t)idv.z >> hist_bits), 1u);
-                if (hm & 8u) atomicAdd(wc + ((uint32_t)idv.w >> hist_bits), 1u);
-              }
-            }
-            wpos += tot;
-          }
-        }
-      }
-    }
-    // ring path of the count pass with the cache: room for the hit bits of
-    // the item's listed leaves (list order = group order); lane g records
-    // group g
-    uint32_t ring_moff = kNoMask;
-    if (PF && MODE == kCount && cache) {
-      const uint32_t ngroups = (uint32_t)((l1 - l0 + 31) >> 5);
-      const uint32_t np = lane < ngroups ? __popc(g_mov & ~g_min) : 0u;
-      uint32_t tot;
-      const uint32_t before = warp_excl_sum(np, &tot);
-      if (tot) ring_moff = mask_alloc(tot * wpl);
-      if (lane < ngroups) {
-        grec[lane * kGrpWords + 0] = g_mov;
-        grec[lane * kGrpWords + 1] = g_min;
-        grec[lane * kGrpWords + 2] = (np && ring_moff != kNoMask) ? ring_moff + before * wpl : kNoMask;
-      }
-    }
-    if (PF && npart) {
-      // partially covered leaves through the ring: leaf k of the list goes
-      // to buffer k % nbuf, nbuf leaves ahead of the one being tested
-      __syncwarp();  // the list is complete
-      const uint32_t run_bytes = F * 4u;
-      // one lane arms the buffer's barrier and issues the leaf's NR copies;
-      // the warp's reads of the buffer's previous leaf are done (they fed
-      // the tests before this point, and the syncwarp orders every lane's)
-      auto issue = [&](uint32_t k, uint32_t bb) {
-        __syncwarp();
-        if (lane == 0) {
-          const uint64_t leaf = l0 + plist[k];
-          float* dst = bufs + (size_t)bb * buf_floats;
-          mbar_arrive_expect_tx(&bars[bb], NR * run_bytes);
+        uint64_t e1 = (lb + s + len) * F;
+        if (e1 > t.n) e1 = t.n;
+        const int32_t* src = t.ids + e0;
+        const uint32_t cnt = (uint32_t)(e1 - e0);
+        int32_t* dst = out + wpos;
+        // eight loads in flight per lane before their stores
+        uint32_t j = lane;
+        for (; j + 224 < cnt; j += 256) {
+          int32_t v[8];
 #pragma unroll
-          for (uint32_t r = 0; r < NC; ++r)
-            bulk_copy_g2s(dst + r * F, t.coords + (uint64_t)r * t.npad + leaf * F, run_bytes, &bars[bb]);
-          if (NR > NC) bulk_copy_g2s(dst + NC * F, t.ids + leaf * F, run_bytes, &bars[bb]);
-        }
-        pending |= 1u << bb;
-      };
-      const uint32_t pre = npart < nbuf ? npart : nbuf;
-      for (uint32_t k = 0; k < pre; ++k) issue(k, k);
-      uint32_t bb = 0;
-      for (uint32_t k = 0; k < npart; ++k) {
-        const bool ok = __all_sync(0xffffffffu, mbar_wait_bounded(&bars[bb], (phase >> bb) & 1u));
-        if (!ok) {
-          dead = true;
-          break;
-        }
-        phase ^= 1u << bb;
-        pending &= ~(1u << bb);
-        const float* sb = bufs + (size_t)bb * buf_floats;
-        const uint64_t e0 = (l0 + plist[k]) * F;
-        const uint32_t valid = (t.n > e0) ? (uint32_t)min((uint64_t)F, t.n - e0) : 0u;
-        for (uint32_t g0 = 0; g0 < F; g0 += 128) {  // warp-uniform trip count
-          const uint32_t g = g0 + lane * 4;
-          const uint32_t hm = (g < F) ? test4_staged<D, RECT>(b, sb, F, g, valid) : 0u;
-          if (MODE == kCount) {
-            hits += __popc(hm);
-            if (ring_moff != kNoMask) {
-              const uint32_t b0 = __ballot_sync(0xffffffffu, hm & 1u), b1 = __ballot_sync(0xffffffffu, hm & 2u);
-              const uint32_t b2 = __ballot_sync(0xffffffffu, hm & 4u), b3 = __ballot_sync(0xffffffffu, hm & 8u);
-              if (lane == 0)
-                *reinterpret_cast<uint4*>(hc.mask + ring_moff + k * wpl + (g0 >> 5)) = make_uint4(b0, b1, b2, b3);
-            }
-          } else {
-            uint32_t tot;
-            const uint32_t ex = warp_excl_sum(__popc(hm), &tot);
-            if (hm) {
-              const int4 idv = *reinterpret_cast<const int4*>(sb + NC * F + g);
-              uint64_t o = wpos + ex;
-              if (hm & 1u) out[o++] = idv.x;
-              if (hm & 2u) out[o++] = idv.y;
-              if (hm & 4u) out[o++] = idv.z;
-              if (hm & 8u) out[o++] = idv.w;
-              if (hist) {
-                if (hm & 1u) atomicAdd(wc + ((uint32_t)idv.x >> hist_bits), 1u);
-                if (hm & 2u) atomicAdd(wc + ((uint32_t)idv.y >> hist_bits), 1u);
-                if (hm & 4u) atomicAdd(wc + ((uint32_t)idv.z >> hist_bits), 1u);
-                if (hm & 8u) atomicAdd(wc + ((uint32_t)idv.w >> hist_bits), 1u);
-              }
-            }
-            wpos += tot;
+          for (int k = 0; k < 8; ++k) v[k] = __ldg(src + j + 32 * k);
+#pragma unroll
+          for (int k = 0; k < 8; ++k) dst[j + 32 * k] = v[k];
+          if (hist) {
+#pragma unroll
+            for (int k = 0; k < 8; ++k) atomicAdd(wc + ((uint32_t)v[k] >> hist_bits), 1u);
           }
         }
-        if (k + nbuf < npart) issue(k + nbuf, bb);
-        bb = (bb + 1 == nbuf) ? 0u : bb + 1;
+        for (; j + 96 < cnt; j += 128) {
+          int32_t v[4];
+#pragma unroll
+          for (int k = 0; k < 4; ++k) v[k] = __ldg(src + j + 32 * k);
+#pragma unroll
+          for (int k = 0; k < 4; ++k) dst[j + 32 * k] = v[k];
+          if (hist) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) atomicAdd(wc + ((uint32_t)v[k] >> hist_bits), 1u);
+          }
+        }
+        for (; j < cnt; j += 32) {
+          const int32_t a = __ldg(src + j);
+          dst[j] = a;
+          if (hist) atomicAdd(wc + ((uint32_t)a >> hist_bits), 1u);
+        }
+        wpos += cnt;
       }
-      if (dead) break;
-    }
+      // partially covered leaves: chunk c of the group's list is 128 objects
+      // of its (c / cpl)-th leaf; its hit bits are the bytes of the words at
+      // moff + kChunkWords c, or are found by testing the objects
+      uint32_t mp = mov & ~mcov;
+      const uint32_t nchunk = __popc(mp) * cpl;
+      const bool cached = moff != kNoMask;
+      uint32_t sub = 0;  // chunk of the leaf at mp's lowest bit
+      const uint8_t* hb = reinterpret_cast<const uint8_t*>(hmask + moff) + lane;
+      for (uint32_t c0 = 0; c0 < nchunk; c0 += kWriteUnroll) {
+        uint32_t hm[kWriteUnroll];
+        int4 idv[kWriteUnroll];
+        if (cached) {
+#pragma unroll
+          for (uint32_t u = 0; u < kWriteUnroll; ++u)
+            hm[u] = c0 + u < nchunk ? __ldg(hb + (c0 + u) * (kChunkWords * 4)) : 0u;
+        }
+#pragma unroll
+        for (uint32_t u = 0; u < kWriteUnroll; ++u) {
+          idv[u] = make_int4(0, 0, 0, 0);
+          if (!cached) hm[u] = 0;
+          if (c0 + u >= nchunk) continue;  // warp-uniform
+          const uint32_t o = sub * 128 + lane * 4;
+          const uint64_t p = (lb + (__ffs(mp) - 1)) * F + o;
+          if (++sub == cpl) {
+            sub = 0;
+            mp &= mp - 1;
+          }
+          if (!cached && o < F)
+            hm[u] = test4_rolled<D, RECT>(boxes + (uint64_t)it.x * (2 * D), t.coords, t.npad, p, t.n);
+          if (hm[u]) idv[u] = __ldg(reinterpret_cast<const int4*>(t.ids + p));
+        }
+#pragma unroll
+        for (uint32_t u = 0; u < kWriteUnroll; ++u) {
+          const int32_t ids[4] = {idv[u].x, idv[u].y, idv[u].z, idv[u].w};
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const bool on = (hm[u] >> k) & 1u;
+            const uint32_t w = __ballot_sync(0xffffffffu, on);
+            if (on) {
+              out[wpos + __popc(w & lt)] = ids[k];
+              if (hist) atomicAdd(wc + ((uint32_t)ids[k] >> hist_bits), 1u);
+            }
+            wpos += __popc(w);
+          }
+        }
+      }
+    } while (todo);
     if (hist) {
       __syncwarp();
       for (uint32_t w = lane; w < hist_G; w += 32) {
@@ -485,29 +735,6 @@ __global__ void __launch_bounds__(256) k_leafscan(TreeView t, const float* __res
       }
       __syncwarp();
     }
-    if (MODE == kCount) {
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        hits += __shfl_xor_sync(0xffffffffu, hits, o);
-        n_cov += __shfl_xor_sync(0xffffffffu, n_cov, o);
-        n_part += __shfl_xor_sync(0xffffffffu, n_part, o);
-        o_cov += __shfl_xor_sync(0xffffffffu, o_cov, o);
-      }
-      if (lane == 0) {
-        item_hits[i] = hits;
-        if (hits) atomicAdd(qcount + it.x, (unsigned long long)hits);
-        if (n_cov) atomicAdd(stats + kStatCovered, (unsigned long long)n_cov);
-        if (n_part) atomicAdd(stats + kStatPartial, (unsigned long long)n_part);
-        if (o_cov) atomicAdd(stats + kStatObjCovered, (unsigned long long)o_cov);
-      }
-    }
-  }
-  if (PF && dead) {
-    if (lane == 0) atomicOr(err, 1u);
-    // copies still in flight land in this warp's ring: wait for them (again
-    // bounded) before the CTA's shared memory goes away
-    for (uint32_t bb = 0; bb < nbuf; ++bb)
-      if ((pending >> bb) & 1u) mbar_wait_bounded(&bars[bb], (phase >> bb) & 1u);
   }
 }
 
@@ -644,75 +871,56 @@ __global__ void k_gate_zero(unsigned long long* offsets, uint32_t q, const uint3
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i <= q; i += gridDim.x * blockDim.x) offsets[i] = 0;
 }
 
+// in == nullptr: the root level of nroot queries.
 template <int D>
 void launch_expand(uint32_t grid, cudaStream_t s, const float* boxes, const uint2* in,
-                   const uint32_t* in_count, uint2* out, uint32_t* out_count, uint64_t cap,
+                   const uint32_t* in_count, uint32_t nroot, uint2* out, uint32_t* out_count, uint64_t cap,
                    const float* child_mbr, uint64_t nchild, uint64_t child_pad, uint32_t fanout,
                    uint32_t* overflow, uint32_t* need, uint32_t lanes = 32) {
   if (lanes == 8)
-    k_expand<D, 8><<<grid, 256, 0, s>>>(boxes, in, in_count, out, out_count, cap, child_mbr, nchild, child_pad,
+    k_expand<D, 8><<<grid, 256, 0, s>>>(boxes, in, in_count, nroot, out, out_count, cap, child_mbr, nchild, child_pad,
                                         fanout, overflow, need);
   else if (lanes == 16)
-    k_expand<D, 16><<<grid, 256, 0, s>>>(boxes, in, in_count, out, out_count, cap, child_mbr, nchild, child_pad,
-                                         fanout, overflow, need);
+    k_expand<D, 16><<<grid, 256, 0, s>>>(boxes, in, in_count, nroot, out, out_count, cap, child_mbr, nchild,
+                                         child_pad, fanout, overflow, need);
   else
-    k_expand<D, 32><<<grid, 256, 0, s>>>(boxes, in, in_count, out, out_count, cap, child_mbr, nchild, child_pad,
-                                         fanout, overflow, need);
+    k_expand<D, 32><<<grid, 256, 0, s>>>(boxes, in, in_count, nroot, out, out_count, cap, child_mbr, nchild,
+                                         child_pad, fanout, overflow, need);
 }
 
-// Ring buffers per warp that fit the leaf prefetch of this launch: at most
-// `want` (kRingMaxBuf), fewer when eight warps' rings would not leave room
-// for two CTAs per SM; 0 = no ring (direct loads).
-inline uint32_t ring_buffers(uint32_t runs, uint32_t F, uint32_t want) {
-  if (want < 2) return 0;
-  uint32_t nb = want > kRingMaxBuf ? kRingMaxBuf : want;
-  while (nb >= 2 && 8u * ring_warp_bytes(runs, F, nb) > 100u * 1024u) --nb;
-  return nb >= 2 ? nb : 0;
+// The count pass.  nodes == 0: k_count; otherwise the level-1 nodes of a batch
+// that order_items has been over: k_count and k_join, one of which finds the
+// batch to be the other's.  At most blocks_per_sm CTAs of 256 threads per SM
+// (k_join's have 128), and no more of k_join's than are resident (its run
+// length follows from the grid).
+template <int D>
+qcp_status launch_count(bool rect, uint64_t nodes, uint32_t blocks_per_sm, cudaStream_t s, const TreeView& t,
+                        const float* boxes, const uint2* items, const uint32_t* item_count, uint32_t* work,
+                        uint64_t* qcount, uint64_t item_cap, unsigned long long* stats, HitCache hc) {
+  auto* count = rect ? k_count<D, true> : k_count<D, false>;
+  count<<<(uint32_t)num_sms() * blocks_per_sm, 256, 0, s>>>(t, boxes, items, item_count, (unsigned long long*)qcount,
+                                                            item_cap, nodes, stats, hc);
+  note_launch();
+  QCP_TRY(check_launch("k_count"));
+  if (!nodes) return QCP_OK;
+  auto* join = rect ? k_join<D, true> : k_join<D, false>;
+  int fit = 0;
+  QCP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, join, kJoinThreads, 0));
+  const uint32_t per_sm = fit < 1 ? 1u : ((uint32_t)fit < 2 * blocks_per_sm ? (uint32_t)fit : 2 * blocks_per_sm);
+  join<<<(uint32_t)num_sms() * per_sm, kJoinThreads, 0, s>>>(t, boxes, items, item_count, work,
+                                                             (unsigned long long*)qcount, item_cap, nodes, stats, hc);
+  note_launch();
+  return check_launch("k_join");
 }
 
-template <int D, bool RECT, int MODE>
-void launch_leafscan_t(uint32_t grid, cudaStream_t s, const TreeView& t, const float* boxes, const uint2* items,
-                       const uint32_t* item_count, uint32_t* work, uint32_t* item_hits, uint64_t* qcount,
-                       const uint64_t* offsets, uint64_t* qcursor, int32_t* out, uint64_t item_cap,
-                       unsigned long long* stats, uint32_t* qwhist, uint32_t hist_G, uint32_t hist_bits,
-                       uint32_t ring, uint32_t* err, HitCache hc) {
-  const uint32_t nb = ring_buffers(leaf_runs(D, RECT, MODE), t.fanout, ring);
-  // the hit-cache code costs registers (occupancy of a latency-bound pass):
-  // calls without a cache run an instantiation without it
-  if (nb) {
-    const size_t smem = 8u * (size_t)ring_warp_bytes(leaf_runs(D, RECT, MODE), t.fanout, nb);
-    auto* kern = hc.grp ? k_leafscan<D, RECT, MODE, true, true> : k_leafscan<D, RECT, MODE, true, false>;
-    if (smem > 48u * 1024u) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    // no more CTAs than fit on the SMs at once (the static counters and 1 KB
-    // per CTA of reserved shared memory included)
-    const size_t per_cta = smem + sizeof(uint32_t) * 8 * (MODE == kWrite ? kHistMaxG : 1) + 1024;
-    const uint32_t fit = (uint32_t)((228u * 1024u) / per_cta);
-    const uint32_t sms = (uint32_t)num_sms();
-    if (fit >= 1 && grid > sms * fit) grid = sms * fit;
-    kern<<<grid, 256, smem, s>>>(t, boxes, items, item_count, work, item_hits, (unsigned long long*)qcount,
-                                 (const unsigned long long*)offsets, (unsigned long long*)qcursor, out, item_cap,
-                                 stats, qwhist, hist_G, hist_bits, nb, err, hc);
-  } else {
-    auto* kern = hc.grp ? k_leafscan<D, RECT, MODE, false, true> : k_leafscan<D, RECT, MODE, false, false>;
-    kern<<<grid, 256, 0, s>>>(t, boxes, items, item_count, work, item_hits, (unsigned long long*)qcount,
-                              (const unsigned long long*)offsets, (unsigned long long*)qcursor, out, item_cap, stats,
-                              qwhist, hist_G, hist_bits, 0u, err, hc);
-  }
-}
-
-template <int D, int MODE>
-void launch_leafscan(bool rect, uint32_t grid, cudaStream_t s, const TreeView& t, const float* boxes,
-                     const uint2* items, const uint32_t* item_count, uint32_t* work,
-                     uint32_t* item_hits, uint64_t* qcount, const uint64_t* offsets,
-                     uint64_t* qcursor, int32_t* out, uint64_t item_cap,
-                     unsigned long long* stats, uint32_t* qwhist, uint32_t hist_G,
-                     uint32_t hist_bits, uint32_t ring, uint32_t* err, HitCache hc = HitCache{}) {
-  if (rect)
-    launch_leafscan_t<D, true, MODE>(grid, s, t, boxes, items, item_count, work, item_hits, qcount, offsets, qcursor,
-                                     out, item_cap, stats, qwhist, hist_G, hist_bits, ring, err, hc);
-  else
-    launch_leafscan_t<D, false, MODE>(grid, s, t, boxes, items, item_count, work, item_hits, qcount, offsets,
-                                      qcursor, out, item_cap, stats, qwhist, hist_G, hist_bits, ring, err, hc);
+template <int D>
+void launch_leafwrite(bool rect, uint32_t grid, cudaStream_t s, const TreeView& t, const float* boxes,
+                      const uint2* items, const uint32_t* item_count, uint32_t* work, const HitCache& hc,
+                      const uint64_t* offsets, uint64_t* qcursor, int32_t* out, uint64_t item_cap, uint32_t* qwhist,
+                      uint32_t hist_G, uint32_t hist_bits) {
+  auto* kern = rect ? k_leafwrite<D, true> : k_leafwrite<D, false>;
+  kern<<<grid, 256, 0, s>>>(t, boxes, items, item_count, work, hc.rec, hc.mask, (const unsigned long long*)offsets,
+                            (unsigned long long*)qcursor, out, item_cap, qwhist, hist_G, hist_bits);
 }
 
 template <int D, int MODE>
@@ -741,12 +949,15 @@ qcp_status init_items(Workspace* ws, uint32_t q, cudaStream_t s) {
   return QCP_OK;
 }
 
-qcp_status expand_level(qcp_index* ix, Workspace* ws, uint32_t l, int cur, cudaStream_t s) {
+// Items of level l (the root's: nroot queries, when cur < 0) in items[cur] ->
+// items of level l - 1 in items[nxt].
+static qcp_status expand_level(qcp_index* ix, Workspace* ws, uint32_t l, int cur, int nxt, uint32_t nroot,
+                               cudaStream_t s) {
   const TreeView t = view_of(ix);
   const uint32_t grid = (uint32_t)num_sms() * ws->blocks_per_sm;
-  const int nxt = cur ^ 1;
   uint32_t* ctr = ws->ctr;
-  QCP_DISPATCH_D(ix->dims, launch_expand<DD>(grid, s, ws->boxes, ws->items[cur], ctr + kCtrFrontier0 + cur,
+  QCP_DISPATCH_D(ix->dims, launch_expand<DD>(grid, s, ws->boxes, cur < 0 ? nullptr : ws->items[cur],
+                                             ctr + kCtrFrontier0 + (cur < 0 ? 0 : cur), nroot,
                                              ws->items[nxt], ctr + kCtrFrontier0 + nxt, ws->items_cap,
                                              t.mbr[l - 1], t.nodes[l - 1], t.pad[l - 1], t.fanout,
                                              ctr + kCtrOverflow, ctr + kCtrNeedItems, ws->lanes_per_item));
@@ -754,79 +965,125 @@ qcp_status expand_level(qcp_index* ix, Workspace* ws, uint32_t l, int cur, cudaS
   return check_launch("k_expand");
 }
 
-// The hit cache of this call (ws->use_hit_cache), or none.
-static HitCache hit_cache_of(Workspace* ws) {
-  if (!ws->use_hit_cache || !ws->item_grp || !ws->hmask) return HitCache{nullptr, nullptr, 0, nullptr};
-  return HitCache{ws->item_grp, ws->hmask, (uint32_t)(ws->hmask_cap > 0xfffffff0u ? 0xfffffff0u : ws->hmask_cap),
-                  ws->ctr + kCtrMaskWords};
+// Level-1 nodes of a batch whose items may be put in node order (four launches)
+// and counted by k_join, 0 for one that is not: many queries, and more leaves
+// than stay close to every warp anyway (the order alone is worth little:
+// 1 M points, 7,813 leaves, 10,000 boxes 105 us with it, 102 without; 103,699
+// rectangles, 2,502 boxes 39 and 15).  16 M points, 10,000 boxes: 306 us, 586
+// without; 64 M 2-D points 262, 377; 32 M 8-D rectangles 0.85 ms, 3.4.
+constexpr uint32_t kNodeOrderMinQueries = 1024;
+constexpr uint64_t kNodeOrderMinLeaves = 16384;
+
+static uint64_t order_nodes(const qcp_index* ix, uint32_t q) {
+  const bool may = q >= kNodeOrderMinQueries && ix->levels > 2 && ix->level_nodes[0] >= kNodeOrderMinLeaves &&
+                   q >= ix->level_nodes[1];
+  return may ? ix->level_nodes[1] : 0;
 }
 
-qcp_status write_items(qcp_index* ix, Workspace* ws, int cur, cudaStream_t s) {
+// The level-1 items in items[*cur] in node order, into the other buffer.
+static qcp_status order_items(qcp_index* ix, Workspace* ws, int* cur, cudaStream_t s) {
+  const uint32_t grid = (uint32_t)num_sms() * 8;
+  const int nxt = *cur ^ 1;
+  const uint64_t nodes = ix->level_nodes[1];
+  uint32_t* ctr = ws->ctr;
+  QCP_CUDA(cudaMemsetAsync(ws->node_hist, 0, sizeof(uint32_t) * nodes, s));
+  k_node_hist<<<grid, 256, 0, s>>>(ws->items[*cur], ctr + kCtrFrontier0 + *cur, ws->items_cap, nodes,
+                                   ws->node_hist);
+  uint32_t* cursor = ws->node_hist + nodes;
+  QCP_TRY(exclusive_scan<uint32_t>(ws->node_hist, cursor, nodes, nullptr, ix->pool, s, ws->scan_tmp,
+                                   ws->scan_tmp_cap));
+  k_node_scatter<<<grid, 256, 0, s>>>(ws->items[*cur], ctr + kCtrFrontier0 + *cur, ws->items_cap, nodes, cursor,
+                                      ws->items[nxt], ctr + kCtrFrontier0 + nxt);
+  note_launch(2);
+  *cur = nxt;
+  return check_launch("order_items");
+}
+
+// What the count pass of this call records for its write pass.
+static HitCache hit_cache_of(Workspace* ws) {
+  const bool bits = ws->use_hit_cache && ws->hmask;
+  return HitCache{ws->item_grp, bits ? ws->hmask : nullptr,
+                  (uint32_t)(ws->hmask_cap > 0xfffffff0u ? 0xfffffff0u : ws->hmask_cap),
+                  reinterpret_cast<unsigned long long*>(ws->ctr + kCtrMaskWords)};
+}
+
+static qcp_status count_items(qcp_index* ix, Workspace* ws, uint32_t q, int cur, bool counts_only, cudaStream_t s) {
+  const TreeView t = view_of(ix);
+  uint32_t* ctr = ws->ctr;
+  const HitCache hc = counts_only ? HitCache{} : hit_cache_of(ws);
+  qcp_status st = QCP_OK;
+  QCP_DISPATCH_D(ix->dims, st = launch_count<DD>(ix->is_rect != 0, order_nodes(ix, q), ws->blocks_per_sm, s, t, ws->boxes, ws->items[cur],
+                                                ctr + kCtrFrontier0 + cur, ctr + kCtrWork, ws->qcount,
+                                                ws->items_cap, ws->timing ? ws->d_stats : nullptr, hc));
+  return st;
+}
+
+static qcp_status write_items(qcp_index* ix, Workspace* ws, int cur, cudaStream_t s) {
   const TreeView t = view_of(ix);
   const uint32_t grid = (uint32_t)num_sms() * ws->blocks_per_sm;
   uint32_t* ctr = ws->ctr;
-  QCP_DISPATCH_D(ix->dims, launch_leafscan<DD, kWrite>(ix->is_rect != 0, grid, s, t, ws->boxes, ws->items[cur],
-                                                       ctr + kCtrFrontier0 + cur, ctr + kCtrWork,
-                                                       ws->item_hits, nullptr, ws->offsets, ws->qcursor,
-                                                       ws->out_ids, ws->items_cap, ws->d_stats,
-                                                       ws->hist_G ? ws->qwhist : nullptr, ws->hist_G,
-                                                       ws->hist_bits, ws->leaf_ring, ctr + kCtrTimeout,
-                                                       hit_cache_of(ws)));
+  QCP_DISPATCH_D(ix->dims, launch_leafwrite<DD>(ix->is_rect != 0, grid, s, t, ws->boxes, ws->items[cur],
+                                                ctr + kCtrFrontier0 + cur, ctr + kCtrWork, hit_cache_of(ws),
+                                                ws->offsets, ws->qcursor, ws->out_ids, ws->items_cap,
+                                                ws->hist_G ? ws->qwhist : nullptr, ws->hist_G, ws->hist_bits));
   note_launch();
-  return check_launch("k_leafscan<write>");
+  return check_launch("k_leafwrite");
 }
 
 qcp_status run_batched(qcp_index* ix, Workspace* ws, uint32_t q, bool counts_only, bool sort,
                        cudaStream_t s) {
-  const TreeView t = view_of(ix);
-  const uint32_t D = ix->dims;
-  const bool rect = ix->is_rect != 0;
-  const uint32_t sms = (uint32_t)num_sms();
-  const uint32_t grid = sms * ws->blocks_per_sm;  // 256-thread blocks
   uint32_t* ctr = ws->ctr;
   // start level: items at level `start` are (query, node) pairs
   const uint32_t start = (ix->levels >= 2) ? ix->levels - 1 : 1;
+  const bool order = order_nodes(ix, q) != 0;
+  if (order) QCP_TRY(ws_reserve_nodes(ws, ix->level_nodes[1]));
   ws->use_hit_cache = false;
   for (int attempt = 0; attempt < 8; ++attempt) {
     mark(ws, kEvStart, s);
     QCP_CUDA(cudaMemsetAsync(ctr, 0, sizeof(uint32_t) * kCtrCount, s));
-    QCP_CUDA(cudaMemsetAsync(ws->d_stats, 0, sizeof(unsigned long long) * kStatCount, s));
     QCP_CUDA(cudaMemsetAsync(ws->qcount, 0, sizeof(uint64_t) * q, s));
+    if (ws->timing) QCP_CUDA(cudaMemsetAsync(ws->d_stats, 0, sizeof(unsigned long long) * kStatCount, s));
     // the GPU's first level: the root's, or the hand-off level of a CPU + GPU
     // co-processing call whose host threads walked the levels above
     uint32_t gpu_start = start;
     if (ws->hybrid) {
       gpu_start = ws->handoff_level < 1 ? 1u : (ws->handoff_level > start ? start : ws->handoff_level);
     }
+    // frontier sizes of the levels (kStatLevel0 slots), for timed calls
+    auto note_level = [&](uint32_t l, int slot) -> qcp_status {
+      if (ws->timing)
+        QCP_CUDA(cudaMemcpyAsync(ws->d_stats + kStatLevel0 + l, ctr + kCtrFrontier0 + slot, sizeof(uint32_t),
+                                 cudaMemcpyDeviceToDevice, s));
+      return QCP_OK;
+    };
+    int cur = 0;
+    bool root = false;  // the next expansion starts from the root's implied items
     if (gpu_start < start) {
       QCP_TRY(host_frontier(ix, ws, q, gpu_start, s));
-    } else {
+    } else if (gpu_start == 1 || ws->timing) {
       QCP_TRY(init_items(ws, q, s));
+    } else {
+      root = true;
     }
-    QCP_CUDA(cudaMemcpyAsync(ws->d_stats + kStatLevel0 + gpu_start, ctr + kCtrFrontier0, sizeof(uint32_t),
-                             cudaMemcpyDeviceToDevice, s));
-    int cur = 0;
+    if (!root) QCP_TRY(note_level(gpu_start, cur));
+    const uint32_t held = root ? gpu_start - 1 : gpu_start;  // first level whose items are in a buffer
     for (uint32_t l = gpu_start; l > 1; --l) {
-      const int nxt = cur ^ 1;
-      QCP_CUDA(cudaMemsetAsync(ctr + kCtrFrontier0 + nxt, 0, sizeof(uint32_t), s));
-      QCP_TRY(expand_level(ix, ws, l, cur, s));
-      QCP_CUDA(cudaMemcpyAsync(ws->d_stats + kStatLevel0 + (l - 1), ctr + kCtrFrontier0 + nxt,
-                               sizeof(uint32_t), cudaMemcpyDeviceToDevice, s));
+      const int nxt = root ? 0 : cur ^ 1;
+      // (from then on the output counter is that of the items of two levels up)
+      if (l < held) QCP_CUDA(cudaMemsetAsync(ctr + kCtrFrontier0 + nxt, 0, sizeof(uint32_t), s));
+      QCP_TRY(expand_level(ix, ws, l, root ? -1 : cur, nxt, q, s));
+      QCP_TRY(note_level(l - 1, nxt));
       cur = nxt;
+      root = false;
     }
+    if (order) QCP_TRY(order_items(ix, ws, &cur, s));
     mark(ws, kEvExpand, s);
-    // the level-1 items must fit the per-item hit array too
-    QCP_TRY(ws_reserve_items(ix, ws, 0));
     // a call that writes ids keeps the count pass's hits for the write pass
     ws->use_hit_cache = !counts_only && ws->hit_cache_on;
-    if (ws->use_hit_cache) QCP_TRY(ws_reserve_hitcache(ws, ws->items_cap, ws->hmask_cap ? 0 : (size_t)1 << 20));
-    QCP_DISPATCH_D(D, launch_leafscan<DD, kCount>(rect, grid, s, t, ws->boxes, ws->items[cur],
-                                                  ctr + kCtrFrontier0 + cur, ctr + kCtrWork,
-                                                  ws->item_hits, ws->qcount, nullptr, nullptr, nullptr,
-                                                  ws->items_cap, ws->d_stats, nullptr, 0, 0, ws->leaf_ring,
-                                                  ctr + kCtrTimeout, hit_cache_of(ws)));
-    note_launch();
-    QCP_TRY(check_launch("k_leafscan<count>"));
+    if (!counts_only)
+      QCP_TRY(ws_reserve_hitcache(ws, ws->items_cap * (ix->fanout / 32),
+                                  ws->use_hit_cache && !ws->hmask_cap ? (size_t)1 << 21 : 0));
+    QCP_TRY(count_items(ix, ws, q, cur, counts_only, s));
     mark(ws, kEvCount, s);
     QCP_TRY(exclusive_scan_counts(ws->qcount, ws->offsets, q, ix->pool, s));
     mark(ws, kEvScan, s);
@@ -834,10 +1091,6 @@ qcp_status run_batched(qcp_index* ix, Workspace* ws, uint32_t q, bool counts_onl
     QCP_CUDA(cudaMemcpyAsync(ws->h_ctr, ctr, sizeof(uint32_t) * kCtrCount, cudaMemcpyDeviceToHost, s));
     QCP_CUDA(cudaMemcpyAsync(ws->h_total, ws->offsets + q, sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
     QCP_CUDA(cudaStreamSynchronize(s));
-    if (ws->h_ctr[kCtrTimeout]) {
-      set_error("a bounded wait for a leaf's bulk copy ran out in the count pass");
-      return QCP_ERR_TIMEOUT;
-    }
     if (ws->h_ctr[kCtrOverflow]) {
       size_t need = (size_t)ws->h_ctr[kCtrNeedItems];
       if (need < ws->items_cap * 2) need = ws->items_cap * 2;
@@ -865,21 +1118,24 @@ qcp_status run_batched(qcp_index* ix, Workspace* ws, uint32_t q, bool counts_onl
       mark(ws, kEvWrite, s);
       if (sort) QCP_TRY(segmented_sort(ix, ws, q, s));
       mark(ws, kEvSort, s);
-      // bounded waits of the write pass's leaf ring and the window sort's
-      // bulk prefetch
+      // bounded waits of the window sort's bulk prefetch
       QCP_CUDA(cudaMemcpyAsync(ws->h_ctr + kCtrTimeout, ctr + kCtrTimeout, sizeof(uint32_t),
                                cudaMemcpyDeviceToHost, s));
       QCP_CUDA(cudaStreamSynchronize(s));
       if (ws->h_ctr[kCtrTimeout]) {
-        set_error("a bounded wait for a bulk copy ran out in the write pass or the sort");
+        set_error("a bounded wait for a bulk copy ran out in the sort");
         return QCP_ERR_TIMEOUT;
       }
     }
     // hit bits that did not fit this call were tested again by the write
     // pass; the next call gets room for them (after this call's passes)
-    if (ws->use_hit_cache && ws->h_ctr[kCtrMaskWords] > ws->hmask_cap) {
-      QCP_CUDA(cudaStreamSynchronize(s));
-      QCP_TRY(ws_reserve_hitcache(ws, 0, ws->h_ctr[kCtrMaskWords]));
+    if (ws->use_hit_cache) {
+      uint64_t words;
+      memcpy(&words, ws->h_ctr + kCtrMaskWords, sizeof(words));
+      if (words > ws->hmask_cap && ws->hmask_cap < kMaxMaskWords) {
+        QCP_CUDA(cudaStreamSynchronize(s));
+        QCP_TRY(ws_reserve_hitcache(ws, 0, (size_t)(words < kMaxMaskWords ? words : kMaxMaskWords)));
+      }
     }
     ws->use_hit_cache = false;
     return QCP_OK;
@@ -925,12 +1181,10 @@ qcp_status run_plain(qcp_index* ix, Workspace* ws, uint32_t q, bool counts_only,
 
 // Batched per-query hit counts into caller-provided device buffers (boxes,
 // counts) with scratch supplied by the caller as well: two frontier buffers
-// of item_cap items, item_cap per-item counts, kCtrCount counters and
-// kStatCount statistics words.  Nothing is allocated.  Returns
+// of item_cap items and kCtrCount counters.  Nothing is allocated.  Returns
 // QCP_ERR_OUTPUT_OVERFLOW when the batch's frontier exceeds item_cap.
 qcp_status run_batched_counts_into(qcp_index* ix, const float* boxes, uint32_t q, uint64_t* counts,
-                                   uint2* items0, uint2* items1, uint32_t* item_hits, size_t item_cap,
-                                   uint32_t* ctr, unsigned long long* stats, cudaStream_t s) {
+                                   uint2* items0, uint2* items1, size_t item_cap, uint32_t* ctr, cudaStream_t s) {
   const TreeView t = view_of(ix);
   const uint32_t D = ix->dims;
   const bool rect = ix->is_rect != 0;
@@ -938,25 +1192,26 @@ qcp_status run_batched_counts_into(qcp_index* ix, const float* boxes, uint32_t q
   uint2* items[2] = {items0, items1};
   const uint32_t start = (ix->levels >= 2) ? ix->levels - 1 : 1;
   QCP_CUDA(cudaMemsetAsync(ctr, 0, sizeof(uint32_t) * kCtrCount, s));
-  QCP_CUDA(cudaMemsetAsync(stats, 0, sizeof(unsigned long long) * kStatCount, s));
   QCP_CUDA(cudaMemsetAsync(counts, 0, sizeof(uint64_t) * q, s));
-  k_init_items<<<(q + 255) / 256, 256, 0, s>>>(items[0], q, 0, ctr + kCtrFrontier0);
-  note_launch();
   int cur = 0;
+  if (start == 1) {
+    k_init_items<<<(q + 255) / 256, 256, 0, s>>>(items[0], q, 0, ctr + kCtrFrontier0);
+    note_launch();
+  }
   for (uint32_t l = start; l > 1; --l) {
-    const int nxt = cur ^ 1;
-    QCP_CUDA(cudaMemsetAsync(ctr + kCtrFrontier0 + nxt, 0, sizeof(uint32_t), s));
-    QCP_DISPATCH_D(D, launch_expand<DD>(grid, s, boxes, items[cur], ctr + kCtrFrontier0 + cur, items[nxt],
-                                        ctr + kCtrFrontier0 + nxt, item_cap, t.mbr[l - 1], t.nodes[l - 1],
+    const bool root = l == start;
+    const int nxt = root ? 0 : cur ^ 1;
+    if (l + 1 < start) QCP_CUDA(cudaMemsetAsync(ctr + kCtrFrontier0 + nxt, 0, sizeof(uint32_t), s));
+    QCP_DISPATCH_D(D, launch_expand<DD>(grid, s, boxes, root ? nullptr : items[cur], ctr + kCtrFrontier0 + cur, q,
+                                        items[nxt], ctr + kCtrFrontier0 + nxt, item_cap, t.mbr[l - 1], t.nodes[l - 1],
                                         t.pad[l - 1], t.fanout, ctr + kCtrOverflow, ctr + kCtrNeedItems));
     note_launch();
     cur = nxt;
   }
-  QCP_DISPATCH_D(D, launch_leafscan<DD, kCount>(rect, grid, s, t, boxes, items[cur], ctr + kCtrFrontier0 + cur,
-                                                ctr + kCtrWork, item_hits, counts, nullptr, nullptr, nullptr,
-                                                item_cap, stats, nullptr, 0, 0, 0, ctr + kCtrTimeout));
-  note_launch();
-  QCP_TRY(check_launch("batched counts"));
+  qcp_status st = QCP_OK;
+  QCP_DISPATCH_D(D, st = launch_count<DD>(rect, 0, 8, s, t, boxes, items[cur], ctr + kCtrFrontier0 + cur,
+                                         ctr + kCtrWork, counts, item_cap, nullptr, HitCache{}));
+  QCP_TRY(st);
   uint32_t overflow = 0;  // pageable host word: no pinned buffer is allocated
   QCP_CUDA(cudaMemcpyAsync(&overflow, ctr + kCtrOverflow, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
   QCP_CUDA(cudaStreamSynchronize(s));
@@ -976,27 +1231,22 @@ qcp_status run_batched_counts_into(qcp_index* ix, const float* boxes, uint32_t q
 // Stream-capturable.
 qcp_status run_batched_device(qcp_index* ix, Workspace* ws, uint32_t q, uint64_t ids_cap, bool sort,
                               void* sort_tables, cudaStream_t s) {
-  const TreeView t = view_of(ix);
-  const uint32_t D = ix->dims;
-  const bool rect = ix->is_rect != 0;
-  const uint32_t grid = (uint32_t)num_sms() * ws->blocks_per_sm;
   uint32_t* ctr = ws->ctr;
   const uint32_t start = (ix->levels >= 2) ? ix->levels - 1 : 1;
-  ws->use_hit_cache = false;  // the captured pipeline tests every leaf in both passes
+  ws->use_hit_cache = ws->hmask != nullptr;
   QCP_CUDA(cudaMemsetAsync(ctr, 0, sizeof(uint32_t) * kCtrCount, s));
   QCP_CUDA(cudaMemsetAsync(ws->qcount, 0, sizeof(uint64_t) * q, s));
-  QCP_TRY(init_items(ws, q, s));
   int cur = 0;
+  if (start == 1) QCP_TRY(init_items(ws, q, s));
   for (uint32_t l = start; l > 1; --l) {
-    QCP_CUDA(cudaMemsetAsync(ctr + kCtrFrontier0 + (cur ^ 1), 0, sizeof(uint32_t), s));
-    QCP_TRY(expand_level(ix, ws, l, cur, s));
-    cur ^= 1;
+    const bool root = l == start;
+    const int nxt = root ? 0 : cur ^ 1;
+    if (l + 1 < start) QCP_CUDA(cudaMemsetAsync(ctr + kCtrFrontier0 + nxt, 0, sizeof(uint32_t), s));
+    QCP_TRY(expand_level(ix, ws, l, root ? -1 : cur, nxt, q, s));
+    cur = nxt;
   }
-  QCP_DISPATCH_D(D, launch_leafscan<DD, kCount>(rect, grid, s, t, ws->boxes, ws->items[cur],
-                                                ctr + kCtrFrontier0 + cur, ctr + kCtrWork, ws->item_hits,
-                                                ws->qcount, nullptr, nullptr, nullptr, ws->items_cap,
-                                                ws->d_stats, nullptr, 0, 0, ws->leaf_ring, ctr + kCtrTimeout));
-  note_launch();
+  if (order_nodes(ix, q)) QCP_TRY(order_items(ix, ws, &cur, s));
+  QCP_TRY(count_items(ix, ws, q, cur, false, s));
   QCP_TRY(exclusive_scan_counts(ws->qcount, ws->offsets, q, ix->pool, s, ws->scan_tmp, ws->scan_tmp_cap));
   k_gate<<<1, 32, 0, s>>>((const unsigned long long*)ws->offsets, q, ids_cap, ctr + kCtrFrontier0 + cur,
                           ctr + kCtrOverflow);

@@ -64,43 +64,27 @@ __device__ __forceinline__ void test_node(const Box<D>& b, const float* mbr, uin
   }
 }
 
-// Hit mask of 4 consecutive objects starting at position p (p % 4 == 0).
+// Hit mask of 4 consecutive objects starting at position p (p % 4 == 0)
+// against the box at b, one dimension at a time (few registers: the fallback
+// of a pass that otherwise tests nothing).
 template <int D, bool RECT>
-__device__ __forceinline__ uint32_t test4(const Box<D>& b, const float* coords, uint64_t npad, uint64_t p,
-                                          uint64_t n) {
+__device__ __forceinline__ uint32_t test4_rolled(const float* b, const float* coords, uint64_t npad, uint64_t p,
+                                                 uint64_t n) {
   uint32_t m = 0xfu;
-#pragma unroll
+#pragma unroll 1
   for (int d = 0; d < D; ++d) {
+    const float blo = __ldg(b + d), bhi = __ldg(b + D + d);
     const float4 lo = __ldg(reinterpret_cast<const float4*>(coords + (uint64_t)d * npad + p));
     float4 hi = lo;
     if (RECT) hi = __ldg(reinterpret_cast<const float4*>(coords + (uint64_t)(D + d) * npad + p));
-    m &= (overlaps1(b.lo[d], b.hi[d], lo.x, hi.x) ? 1u : 0u) | (overlaps1(b.lo[d], b.hi[d], lo.y, hi.y) ? 2u : 0u) |
-         (overlaps1(b.lo[d], b.hi[d], lo.z, hi.z) ? 4u : 0u) | (overlaps1(b.lo[d], b.hi[d], lo.w, hi.w) ? 8u : 0u);
+    m &= (overlaps1(blo, bhi, lo.x, hi.x) ? 1u : 0u) | (overlaps1(blo, bhi, lo.y, hi.y) ? 2u : 0u) |
+         (overlaps1(blo, bhi, lo.z, hi.z) ? 4u : 0u) | (overlaps1(blo, bhi, lo.w, hi.w) ? 8u : 0u);
   }
   // objects past n (padding of the last leaf) never hit
   if (p + 4 > n) {
     const uint64_t valid = (n > p) ? (n - p) : 0;
     m &= (1u << valid) - 1u;
   }
-  return m;
-}
-
-// Hit mask of objects g..g+3 of a leaf staged in shared memory: coordinate
-// run c of the leaf at s + c * F (lo0..lo(D-1), then hi.. for rectangles);
-// objects at or past `valid` (padding of the last leaf) never hit.
-template <int D, bool RECT>
-__device__ __forceinline__ uint32_t test4_staged(const Box<D>& b, const float* s, uint32_t F, uint32_t g,
-                                                 uint32_t valid) {
-  uint32_t m = 0xfu;
-#pragma unroll
-  for (int d = 0; d < D; ++d) {
-    const float4 lo = *reinterpret_cast<const float4*>(s + (uint32_t)d * F + g);
-    float4 hi = lo;
-    if (RECT) hi = *reinterpret_cast<const float4*>(s + (uint32_t)(D + d) * F + g);
-    m &= (overlaps1(b.lo[d], b.hi[d], lo.x, hi.x) ? 1u : 0u) | (overlaps1(b.lo[d], b.hi[d], lo.y, hi.y) ? 2u : 0u) |
-         (overlaps1(b.lo[d], b.hi[d], lo.z, hi.z) ? 4u : 0u) | (overlaps1(b.lo[d], b.hi[d], lo.w, hi.w) ? 8u : 0u);
-  }
-  if (g + 4 > valid) m &= (g < valid) ? (1u << (valid - g)) - 1u : 0u;
   return m;
 }
 

@@ -115,7 +115,7 @@ extern "C" qcp_status qcp_autotune(const float* objs, uint64_t n, uint32_t dims,
     };
     // 1. fan-out, default knobs
     const uint32_t fanouts[] = {64, 128, 256};
-    uint32_t best_f = 0, best_b = 8, best_w = qcp::kDefaultWinBits, best_lp = qcp::kDefaultLeafRing;
+    uint32_t best_f = 0, best_b = 8, best_w = qcp::kDefaultWinBits, best_lp = 2;
     float best = 0.f, best_build = 0.f;
     for (uint32_t f : fanouts) {
       bo.fanout = f;
