@@ -120,10 +120,11 @@ __global__ void __launch_bounds__(256) k_expand(const float* __restrict__ boxes,
 // to pay for k_join's staging (4.8 M points, 2,400 boxes of four ids, 2 items
 // per node: k_join 34 us, k_count 12); 16 M points, 1,900 boxes, 29 per node:
 // 110 against 143, and 32 M 8-D rectangles, 3,000 boxes, 13 per node: 154
-// against 202.
-constexpr uint32_t kNodeOrderItems = 12;
+// against 202.  Nor with so few items in all that k_join's runs are short (3 M
+// points, 2,314 boxes, 5,000 items: 34 against 12).
+constexpr uint32_t kNodeOrderItems = 12, kNodeOrderMinItems = 24576;
 __device__ __forceinline__ bool is_ordered(uint32_t nitems, uint64_t nodes) {
-  return nodes && nitems >= nodes * kNodeOrderItems;
+  return nodes && nitems >= kNodeOrderMinItems && nitems >= nodes * kNodeOrderItems;
 }
 
 // Items per level-1 node, and the items in node order (cursor: the exclusive

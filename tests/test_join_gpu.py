@@ -20,6 +20,9 @@ def make(dims, rect, n, q, seed):
     # about as many ids in all for the larger sets
     side = 0.5 * min(1.0, (1e8 / (n * q)) ** (1.0 / dims))
     h = (rng.uniform(0.0, side, (q, 1)) * rng.uniform(0.5, 1.0, (q, dims))).astype(np.float32)
+    if dims > 1:  # long boxes: many partially covered leaves for their ids
+        h[:, 0] *= 12
+        h[:, 1:] /= np.float32(12 ** (1 / (dims - 1)))
     boxes = np.concatenate([c - h, c + h], 1)
     boxes[0, :dims], boxes[0, dims:] = -np.inf, np.inf  # everything
     boxes[1, :dims], boxes[1, dims:] = 1.0, 0.0         # nothing
@@ -36,7 +39,7 @@ def make(dims, rect, n, q, seed):
     (8, True, 256, 70_003, 300),
     # at least 16,384 leaves and 2,048 boxes: node order
     (3, False, 32, 524_289, 2049), (2, False, 64, 1_048_600, 2048), (2, True, 96, 1_600_001, 2100),
-    (8, True, 128, 2_097_200, 2048), (3, False, 160, 2_700_001, 2048)])
+    (8, True, 128, 2_097_200, 2700), (2, False, 160, 2_700_001, 3700)])
 def test_counts_and_ids(qcp, oracle, dims, rect, fanout, n, q):
     objs, boxes = make(dims, rect, n, q, n)
     offs, ids = oracle.ids(objs, dims, rect, boxes)
@@ -46,6 +49,11 @@ def test_counts_and_ids(qcp, oracle, dims, rect, fanout, n, q):
             for lanes in (32, 16, 8):
                 res = ix.search(boxes, hit_cache=hit_cache, lanes_per_item=lanes)
                 assert_same_hits(res.offsets, res.ids, offs, ids)
+        if n >= 500_000:
+            ix.search(boxes, timing=True).release()
+            st = qcp.last_stats()
+            assert st["leaf_items"] >= max(24576, 12 * ix.info()["level_nodes"][1])
+            assert st["hits"] == len(ids) and 0 < st["objects_covered"] < len(ids)
         with qcp.Plan(ix, q, len(ids) + 1) as plan:
             got = plan.run(boxes)
             assert_same_hits(got[0], got[1], offs, ids)
@@ -59,6 +67,7 @@ def test_hit_bits_without_room(qcp, oracle):
     objs, boxes = make(2, False, 524_301, 3000, 5)
     boxes[3:, 1] = -1.0
     boxes[3:, 3] = 2.0
+    boxes[3:, 0] = np.random.default_rng(6).random(len(boxes) - 3, dtype=np.float32) ** 2
     boxes[3:, 2] = boxes[3:, 0] + np.float32(2e-3)
     offs, ids = oracle.ids(objs, 2, False, boxes)
     with qcp.Index.build(objs, fanout=32) as ix:
