@@ -506,7 +506,8 @@ static qcp_status build_impl(const float* objs, uint64_t n, uint32_t dims, uint3
   if ((st = ix->pool.get(sizeof(uint64_t) * n, &keys_tmp)) != QCP_OK) goto fail;
   if ((st = ix->pool.get(sizeof(uint32_t) * n, &vals)) != QCP_OK) goto fail;
   if ((st = ix->pool.get(sizeof(uint32_t) * n, &vals_tmp)) != QCP_OK) goto fail;
-  if ((st = ix->pool.get(sizeof(uint32_t), &bad)) != QCP_OK) goto fail;
+  // error bits, and eight bytes on the largest key
+  if ((st = ix->pool.get(16, &bad)) != QCP_OK) goto fail;
   if (cudaMemsetAsync(bad, 0, sizeof(uint32_t), s) != cudaSuccess) {
     st = cuda_status(cudaGetLastError(), "memset");
     goto fail;
@@ -514,14 +515,15 @@ static qcp_status build_impl(const float* objs, uint64_t n, uint32_t dims, uint3
   if (ix->key_mode == QCP_KEY_KMEANS) {
     const uint32_t K = o.kmeans_clusters ? o.kmeans_clusters : (uint32_t)(n < 1024 ? n : 1024);
     if ((st = build_keys_kmeans((const float*)d_objs, n, dims, is_rect, bits, K,
-                                o.kmeans_iters ? o.kmeans_iters : 30u, ix->keys, (uint32_t*)vals, s)) != QCP_OK)
+                                o.kmeans_iters ? o.kmeans_iters : 30u, ix->keys, (uint64_t*)bad + 1, s)) != QCP_OK)
       goto fail;
   } else if ((st = build_keys((const float*)d_objs, n, dims, is_rect, ix->key_mode, bits, ix->keys,
-                              (uint32_t*)vals, s)) != QCP_OK) {
+                              (uint64_t*)bad + 1, s)) != QCP_OK) {
     goto fail;
   }
   if ((st = radix_sort_pairs(ix->keys, (uint32_t*)vals, (uint64_t*)keys_tmp, (uint32_t*)vals_tmp, n,
-                             ix->key_mode == QCP_KEY_KMEANS ? 64u : dims * bits, ix->pool, s, &in_tmp)) != QCP_OK)
+                             ix->key_mode == QCP_KEY_KMEANS ? 64u : dims * bits, (uint64_t*)bad + 1,
+                             (uint32_t*)bad, s, &in_tmp)) != QCP_OK)
     goto fail;
   if (in_tmp) {
     if (cudaMemcpyAsync(ix->keys, keys_tmp, sizeof(uint64_t) * n, cudaMemcpyDeviceToDevice, s) !=
@@ -540,8 +542,8 @@ static qcp_status build_impl(const float* objs, uint64_t n, uint32_t dims, uint3
     goto fail;
   }
   if (h_bad) {
-    set_error("object coordinates must be finite");
-    st = QCP_ERR_BAD_ARG;
+    set_error(h_bad & 1u ? "object coordinates must be finite" : "a bounded wait of the radix sort ran out");
+    st = h_bad & 1u ? QCP_ERR_BAD_ARG : QCP_ERR_TIMEOUT;
     goto fail;
   }
   ix->pool.put(0, keys_tmp);
@@ -703,7 +705,7 @@ struct qcp_build_plan {
   uint64_t* keys_tmp = nullptr;
   uint32_t* vals = nullptr;
   uint32_t* vals_tmp = nullptr;
-  uint32_t* bad = nullptr;      // nonzero: a coordinate was not finite
+  uint32_t* bad = nullptr;      // error bits (1: a coordinate was not finite); at 8 bytes the largest key
   uint32_t* h_bad = nullptr;    // pinned mirror
   void* rs_scratch = nullptr;
   size_t rs_bytes = 0;
@@ -732,9 +734,11 @@ static void build_plan_destroy(qcp_build_plan* p) {
 static qcp_status build_plan_record(qcp_build_plan* p, cudaStream_t s) {
   qcp_index* ix = p->ix;
   QCP_CUDA(cudaMemsetAsync(p->bad, 0, sizeof(uint32_t), s));
-  QCP_TRY(build_keys(p->d_in, ix->n, ix->dims, ix->is_rect, ix->key_mode, ix->key_bits, ix->keys, p->vals, s));
+  QCP_TRY(build_keys(p->d_in, ix->n, ix->dims, ix->is_rect, ix->key_mode, ix->key_bits, ix->keys,
+                     reinterpret_cast<uint64_t*>(p->bad) + 1, s));
   bool in_tmp = false;
-  QCP_TRY(radix_sort_pairs(ix->keys, p->vals, p->keys_tmp, p->vals_tmp, ix->n, ix->dims * ix->key_bits, ix->pool, s,
+  QCP_TRY(radix_sort_pairs(ix->keys, p->vals, p->keys_tmp, p->vals_tmp, ix->n, ix->dims * ix->key_bits,
+                           reinterpret_cast<uint64_t*>(p->bad) + 1, p->bad, s,
                            &in_tmp, p->rs_scratch, p->rs_bytes));
   if (in_tmp)
     QCP_CUDA(cudaMemcpyAsync(ix->keys, p->keys_tmp, sizeof(uint64_t) * ix->n, cudaMemcpyDeviceToDevice, s));
@@ -811,7 +815,7 @@ qcp_status qcp_build_plan_create(uint64_t n, uint32_t dims, uint32_t is_rect, co
         cudaMalloc(&p->keys_tmp, sizeof(uint64_t) * n) != cudaSuccess ||
         cudaMalloc(&p->vals, sizeof(uint32_t) * n) != cudaSuccess ||
         cudaMalloc(&p->vals_tmp, sizeof(uint32_t) * n) != cudaSuccess ||
-        cudaMalloc(&p->bad, sizeof(uint32_t)) != cudaSuccess ||
+        cudaMalloc(&p->bad, 16) != cudaSuccess ||
         cudaMalloc(&p->rs_scratch, p->rs_bytes) != cudaSuccess ||
         cudaMallocHost(&p->h_bad, sizeof(uint32_t)) != cudaSuccess) {
       st = cuda_status(cudaGetLastError(), "qcp_build_plan_create allocation");
@@ -872,8 +876,8 @@ qcp_status qcp_build_plan_run(qcp_build_plan* p, const float* objs, uint32_t obj
     p->ix->host_mbr_ready = false;  // host copies of the old levels are stale
   }
   if (*p->h_bad) {
-    set_error("object coordinates must be finite");
-    return QCP_ERR_BAD_ARG;
+    set_error(*p->h_bad & 1u ? "object coordinates must be finite" : "a bounded wait of the radix sort ran out");
+    return *p->h_bad & 1u ? QCP_ERR_BAD_ARG : QCP_ERR_TIMEOUT;
   }
   *index = p->ix;
   return QCP_OK;

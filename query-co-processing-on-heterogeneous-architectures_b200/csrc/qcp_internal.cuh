@@ -319,55 +319,37 @@ __host__ __device__ inline uint64_t hilbert_index_t(uint32_t bits, const int64_t
   return hilbert_finish<D>(index, bits);
 }
 
-// Table-driven levels for D = 2 and 3: kHilbertLevels<D> levels per lookup.
-// A rotation state (rot, flip) is encoded as rot * (D + 1) + f, f = 0 for
-// flip == 0 and 1 + log2(flip) otherwise.  Entry [state << (L*D) | input]
-// holds the L*D index bits of the L levels in its low byte and the state
-// after them in bits 8..15; it is filled from hilbert_step, so a lookup is
-// exactly L steps.
-template <int D> struct HilbertTab;
-template <> struct HilbertTab<2> { static constexpr uint32_t L = 4, kStates = 6; };
-template <> struct HilbertTab<3> { static constexpr uint32_t L = 2, kStates = 12; };
+// Table-driven levels: HilbertTab<D>::L levels per lookup.  A rotation state
+// (rot, flip) is encoded as rot * (D + 1) + f, f = 0 for flip == 0 and 1 +
+// log2(flip) otherwise.  The input of a lookup is the L Gray-coded bits of
+// every coordinate, coordinate d's at bits [d * L, (d + 1) * L), its highest
+// level's bit on top.  Entry [state << (L * D) | input] holds the L * D index
+// bits of the L levels below the state after them (16 bits in all); it is
+// filled from hilbert_step, so a lookup is exactly L steps.
+template <int D> struct HilbertTab { static constexpr uint32_t L = 1; };
+template <> struct HilbertTab<2> { static constexpr uint32_t L = 4; };  // 3 KB
+template <> struct HilbertTab<3> { static constexpr uint32_t L = 3; };  // 12 KB
+template <> struct HilbertTab<4> { static constexpr uint32_t L = 2; };  // 10 KB; 8-D: 36 KB
 
 template <int D>
-__host__ __device__ __forceinline__ uint16_t hilbert_tab_entry(uint32_t e) {
+__host__ __device__ constexpr uint32_t hilbert_tab_size() {
+  return (uint32_t)(D * (D + 1)) << (HilbertTab<D>::L * D);
+}
+
+template <int D>
+__host__ __device__ __forceinline__ uint16_t hilbert_field_entry(uint32_t e) {
   constexpr uint32_t L = HilbertTab<D>::L, IB = L * D;
   const uint32_t state = e >> IB, in = e & ((1u << IB) - 1u);
   uint32_t rot = state / (D + 1), f = state % (D + 1);
   uint64_t flip = f ? (1ull << (f - 1)) : 0ull;
   uint32_t out = 0;
   for (uint32_t j = 0; j < L; ++j) {
-    const uint64_t gin = (in >> ((L - 1 - j) * D)) & ((1u << D) - 1u);
+    uint32_t gin = 0;
+    for (uint32_t d = 0; d < (uint32_t)D; ++d) gin |= ((in >> (d * L + L - 1 - j)) & 1u) << d;
     out = (out << D) | (uint32_t)hilbert_step<D>(gin, rot, flip);
   }
   const uint32_t nf = flip ? (uint32_t)(63u - clz64(flip)) + 1u : 0u;
-  return (uint16_t)(out | ((rot * (D + 1) + nf) << 8));
-}
-
-// hilbert_index_t through a filled table (HilbertTab<D>::kStates << (L*D)
-// entries of hilbert_tab_entry), then plain steps for the bits % L lowest
-// levels.
-template <int D>
-__host__ __device__ __forceinline__ uint64_t hilbert_index_tab(uint32_t bits, const int64_t* coord,
-                                                             const uint16_t* tab) {
-  constexpr uint32_t L = HilbertTab<D>::L, IB = L * D;
-  uint64_t t = hilbert_transpose<D>(bits, coord);
-  if (bits <= 1) return hilbert_finish<D>(t, bits);
-  t ^= t >> D;
-  uint64_t index = 0;
-  uint32_t state = 0;
-  int lvl = (int)bits - 1;
-  for (; lvl + 1 >= (int)L; lvl -= (int)L) {
-    const uint32_t in = (uint32_t)(t >> ((lvl + 1 - (int)L) * D)) & ((1u << IB) - 1u);
-    const uint32_t e = tab[(state << IB) | in];
-    index = (index << IB) | (e & 0xffu);
-    state = e >> 8;
-  }
-  uint32_t rot = state / (D + 1), f = state % (D + 1);
-  uint64_t flip = f ? (1ull << (f - 1)) : 0ull;
-  for (; lvl >= 0; --lvl)
-    index = (index << D) | hilbert_step<D>((t >> (lvl * D)) & ((1ull << D) - 1ull), rot, flip);
-  return hilbert_finish<D>(index, bits);
+  return (uint16_t)(out | ((rot * (D + 1) + nf) << IB));
 }
 
 __host__ __device__ inline uint64_t hilbert_index(uint32_t dims, uint32_t bits, const int64_t* coord) {
@@ -404,17 +386,19 @@ int num_sms();
 
 // Build
 qcp_status build_keys(const float* objs, uint64_t n, uint32_t dims, uint32_t is_rect,
-                      uint32_t key_mode, uint32_t key_bits, uint64_t* keys, uint32_t* vals,
-                      cudaStream_t s);
-// With `scratch` (at least radix_scratch_bytes(n)) nothing is allocated, so
-// the sort can be captured into a graph.
+                      uint32_t key_mode, uint32_t key_bits, uint64_t* keys, uint64_t* max_key, cudaStream_t s);
+// Sorts the keys, none larger than the device's *max_key; the values are their positions before the sort (vals and
+// vals_tmp are output only).  With `scratch` (at least radix_scratch_bytes(n))
+// nothing is allocated, so the sort can be captured into a graph.  *err |= 2
+// on the device when a bounded wait ran out.
 qcp_status radix_sort_pairs(uint64_t* keys, uint32_t* vals, uint64_t* keys_tmp, uint32_t* vals_tmp,
-                            uint64_t n, uint32_t key_bits, DevPool& pool, cudaStream_t s,
+                            uint64_t n, uint32_t key_bits, const uint64_t* max_key, uint32_t* err, cudaStream_t s,
                             bool* result_in_tmp, void* scratch = nullptr, size_t scratch_bytes = 0);
 size_t radix_scratch_bytes(uint64_t n);
 qcp_status build_keys_kmeans(const float* objs, uint64_t n, uint32_t dims, uint32_t is_rect, uint32_t bits,
-                             uint32_t K, uint32_t max_iters, uint64_t* keys, uint32_t* vals, cudaStream_t s);
+                             uint32_t K, uint32_t max_iters, uint64_t* keys, uint64_t* max_key, cudaStream_t s);
 uint32_t kmeans_rank_bits(uint32_t K);
+// Packing with the leaf MBRs; the levels above them.
 qcp_status build_pack(qcp_index* ix, const float* objs, const uint32_t* perm, cudaStream_t s,
                       uint32_t* d_bad);
 qcp_status build_levels(qcp_index* ix, cudaStream_t s);

@@ -304,7 +304,7 @@ uint32_t kmeans_rank_bits(uint32_t K) {
 }
 
 qcp_status build_keys_kmeans(const float* objs, uint64_t n, uint32_t dims, uint32_t is_rect, uint32_t bits,
-                             uint32_t K, uint32_t max_iters, uint64_t* keys, uint32_t* vals, cudaStream_t s) {
+                             uint32_t K, uint32_t max_iters, uint64_t* keys, uint64_t* max_key, cudaStream_t s) {
   if (K > n) K = (uint32_t)n;
   if (K == 0) K = 1;
   const uint32_t sms = (uint32_t)num_sms();
@@ -405,13 +405,15 @@ qcp_status build_keys_kmeans(const float* objs, uint64_t n, uint32_t dims, uint3
       break;
     }
     // own keys, then cluster-major keys
-    if ((st = build_keys(objs, n, dims, is_rect, QCP_KEY_NORM, bits, keys, vals, s)) != QCP_OK) break;
+    if ((st = build_keys(objs, n, dims, is_rect, QCP_KEY_NORM, bits, keys, max_key, s)) != QCP_OK) break;
     const uint32_t rbits = kmeans_rank_bits(K);
     const uint32_t own_bits = dims * bits;
     const uint32_t own_shift = own_bits > 64 - rbits ? own_bits - (64 - rbits) : 0;
     k_combine<<<grid, 256, 0, s>>>(member, rank, n, rbits, own_shift, keys);
     note_launch();
-    st = check_launch("kmeans keys");
+    // ranks and own keys may fill all 64 bits
+    if (cudaMemsetAsync(max_key, 0xff, sizeof(uint64_t), s) != cudaSuccess) st = cuda_status(cudaGetLastError(), "memset");
+    if (st == QCP_OK) st = check_launch("kmeans keys");
     if (st == QCP_OK && cudaStreamSynchronize(s) != cudaSuccess) st = cuda_status(cudaGetLastError(), "kmeans");
   } while (false);
   cudaFree(buf);
