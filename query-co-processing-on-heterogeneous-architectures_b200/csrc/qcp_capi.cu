@@ -71,11 +71,11 @@ qcp_status DevPool::get(size_t bytes, void** out) {
   }
   const size_t sz = round_alloc(bytes);
   void* p = nullptr;
-  cudaError_t e = cudaMalloc(&p, sz);
+  cudaError_t e = dev_malloc(&p, sz);
   if (e == cudaErrorMemoryAllocation) {
     cudaGetLastError();
     trim();
-    e = cudaMalloc(&p, sz);
+    e = dev_malloc(&p, sz);
   }
   if (e != cudaSuccess) return cuda_status(e, "cudaMalloc");
   // remember the real size through the free list protocol: callers hand the
@@ -102,7 +102,7 @@ void DevPool::put(size_t bytes, void* p) {
 void DevPool::trim() {
   std::lock_guard<std::mutex> g(mu);
   for (auto& kv : free_list) {
-    cudaFree(kv.second);
+    dev_free(kv.second);
     for (size_t i = 0; i < sizes.size(); ++i)
       if (sizes[i].first == kv.second) {
         sizes.erase(sizes.begin() + i);
@@ -184,10 +184,10 @@ static qcp_status grow(T** p, size_t* cap, size_t need, size_t elems_min = 1) {
   if (*p && *cap >= need) return QCP_OK;
   size_t n = need < elems_min ? elems_min : need;
   n += n >> 2;  // headroom
-  if (*p) cudaFree(*p);
+  if (*p) dev_free(*p);
   *p = nullptr;
   *cap = 0;
-  cudaError_t e = cudaMalloc((void**)p, sizeof(T) * n);
+  cudaError_t e = dev_malloc(p, sizeof(T) * n);
   if (e != cudaSuccess) return cuda_status(e, "workspace cudaMalloc");
   *cap = n;
   return QCP_OK;
@@ -197,12 +197,12 @@ qcp_status ws_reserve_items(qcp_index* ix, Workspace* ws, size_t items) {
   (void)ix;
   if (items == 0 || (ws->items[0] && ws->items_cap >= items)) return QCP_OK;
   size_t n = items + (items >> 2) + 1024;
-  cudaFree(ws->items[0]);
-  cudaFree(ws->items[1]);
+  dev_free(ws->items[0]);
+  dev_free(ws->items[1]);
   ws->items[0] = ws->items[1] = nullptr;
   ws->items_cap = 0;
-  QCP_CUDA(cudaMalloc(&ws->items[0], sizeof(uint2) * n));
-  QCP_CUDA(cudaMalloc(&ws->items[1], sizeof(uint2) * n));
+  QCP_CUDA(dev_malloc(&ws->items[0], sizeof(uint2) * n));
+  QCP_CUDA(dev_malloc(&ws->items[1], sizeof(uint2) * n));
   ws->items_cap = n;
   return QCP_OK;
 }
@@ -211,12 +211,12 @@ qcp_status ws_reserve_queries(qcp_index* ix, Workspace* ws, uint32_t q) {
   const size_t need = (size_t)q + 1;
   if (!ws->qcount || ws->q_cap < need) {
     const size_t n = need + (need >> 2) + 64;
-    cudaFree(ws->qcount);
-    cudaFree(ws->qcursor);
+    dev_free(ws->qcount);
+    dev_free(ws->qcursor);
     ws->qcount = ws->qcursor = nullptr;
     ws->q_cap = 0;
-    QCP_CUDA(cudaMalloc(&ws->qcount, sizeof(uint64_t) * n));
-    QCP_CUDA(cudaMalloc(&ws->qcursor, sizeof(uint64_t) * n));
+    QCP_CUDA(dev_malloc(&ws->qcount, sizeof(uint64_t) * n));
+    QCP_CUDA(dev_malloc(&ws->qcursor, sizeof(uint64_t) * n));
     ws->q_cap = n;
   }
   if (!ws->offsets || ws->offsets_cap < need) {
@@ -230,13 +230,12 @@ qcp_status ws_reserve_queries(qcp_index* ix, Workspace* ws, uint32_t q) {
   }
   QCP_TRY(grow(&ws->boxes, &ws->boxes_cap, (size_t)q * 2 * ix->dims, 64));
   if (!ws->ctr) {
-    QCP_CUDA(cudaMalloc(&ws->ctr, sizeof(uint32_t) * kCtrCount));
-    QCP_CUDA(cudaHostAlloc(&ws->h_ctr, sizeof(uint32_t) * kCtrCount, cudaHostAllocDefault));
-    QCP_CUDA(cudaHostAlloc(&ws->h_total, sizeof(uint64_t), cudaHostAllocDefault));
-    QCP_CUDA(cudaMalloc(&ws->d_stats, sizeof(unsigned long long) * kStatCount));
-    QCP_CUDA(cudaMemset(ws->d_stats, 0, sizeof(unsigned long long) * kStatCount));
-    QCP_CUDA(cudaHostAlloc(&ws->h_stats, sizeof(unsigned long long) * kStatCount, cudaHostAllocDefault));
-    for (int i = 0; i < kEvCountSlots; ++i) QCP_CUDA(cudaEventCreate(&ws->ev[i]));
+    QCP_CUDA(dev_malloc(&ws->d_stats, sizeof(unsigned long long) * kStatCount));
+    QCP_TRY(host_pool().get(sizeof(uint64_t) * (kStatCount + 1) + sizeof(uint32_t) * kCtrCount, &ws->h_block));
+    ws->h_stats = static_cast<unsigned long long*>(ws->h_block);
+    ws->h_total = reinterpret_cast<uint64_t*>(ws->h_stats + kStatCount);
+    ws->h_ctr = reinterpret_cast<uint32_t*>(ws->h_total + 1);
+    QCP_CUDA(dev_malloc(&ws->ctr, sizeof(uint32_t) * kCtrCount));
   }
   // the root frontier holds one item per query
   if (!ws->items[0] || ws->items_cap < q) {
@@ -271,12 +270,12 @@ qcp_status ws_reserve_sort(qcp_index* ix, Workspace* ws, size_t jobs, size_t til
   (void)ix;
   if (jobs && (!ws->jobs[0] || ws->jobs_cap < jobs)) {
     size_t n = jobs + (jobs >> 2) + 256;
-    cudaFree(ws->jobs[0]);
-    cudaFree(ws->jobs[1]);
+    dev_free(ws->jobs[0]);
+    dev_free(ws->jobs[1]);
     ws->jobs[0] = ws->jobs[1] = nullptr;
     ws->jobs_cap = 0;
-    QCP_CUDA(cudaMalloc(&ws->jobs[0], sizeof(uint4) * n));
-    QCP_CUDA(cudaMalloc(&ws->jobs[1], sizeof(uint4) * n));
+    QCP_CUDA(dev_malloc(&ws->jobs[0], sizeof(uint4) * n));
+    QCP_CUDA(dev_malloc(&ws->jobs[1], sizeof(uint4) * n));
     ws->jobs_cap = n;
   }
   if (tiles) {
@@ -291,18 +290,18 @@ qcp_status ws_reserve_sort(qcp_index* ix, Workspace* ws, size_t jobs, size_t til
 // `mask_words` words of partial-leaf hit bits (each grown on its own).
 qcp_status ws_reserve_hitcache(Workspace* ws, size_t recs, size_t mask_words) {
   if (recs && (!ws->item_grp || ws->item_grp_cap < recs)) {
-    cudaFree(ws->item_grp);
+    dev_free(ws->item_grp);
     ws->item_grp = nullptr;
     ws->item_grp_cap = 0;
-    QCP_CUDA(cudaMalloc(&ws->item_grp, sizeof(uint4) * recs));
+    QCP_CUDA(dev_malloc(&ws->item_grp, sizeof(uint4) * recs));
     ws->item_grp_cap = recs;
   }
   if (mask_words && (!ws->hmask || ws->hmask_cap < mask_words)) {
-    cudaFree(ws->hmask);
+    dev_free(ws->hmask);
     ws->hmask = nullptr;
     ws->hmask_cap = 0;
     const size_t n = mask_words + (mask_words >> 2) + 4096;
-    QCP_CUDA(cudaMalloc(&ws->hmask, sizeof(uint32_t) * n));
+    QCP_CUDA(dev_malloc(&ws->hmask, sizeof(uint32_t) * n));
     ws->hmask_cap = n;
   }
   return QCP_OK;
@@ -320,37 +319,35 @@ qcp_status ws_reserve_nodes(Workspace* ws, size_t nodes) {
   QCP_TRY(grow(&ws->node_hist, &ws->node_hist_cap, 2 * nodes, 1024));
   const size_t need = scan_scratch_bytes(nodes);
   if (!ws->scan_tmp || ws->scan_tmp_cap < need) {
-    cudaFree(ws->scan_tmp);
+    dev_free(ws->scan_tmp);
     ws->scan_tmp = nullptr;
     ws->scan_tmp_cap = 0;
-    QCP_CUDA(cudaMalloc(&ws->scan_tmp, need));
+    QCP_CUDA(dev_malloc(&ws->scan_tmp, need));
     ws->scan_tmp_cap = need;
   }
   return QCP_OK;
 }
 
 void ws_destroy(Workspace* ws, qcp_index* ix) {
-  cudaFree(ws->node_hist);
-  cudaFree(ws->qwhist);
-  cudaFree(ws->scan_tmp);
-  cudaFree(ws->boxes);
-  cudaFree(ws->items[0]);
-  cudaFree(ws->items[1]);
-  cudaFree(ws->item_grp);
-  cudaFree(ws->hmask);
-  cudaFree(ws->qcount);
-  cudaFree(ws->qcursor);
+  dev_free(ws->node_hist);
+  dev_free(ws->qwhist);
+  dev_free(ws->scan_tmp);
+  dev_free(ws->boxes);
+  dev_free(ws->items[0]);
+  dev_free(ws->items[1]);
+  dev_free(ws->item_grp);
+  dev_free(ws->hmask);
+  dev_free(ws->qcount);
+  dev_free(ws->qcursor);
   if (ws->offsets) ix->pool.put(0, ws->offsets);
   if (ws->out_ids) ix->pool.put(0, ws->out_ids);
   if (ws->tmp_ids) ix->pool.put(0, ws->tmp_ids);
-  cudaFree(ws->jobs[0]);
-  cudaFree(ws->jobs[1]);
-  cudaFree(ws->seg_hist);
-  cudaFree(ws->ctr);
-  if (ws->h_ctr) cudaFreeHost(ws->h_ctr);
-  if (ws->h_total) cudaFreeHost(ws->h_total);
-  cudaFree(ws->d_stats);
-  if (ws->h_stats) cudaFreeHost(ws->h_stats);
+  dev_free(ws->jobs[0]);
+  dev_free(ws->jobs[1]);
+  dev_free(ws->seg_hist);
+  dev_free(ws->ctr);
+  if (ws->h_block) host_pool().put(0, ws->h_block);
+  dev_free(ws->d_stats);
   for (int i = 0; i < kEvCountSlots; ++i)
     if (ws->ev[i]) cudaEventDestroy(ws->ev[i]);
   delete ws;
@@ -390,10 +387,10 @@ static void index_release(qcp_index* ix) {
   for (Workspace* w : ix->ws_all) ws_destroy(w, ix);
   ix->ws_all.clear();
   ix->ws_free.clear();
-  cudaFree(ix->coords);
-  cudaFree(ix->ids);
-  cudaFree(ix->keys);
-  for (int l = 0; l < kMaxLevels; ++l) cudaFree(ix->mbr[l]);
+  dev_free(ix->coords);
+  dev_free(ix->ids);
+  dev_free(ix->keys);
+  for (int l = 0; l < kMaxLevels; ++l) dev_free(ix->mbr[l]);
   ix->pool.trim();
   delete ix;
 }
@@ -416,12 +413,12 @@ static qcp_status index_alloc(qcp_index* ix) {
   ix->levels = L;
   ix->npad = ix->level_nodes[0] * F;
   ix->device_bytes = 0;
-  QCP_CUDA(cudaMalloc(&ix->coords, sizeof(float) * ix->ncoord * ix->npad));
-  QCP_CUDA(cudaMalloc(&ix->ids, sizeof(int32_t) * ix->npad));
-  QCP_CUDA(cudaMalloc(&ix->keys, sizeof(uint64_t) * ix->n));
+  QCP_CUDA(dev_malloc(&ix->coords, sizeof(float) * ix->ncoord * ix->npad));
+  QCP_CUDA(dev_malloc(&ix->ids, sizeof(int32_t) * ix->npad));
+  QCP_CUDA(dev_malloc(&ix->keys, sizeof(uint64_t) * ix->n));
   ix->device_bytes += sizeof(float) * ix->ncoord * ix->npad + sizeof(int32_t) * ix->npad;
   for (uint32_t l = 0; l < L; ++l) {
-    QCP_CUDA(cudaMalloc(&ix->mbr[l], sizeof(float) * 2 * ix->dims * ix->level_pad[l]));
+    QCP_CUDA(dev_malloc(&ix->mbr[l], sizeof(float) * 2 * ix->dims * ix->level_pad[l]));
     ix->device_bytes += sizeof(float) * 2 * ix->dims * ix->level_pad[l];
   }
   return QCP_OK;
@@ -475,6 +472,7 @@ static qcp_status build_impl(const float* objs, uint64_t n, uint32_t dims, uint3
     return QCP_ERR_NO_DEVICE;
   }
   cudaStream_t s = (cudaStream_t)o.stream;
+  AllocOn on(s);
   qcp_index* ix = new (std::nothrow) qcp_index();
   if (!ix) return QCP_ERR_OOM;
   cudaGetDevice(&ix->device);
@@ -585,10 +583,14 @@ static qcp_status run_query(qcp_index* ix, const float* boxes, uint32_t q, const
     return QCP_ERR_BAD_ARG;
   }
   cudaStream_t s = (cudaStream_t)o.stream;
+  AllocOn on(s);
   Workspace* ws = ws_acquire(ix);
   if (!ws) return QCP_ERR_OOM;
   qcp_status st = ws_reserve_queries(ix, ws, q);
   ws->timing = (o.flags & QCP_QUERY_TIMING) != 0;
+  for (int i = 0; ws->timing && i < kEvCountSlots; ++i)
+    if (!ws->ev[i] && cudaEventCreate(&ws->ev[i]) != cudaSuccess && st == QCP_OK)
+      st = cuda_status(cudaGetLastError(), "cudaEventCreate");
   ws->blocks_per_sm = o.blocks_per_sm ? (o.blocks_per_sm > 32 ? 32u : o.blocks_per_sm) : 8u;
   ws->win_bits = o.win_bits ? (o.win_bits < 12 ? 12u : o.win_bits) : kDefaultWinBits;
   ws->lanes_per_item = lanes_per_item_of(o.lanes_per_item);
@@ -719,12 +721,12 @@ static void build_plan_destroy(qcp_build_plan* p) {
   if (!p) return;
   if (p->exec) cudaGraphExecDestroy(p->exec);
   if (p->graph) cudaGraphDestroy(p->graph);
-  cudaFree(p->d_in);
-  cudaFree(p->keys_tmp);
-  cudaFree(p->vals);
-  cudaFree(p->vals_tmp);
-  cudaFree(p->bad);
-  cudaFree(p->rs_scratch);
+  dev_free(p->d_in);
+  dev_free(p->keys_tmp);
+  dev_free(p->vals);
+  dev_free(p->vals_tmp);
+  dev_free(p->bad);
+  dev_free(p->rs_scratch);
   if (p->h_bad) cudaFreeHost(p->h_bad);
   if (p->ix) index_release(p->ix);
   delete p;
@@ -789,6 +791,7 @@ qcp_status qcp_build_plan_create(uint64_t n, uint32_t dims, uint32_t is_rect, co
     set_error("no CUDA device");
     return QCP_ERR_NO_DEVICE;
   }
+  AllocLasting lasting;
   qcp_build_plan* p = new (std::nothrow) qcp_build_plan();
   if (!p) return QCP_ERR_OOM;
   qcp_index* ix = new (std::nothrow) qcp_index();
@@ -811,12 +814,12 @@ qcp_status qcp_build_plan_create(uint64_t n, uint32_t dims, uint32_t is_rect, co
   qcp_status st = index_alloc(ix);
   cudaStream_t cap = nullptr;
   if (st == QCP_OK) {
-    if (cudaMalloc(&p->d_in, sizeof(float) * p->ncoord * n) != cudaSuccess ||
-        cudaMalloc(&p->keys_tmp, sizeof(uint64_t) * n) != cudaSuccess ||
-        cudaMalloc(&p->vals, sizeof(uint32_t) * n) != cudaSuccess ||
-        cudaMalloc(&p->vals_tmp, sizeof(uint32_t) * n) != cudaSuccess ||
-        cudaMalloc(&p->bad, 16) != cudaSuccess ||
-        cudaMalloc(&p->rs_scratch, p->rs_bytes) != cudaSuccess ||
+    if (dev_malloc(&p->d_in, sizeof(float) * p->ncoord * n) != cudaSuccess ||
+        dev_malloc(&p->keys_tmp, sizeof(uint64_t) * n) != cudaSuccess ||
+        dev_malloc(&p->vals, sizeof(uint32_t) * n) != cudaSuccess ||
+        dev_malloc(&p->vals_tmp, sizeof(uint32_t) * n) != cudaSuccess ||
+        dev_malloc(&p->bad, 16) != cudaSuccess ||
+        dev_malloc(&p->rs_scratch, p->rs_bytes) != cudaSuccess ||
         cudaMallocHost(&p->h_bad, sizeof(uint32_t)) != cudaSuccess) {
       st = cuda_status(cudaGetLastError(), "qcp_build_plan_create allocation");
       if (st == QCP_OK) st = QCP_ERR_OOM;
@@ -824,6 +827,8 @@ qcp_status qcp_build_plan_create(uint64_t n, uint32_t dims, uint32_t is_rect, co
   }
   if (st == QCP_OK && cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking) != cudaSuccess)
     st = cuda_status(cudaGetLastError(), "cudaStreamCreate");
+  // (allocated on the legacy stream, used on the capturing one)
+  if (st == QCP_OK && cudaStreamSynchronize(nullptr) != cudaSuccess) st = cuda_status(cudaGetLastError(), "allocation");
   if (st == QCP_OK) {
     // the build's attributes and lazily loaded kernels are set up by one
     // uncaptured run over the (zeroed) input before the capture

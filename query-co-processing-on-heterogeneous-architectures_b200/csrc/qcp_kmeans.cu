@@ -316,7 +316,7 @@ qcp_status build_keys_kmeans(const float* objs, uint64_t n, uint32_t dims, uint3
   const size_t aux_b = 1024;  // bounds, lo, scale, change counter
   void* buf = nullptr;
   const size_t total = rep_b + cen_b + sum_b + cnt_b + mem_b + aux_b + sizeof(uint32_t) * K + 6 * 256;
-  QCP_CUDA(cudaMalloc(&buf, total));
+  QCP_CUDA(dev_malloc(&buf, total));
   char* p = reinterpret_cast<char*>(buf);
   auto take = [&](size_t b) {
     char* r = p;
@@ -416,7 +416,7 @@ qcp_status build_keys_kmeans(const float* objs, uint64_t n, uint32_t dims, uint3
     if (st == QCP_OK) st = check_launch("kmeans keys");
     if (st == QCP_OK && cudaStreamSynchronize(s) != cudaSuccess) st = cuda_status(cudaGetLastError(), "kmeans");
   } while (false);
-  cudaFree(buf);
+  dev_free(buf);
   return st;
 }
 

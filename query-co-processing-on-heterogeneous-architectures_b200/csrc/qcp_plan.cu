@@ -40,8 +40,8 @@ void plan_destroy(qcp_plan* p) {
   if (p->exec) cudaGraphExecDestroy(p->exec);
   if (p->graph) cudaGraphDestroy(p->graph);
   if (p->capture) cudaStreamDestroy(p->capture);
-  cudaFree(p->tables);
-  cudaFree(p->empty);
+  qcp::dev_free(p->tables);
+  qcp::dev_free(p->empty);
   if (p->ws) qcp::ws_destroy(p->ws, p->ix);
   delete p;
 }
@@ -65,6 +65,7 @@ extern "C" qcp_status qcp_plan_create(qcp_index* ix, uint32_t max_queries, uint6
     return QCP_ERR_BAD_ARG;
   }
   *out = nullptr;
+  AllocLasting lasting;
   qcp_plan* p = new (std::nothrow) qcp_plan();
   if (!p) return QCP_ERR_OOM;
   p->ix = ix;
@@ -110,19 +111,21 @@ extern "C" qcp_status qcp_plan_create(qcp_index* ix, uint32_t max_queries, uint6
     // scan scratch owned by the workspace: no stream-ordered temporaries in the graph
     const size_t scan_need = scan_scratch_bytes((uint64_t)max_queries + 1);
     if (ws->scan_tmp_cap < scan_need) {
-      cudaFree(ws->scan_tmp);
+      dev_free(ws->scan_tmp);
       ws->scan_tmp = nullptr;
       ws->scan_tmp_cap = scan_need;
     }
-    if ((!ws->scan_tmp && cudaMalloc(&ws->scan_tmp, ws->scan_tmp_cap) != cudaSuccess) ||
-        cudaMalloc(&p->tables, sort_tables_bytes(ix, ws, max_queries)) != cudaSuccess ||
-        cudaMalloc(&p->empty, sizeof(float) * row * max_queries) != cudaSuccess) {
+    if ((!ws->scan_tmp && dev_malloc(&ws->scan_tmp, ws->scan_tmp_cap) != cudaSuccess) ||
+        dev_malloc(&p->tables, sort_tables_bytes(ix, ws, max_queries)) != cudaSuccess ||
+        dev_malloc(&p->empty, sizeof(float) * row * max_queries) != cudaSuccess) {
       st = cuda_status(cudaGetLastError(), "qcp_plan_create");
       break;
     }
     std::vector<float> e(row * max_queries);
     for (size_t i = 0; i < e.size(); ++i) e[i] = (i % row) < ix->dims ? INFINITY : -INFINITY;
+    // (allocated and filled on the legacy stream, used on the capturing one)
     if (cudaMemcpy(p->empty, e.data(), sizeof(float) * e.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
+        cudaStreamSynchronize(nullptr) != cudaSuccess ||
         cudaStreamCreateWithFlags(&p->capture, cudaStreamNonBlocking) != cudaSuccess ||
         cudaMemcpyAsync(ws->boxes, p->empty, sizeof(float) * e.size(), cudaMemcpyDeviceToDevice, p->capture) !=
             cudaSuccess) {
