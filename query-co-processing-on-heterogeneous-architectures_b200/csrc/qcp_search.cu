@@ -463,6 +463,15 @@ __global__ void __launch_bounds__(kJoinThreads, (RECT ? 2 * D : D) > 8 ? 4 : ((R
   }
 }
 
+// Whether a warp takes whole items: where their 32-leaf groups would be more
+// than eight rounds of the grid's warps.  15,000 items over 16 M points, six
+// rounds: the groups one by one 59 us to count and 59 to write, whole items 65
+// and 87; 10,000 items of tiny boxes at fan-out 256, nine rounds: 66 and 40,
+// whole items 44 and 23.
+__device__ __forceinline__ bool whole_items(uint32_t nitems, uint32_t G, uint32_t warps) {
+  return (uint64_t)nitems * G >= 8ull * warps;
+}
+
 // Counts of batches that are not in node order: a warp per item, or per
 // 32-leaf group of one where there are too few items to keep the warps busy;
 // no barriers.  Few items share a node, so nothing is staged: the box sits in
@@ -483,7 +492,7 @@ __global__ void __launch_bounds__(256, (RECT ? 2 * D : D) > 8 ? 2 : 4)
   const float* lmbr = t.mbr[0];
   const uint32_t chunks = (F + 127u) >> 7, wpl = chunks * kChunkWords;
   const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
-  const bool whole = nitems >= warps * 2u;
+  const bool whole = whole_items(nitems, G, warps);
   const uint64_t units = whole ? nitems : (uint64_t)nitems * G;
   uint64_t u = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   uint2 next = u < units ? items[whole ? u : u / G] : make_uint2(0, 0);
@@ -500,15 +509,25 @@ __global__ void __launch_bounds__(256, (RECT ? 2 * D : D) > 8 ? 2 : 4)
     }
     uint32_t total = 0;  // hits of the unit
     const uint32_t ga = whole ? 0u : (uint32_t)(u % G), gb = whole ? G : ga + 1;
+    float mlo[D], mhi[D];  // the next group's MBRs, loaded one group ahead
+    auto load_mbrs = [&](uint32_t g) {
+      const uint64_t at = (uint64_t)it.y * F + g * 32 + lane;
+#pragma unroll
+      for (int d = 0; d < D; ++d) {
+        mlo[d] = __ldg(lmbr + d * lpad + at);
+        mhi[d] = __ldg(lmbr + (D + d) * lpad + at);
+      }
+    };
+    load_mbrs(ga);
     for (uint32_t g = ga; g < gb; ++g) {
       const uint64_t l0 = (uint64_t)it.y * F + g * 32;  // the group's first leaf
       bool ov = l0 + lane < nleaves, in = true;
 #pragma unroll
       for (int d = 0; d < D; ++d) {
-        const float lo = __ldg(lmbr + d * lpad + l0 + lane), hi = __ldg(lmbr + (D + d) * lpad + l0 + lane);
-        ov &= overlaps1(-b[2 * d], b[2 * d + 1], lo, hi);
-        in &= inside1(-b[2 * d], b[2 * d + 1], lo, hi);
+        ov &= overlaps1(-b[2 * d], b[2 * d + 1], mlo[d], mhi[d]);
+        in &= inside1(-b[2 * d], b[2 * d + 1], mlo[d], mhi[d]);
       }
+      if (g + 1 < gb) load_mbrs(g + 1);
       const uint32_t mov = __ballot_sync(0xffffffffu, ov), mcov = __ballot_sync(0xffffffffu, ov && in);
       const uint32_t part = mov & ~mcov;
       // room for the hit bits; the objects' reads do not wait for it
@@ -608,14 +627,20 @@ __global__ void __launch_bounds__(256) k_leafwrite(TreeView t, const float* __re
   const uint32_t cpl = (F + 127u) >> 7;  // 128-object chunks per leaf
   const uint32_t nitems = (uint32_t)min((uint64_t)*item_count, item_cap);
   const uint32_t warps = gridDim.x * (blockDim.x >> 5);
-  // groups per fetch: a whole item, or one group in small batches
-  const bool whole = nitems >= warps * 4u;
+  // groups per fetch: a whole item, or one group in small batches; each warp's
+  // first one by its index, more as the warps get free (all in turn, without
+  // the atomic: 59 -> 87 us on the 15,000 items, a heavy item's groups follow
+  // one another; all by the atomic: 13 -> 18 us for 1,000 boxes over 1 M points)
+  const bool whole = whole_items(nitems, G, warps);
   const uint32_t per = whole ? G : 1u;
   const uint32_t nfetch = whole ? nitems : nitems * G;
-  for (;;) {
-    uint32_t f = 0;
-    if (lane == 0) f = atomicAdd(work, 1u);
-    f = __shfl_sync(0xffffffffu, f, 0);
+  for (uint32_t turn = 0;; ++turn) {
+    uint32_t f = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (turn) {
+      if (nfetch <= warps) break;
+      if (lane == 0) f = warps + atomicAdd(work, 1u);
+      f = __shfl_sync(0xffffffffu, f, 0);
+    }
     if (f >= nfetch) break;
     const uint32_t i = whole ? f : f / G, gbase = whole ? 0u : f % G;
     const uint2 it = items[i];
