@@ -209,14 +209,16 @@ qcp_status ws_reserve_items(qcp_index* ix, Workspace* ws, size_t items) {
 
 qcp_status ws_reserve_queries(qcp_index* ix, Workspace* ws, uint32_t q) {
   const size_t need = (size_t)q + 1;
-  if (!ws->qcount || ws->q_cap < need) {
+  if (!ws->zeroed || ws->q_cap < need) {
     const size_t n = need + (need >> 2) + 64;
-    dev_free(ws->qcount);
-    dev_free(ws->qcursor);
-    ws->qcount = ws->qcursor = nullptr;
+    const size_t head = (sizeof(uint32_t) * kCtrCount + 127) & ~(size_t)127;
+    dev_free(ws->zeroed);
+    ws->zeroed = nullptr;
     ws->q_cap = 0;
-    QCP_CUDA(dev_malloc(&ws->qcount, sizeof(uint64_t) * n));
-    QCP_CUDA(dev_malloc(&ws->qcursor, sizeof(uint64_t) * n));
+    QCP_CUDA(dev_malloc(&ws->zeroed, head + 2 * sizeof(uint64_t) * n));
+    ws->ctr = static_cast<uint32_t*>(ws->zeroed);
+    ws->qcount = reinterpret_cast<uint64_t*>(static_cast<char*>(ws->zeroed) + head);
+    ws->qcursor = ws->qcount + n;
     ws->q_cap = n;
   }
   if (!ws->offsets || ws->offsets_cap < need) {
@@ -229,13 +231,12 @@ qcp_status ws_reserve_queries(qcp_index* ix, Workspace* ws, uint32_t q) {
     ws->offsets_cap = need;
   }
   QCP_TRY(grow(&ws->boxes, &ws->boxes_cap, (size_t)q * 2 * ix->dims, 64));
-  if (!ws->ctr) {
+  if (!ws->d_stats) {
     QCP_CUDA(dev_malloc(&ws->d_stats, sizeof(unsigned long long) * kStatCount));
     QCP_TRY(host_pool().get(sizeof(uint64_t) * (kStatCount + 1) + sizeof(uint32_t) * kCtrCount, &ws->h_block));
     ws->h_stats = static_cast<unsigned long long*>(ws->h_block);
     ws->h_total = reinterpret_cast<uint64_t*>(ws->h_stats + kStatCount);
     ws->h_ctr = reinterpret_cast<uint32_t*>(ws->h_total + 1);
-    QCP_CUDA(dev_malloc(&ws->ctr, sizeof(uint32_t) * kCtrCount));
   }
   // the root frontier holds one item per query
   if (!ws->items[0] || ws->items_cap < q) {
@@ -272,8 +273,11 @@ qcp_status ws_reserve_sort(qcp_index* ix, Workspace* ws, size_t jobs, size_t til
     size_t n = jobs + (jobs >> 2) + 256;
     dev_free(ws->jobs[0]);
     dev_free(ws->jobs[1]);
+    dev_free(ws->job_tiles);
     ws->jobs[0] = ws->jobs[1] = nullptr;
+    ws->job_tiles = nullptr;
     ws->jobs_cap = 0;
+    QCP_CUDA(dev_malloc(&ws->job_tiles, sizeof(uint32_t) * n));
     QCP_CUDA(dev_malloc(&ws->jobs[0], sizeof(uint4) * n));
     QCP_CUDA(dev_malloc(&ws->jobs[1], sizeof(uint4) * n));
     ws->jobs_cap = n;
@@ -314,6 +318,8 @@ qcp_status ws_reserve_qwhist(Workspace* ws, size_t n) {
   return QCP_OK;
 }
 
+qcp_status ws_reserve_tables(Workspace* ws, size_t bytes) { return grow(&ws->tables, &ws->tables_cap, bytes, 4096); }
+
 // Counts and cursors per level-1 node and the scratch of their scan.
 qcp_status ws_reserve_nodes(Workspace* ws, size_t nodes) {
   QCP_TRY(grow(&ws->node_hist, &ws->node_hist_cap, 2 * nodes, 1024));
@@ -337,15 +343,18 @@ void ws_destroy(Workspace* ws, qcp_index* ix) {
   dev_free(ws->items[1]);
   dev_free(ws->item_grp);
   dev_free(ws->hmask);
-  dev_free(ws->qcount);
-  dev_free(ws->qcursor);
+  dev_free(ws->zeroed);
+  dev_free(ws->tables);
+  if (ws->side) cudaStreamDestroy(ws->side);
+  for (cudaEvent_t e : ws->side_ev)
+    if (e) cudaEventDestroy(e);
   if (ws->offsets) ix->pool.put(0, ws->offsets);
   if (ws->out_ids) ix->pool.put(0, ws->out_ids);
   if (ws->tmp_ids) ix->pool.put(0, ws->tmp_ids);
   dev_free(ws->jobs[0]);
   dev_free(ws->jobs[1]);
+  dev_free(ws->job_tiles);
   dev_free(ws->seg_hist);
-  dev_free(ws->ctr);
   if (ws->h_block) host_pool().put(0, ws->h_block);
   dev_free(ws->d_stats);
   for (int i = 0; i < kEvCountSlots; ++i)
@@ -613,13 +622,24 @@ static qcp_status run_query(qcp_index* ix, const float* boxes, uint32_t q, const
       ws->h_boxes = ws->h_boxes_copy.data();
     }
   }
+  ws->qboxes = ws->boxes;
   if (st == QCP_OK && q) {
-    const size_t bytes = sizeof(float) * 2 * ix->dims * (size_t)q;
-    cudaError_t e = cudaMemcpyAsync(ws->boxes, boxes, bytes,
-                                    o.boxes_mem == QCP_MEM_HOST ? cudaMemcpyHostToDevice
-                                                                : cudaMemcpyDeviceToDevice,
-                                    s);
-    if (e != cudaSuccess) st = cuda_status(e, "copy query boxes");
+    // boxes in this GPU's own memory, aligned as the workspace's, are read
+    // where they are (the call returns after its last use of them), others are
+    // copied over
+    cudaPointerAttributes at{};
+    if (o.boxes_mem == QCP_MEM_DEVICE && cudaPointerGetAttributes(&at, boxes) != cudaSuccess) cudaGetLastError();
+    if (at.type == cudaMemoryTypeDevice && at.device == ix->device &&
+        (reinterpret_cast<uintptr_t>(boxes) & 15) == 0) {
+      ws->qboxes = boxes;
+    } else {
+      const size_t bytes = sizeof(float) * 2 * ix->dims * (size_t)q;
+      cudaError_t e = cudaMemcpyAsync(ws->boxes, boxes, bytes,
+                                      o.boxes_mem == QCP_MEM_HOST ? cudaMemcpyHostToDevice
+                                                                  : cudaMemcpyDeviceToDevice,
+                                      s);
+      if (e != cudaSuccess) st = cuda_status(e, "copy query boxes");
+    }
   }
   if (st == QCP_OK) {
     if (q == 0) {

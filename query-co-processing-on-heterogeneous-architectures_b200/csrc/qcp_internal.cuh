@@ -122,8 +122,10 @@ enum EvSlot : int {
 struct Workspace {
   float* boxes = nullptr;
   size_t boxes_cap = 0;          // floats
+  const float* qboxes = nullptr; // this call's boxes on the device: boxes, or the caller's own
   uint2* items[2] = {nullptr, nullptr};
   size_t items_cap = 0;          // (query, node) items per buffer
+  void* zeroed = nullptr;        // ctr, qcount and qcursor in one block, cleared by one memset
   uint64_t* qcount = nullptr;    // per-query counts, q
   uint64_t* qcursor = nullptr;   // per-query write cursors, q
   uint64_t* offsets = nullptr;   // q + 1, from the index's pool
@@ -134,7 +136,12 @@ struct Workspace {
   size_t out_cap = 0;            // ids
   // segmented sort job lists
   uint4* jobs[2] = {nullptr, nullptr};
+  uint32_t* job_tiles = nullptr; // first tile of every larger slice
   size_t jobs_cap = 0;
+  cudaStream_t side = nullptr;   // plans: the captured pipeline's second branch
+  cudaEvent_t side_ev[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
+  char* tables = nullptr;        // the window partition's tables
+  size_t tables_cap = 0;
   uint32_t* seg_hist = nullptr;  // MSD tile -> job map
   size_t seg_hist_cap = 0;
   uint32_t* ctr = nullptr;       // device counters (see kCtr*)
@@ -190,6 +197,17 @@ enum StatSlot : uint32_t {
 };
 
 
+// Stream b waits for what stream a holds so far (ev: one of ws->side_ev).
+inline cudaError_t ws_branch(Workspace* ws, int ev, cudaStream_t a, cudaStream_t b) {
+  const cudaError_t e = cudaEventRecord(ws->side_ev[ev], a);
+  return e != cudaSuccess ? e : cudaStreamWaitEvent(b, ws->side_ev[ev], 0);
+}
+
+// Counters, counts and cursors of q queries to zero.
+inline cudaError_t ws_zero(Workspace* ws, uint32_t q, cudaStream_t s) {
+  return cudaMemsetAsync(ws->zeroed, 0, reinterpret_cast<char*>(ws->qcursor + q) - static_cast<char*>(ws->zeroed), s);
+}
+
 inline void mark(Workspace* ws, int slot, cudaStream_t s) {
   if (ws->timing) cudaEventRecord(ws->ev[slot], s);
 }
@@ -204,12 +222,14 @@ enum CtrSlot : uint32_t {
   kCtrJobs0 = 5,      // segmented-sort job list sizes
   kCtrJobs1 = 6,
   kCtrSmall = 7,      // small-segment job count
-  kCtrWork2 = 8,
+  kCtrTiles = 8,      // tiles of the larger slices
   kCtrTimeout = 9,    // nonzero: a bounded device wait ran out (results invalid)
   kCtrWinBig = 11,    // windows listed for the bitmap sort
   kCtrWinSmall = 12,  // windows listed for the one-warp sort
+  kCtrWrite = 13,     // dynamic work fetch counter of the write pass
   kCtrMaskWords = 14, // (64 bits) hit-bit words the count pass asked for (may exceed the capacity)
-  kCtrCount = 16
+  kCtrTotal = 16,     // (64 bits) ids of all queries
+  kCtrCount = 18
 };
 
 }  // namespace qcp
@@ -476,17 +496,21 @@ constexpr uint32_t kNoMask = 0xffffffffu;            // group without cached hit
 constexpr size_t kMaxMaskWords = 0xc0000000u;        // hit-bit words (32-bit offsets)
 qcp_status ws_reserve_hitcache(Workspace* ws, size_t recs, size_t mask_words);
 qcp_status ws_reserve_nodes(Workspace* ws, size_t nodes);
+qcp_status ws_reserve_tables(Workspace* ws, size_t bytes);
 // Workspace construction and buffer reservation (qcp_capi.cu).
 qcp_status ws_reserve_queries(qcp_index* ix, Workspace* ws, uint32_t q);
 qcp_status ws_reserve_items(qcp_index* ix, Workspace* ws, size_t items);
 qcp_status ws_reserve_out(qcp_index* ix, Workspace* ws, size_t ids);
 qcp_status ws_reserve_sort(qcp_index* ix, Workspace* ws, size_t jobs, size_t tiles);
 void ws_destroy(Workspace* ws, qcp_index* ix);
-qcp_status segmented_sort(qcp_index* ix, Workspace* ws, uint32_t q, cudaStream_t s);
-// Sorts the slices of <= kSmallSliceCap ids; the larger slices are returned
-// as a device job list (big, *nbig entries) for the caller.
-qcp_status sort_small_slices(qcp_index* ix, Workspace* ws, uint32_t q, cudaStream_t s,
-                             const SortJob** big, uint32_t* nbig);
+// After the scan of the counts, before the host reads the counters: the
+// batch's total into ctr[kCtrTotal] and, if sort, the slices' job lists and
+// tile counts.  cap: most ids the output holds; more sets bit 2 of
+// ctr[kCtrOverflow] and *item_count = 0 (item_count may be nullptr).
+qcp_status classify_slices(qcp_index* ix, Workspace* ws, uint32_t q, bool sort, uint64_t cap, uint32_t* item_count,
+                           cudaStream_t s);
+// The sort of the listed slices, their numbers in ws->h_ctr.
+qcp_status segmented_sort(qcp_index* ix, Workspace* ws, cudaStream_t s);
 
 qcp_status run_batched_counts_into(qcp_index* ix, const float* boxes, uint32_t q, uint64_t* counts,
                                    uint2* items0, uint2* items1, size_t item_cap, uint32_t* ctr, cudaStream_t s);

@@ -2,8 +2,7 @@
 // into a CUDA graph and replayed (qcp_plan_create / qcp_plan_run).
 //
 // qcp_query_batch decides buffer sizes and launch shapes on the host between
-// its phases (one readback after counting, one after classifying the slices,
-// one for the tile count).  A plan fixes them up front instead -- at most
+// its phases (one readback after counting).  A plan fixes them up front instead -- at most
 // max_queries boxes, at most max_hits ids -- so the whole pipeline (frontier
 // expansion, count, scan, write, per-query sort) runs from device-resident
 // counts with fixed grids (run_batched_device) and is captured into one
@@ -85,6 +84,7 @@ extern "C" qcp_status qcp_plan_create(qcp_index* ix, uint32_t max_queries, uint6
   do {
     const size_t row = 2 * (size_t)ix->dims;
     if ((st = ws_reserve_queries(ix, ws, max_queries)) != QCP_OK) break;
+    ws->qboxes = ws->boxes;
     // (query, node) items per frontier: 64 per query plus one per 1024 hits
     if ((st = ws_reserve_items(ix, ws, (size_t)max_queries * 64 + (size_t)(max_hits >> 10) + (1u << 16))) != QCP_OK)
       break;
@@ -132,6 +132,14 @@ extern "C" qcp_status qcp_plan_create(qcp_index* ix, uint32_t max_queries, uint6
       st = cuda_status(cudaGetLastError(), "qcp_plan_create");
       break;
     }
+    if (cudaStreamCreateWithFlags(&ws->side, cudaStreamNonBlocking) != cudaSuccess) {
+      st = cuda_status(cudaGetLastError(), "qcp_plan_create");
+      break;
+    }
+    for (cudaEvent_t& e : ws->side_ev)
+      if (st == QCP_OK && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess)
+        st = cuda_status(cudaGetLastError(), "qcp_plan_create");
+    if (st != QCP_OK) break;
     // one plain run first: kernel attributes are set up outside the capture
     if ((st = run_batched_device(ix, ws, max_queries, max_hits, p->sort, p->tables, p->capture)) != QCP_OK) break;
     if (cudaStreamSynchronize(p->capture) != cudaSuccess) {

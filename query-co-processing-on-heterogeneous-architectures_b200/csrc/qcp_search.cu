@@ -880,23 +880,6 @@ __global__ void __launch_bounds__(256) k_mprs(TreeView t, const float* __restric
   }
 }
 
-// Output capacity gate of the fixed-capacity pipeline: when the batch's
-// total hits exceed the id buffer, flag it (bit 2 of *flag) and empty the
-// write pass's item list; k_gate_zero then empties every slice, so the
-// write and sort passes that follow do nothing.
-__global__ void k_gate(const unsigned long long* __restrict__ offsets, uint32_t q, unsigned long long cap,
-                       uint32_t* item_count, uint32_t* flag) {
-  if (blockIdx.x == 0 && threadIdx.x == 0 && offsets[q] > cap) {
-    atomicOr(flag, 2u);
-    *item_count = 0;
-  }
-}
-
-__global__ void k_gate_zero(unsigned long long* offsets, uint32_t q, const uint32_t* __restrict__ flag) {
-  if (!(*flag & 2u)) return;
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i <= q; i += gridDim.x * blockDim.x) offsets[i] = 0;
-}
-
 // in == nullptr: the root level of nroot queries.
 template <int D>
 void launch_expand(uint32_t grid, cudaStream_t s, const float* boxes, const uint2* in,
@@ -982,7 +965,7 @@ static qcp_status expand_level(qcp_index* ix, Workspace* ws, uint32_t l, int cur
   const TreeView t = view_of(ix);
   const uint32_t grid = (uint32_t)num_sms() * ws->blocks_per_sm;
   uint32_t* ctr = ws->ctr;
-  QCP_DISPATCH_D(ix->dims, launch_expand<DD>(grid, s, ws->boxes, cur < 0 ? nullptr : ws->items[cur],
+  QCP_DISPATCH_D(ix->dims, launch_expand<DD>(grid, s, ws->qboxes, cur < 0 ? nullptr : ws->items[cur],
                                              ctr + kCtrFrontier0 + (cur < 0 ? 0 : cur), nroot,
                                              ws->items[nxt], ctr + kCtrFrontier0 + nxt, ws->items_cap,
                                              t.mbr[l - 1], t.nodes[l - 1], t.pad[l - 1], t.fanout,
@@ -1038,7 +1021,7 @@ static qcp_status count_items(qcp_index* ix, Workspace* ws, uint32_t q, int cur,
   uint32_t* ctr = ws->ctr;
   const HitCache hc = counts_only ? HitCache{} : hit_cache_of(ws);
   qcp_status st = QCP_OK;
-  QCP_DISPATCH_D(ix->dims, st = launch_count<DD>(ix->is_rect != 0, order_nodes(ix, q), ws->blocks_per_sm, s, t, ws->boxes, ws->items[cur],
+  QCP_DISPATCH_D(ix->dims, st = launch_count<DD>(ix->is_rect != 0, order_nodes(ix, q), ws->blocks_per_sm, s, t, ws->qboxes, ws->items[cur],
                                                 ctr + kCtrFrontier0 + cur, ctr + kCtrWork, ws->qcount,
                                                 ws->items_cap, ws->timing ? ws->d_stats : nullptr, hc));
   return st;
@@ -1048,12 +1031,32 @@ static qcp_status write_items(qcp_index* ix, Workspace* ws, int cur, cudaStream_
   const TreeView t = view_of(ix);
   const uint32_t grid = (uint32_t)num_sms() * ws->blocks_per_sm;
   uint32_t* ctr = ws->ctr;
-  QCP_DISPATCH_D(ix->dims, launch_leafwrite<DD>(ix->is_rect != 0, grid, s, t, ws->boxes, ws->items[cur],
-                                                ctr + kCtrFrontier0 + cur, ctr + kCtrWork, hit_cache_of(ws),
+  QCP_DISPATCH_D(ix->dims, launch_leafwrite<DD>(ix->is_rect != 0, grid, s, t, ws->qboxes, ws->items[cur],
+                                                ctr + kCtrFrontier0 + cur, ctr + kCtrWrite, hit_cache_of(ws),
                                                 ws->offsets, ws->qcursor, ws->out_ids, ws->items_cap,
                                                 ws->hist_G ? ws->qwhist : nullptr, ws->hist_G, ws->hist_bits));
   note_launch();
   return check_launch("k_leafwrite");
+}
+
+// The call's counters to the host (and the total to h_total).
+static qcp_status read_counters(Workspace* ws, cudaStream_t s) {
+  QCP_CUDA(cudaMemcpyAsync(ws->h_ctr, ws->ctr, sizeof(uint32_t) * kCtrCount, cudaMemcpyDeviceToHost, s));
+  QCP_CUDA(cudaStreamSynchronize(s));
+  memcpy(ws->h_total, ws->h_ctr + kCtrTotal, sizeof(uint64_t));
+  return QCP_OK;
+}
+
+// The bounded waits of the window sort's bulk prefetch.
+static qcp_status check_timeout(Workspace* ws, cudaStream_t s) {
+  QCP_CUDA(cudaMemcpyAsync(ws->h_ctr + kCtrTimeout, ws->ctr + kCtrTimeout, sizeof(uint32_t), cudaMemcpyDeviceToHost,
+                           s));
+  QCP_CUDA(cudaStreamSynchronize(s));
+  if (ws->h_ctr[kCtrTimeout]) {
+    set_error("a bounded wait for a bulk copy ran out in the sort");
+    return QCP_ERR_TIMEOUT;
+  }
+  return QCP_OK;
 }
 
 qcp_status run_batched(qcp_index* ix, Workspace* ws, uint32_t q, bool counts_only, bool sort,
@@ -1066,8 +1069,7 @@ qcp_status run_batched(qcp_index* ix, Workspace* ws, uint32_t q, bool counts_onl
   ws->use_hit_cache = false;
   for (int attempt = 0; attempt < 8; ++attempt) {
     mark(ws, kEvStart, s);
-    QCP_CUDA(cudaMemsetAsync(ctr, 0, sizeof(uint32_t) * kCtrCount, s));
-    QCP_CUDA(cudaMemsetAsync(ws->qcount, 0, sizeof(uint64_t) * q, s));
+    QCP_CUDA(ws_zero(ws, q, s));
     if (ws->timing) QCP_CUDA(cudaMemsetAsync(ws->d_stats, 0, sizeof(unsigned long long) * kStatCount, s));
     // the GPU's first level: the root's, or the hand-off level of a CPU + GPU
     // co-processing call whose host threads walked the levels above
@@ -1111,12 +1113,13 @@ qcp_status run_batched(qcp_index* ix, Workspace* ws, uint32_t q, bool counts_onl
                                   ws->use_hit_cache && !ws->hmask_cap ? (size_t)1 << 21 : 0));
     QCP_TRY(count_items(ix, ws, q, cur, counts_only, s));
     mark(ws, kEvCount, s);
-    QCP_TRY(exclusive_scan_counts(ws->qcount, ws->offsets, q, ix->pool, s));
+    if (!counts_only) {
+      QCP_TRY(exclusive_scan_counts(ws->qcount, ws->offsets, q, ix->pool, s));
+      QCP_TRY(classify_slices(ix, ws, q, sort, ~0ull, nullptr, s));
+    }
     mark(ws, kEvScan, s);
-    // one readback: overflow flags, items needed, total hits
-    QCP_CUDA(cudaMemcpyAsync(ws->h_ctr, ctr, sizeof(uint32_t) * kCtrCount, cudaMemcpyDeviceToHost, s));
-    QCP_CUDA(cudaMemcpyAsync(ws->h_total, ws->offsets + q, sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
-    QCP_CUDA(cudaStreamSynchronize(s));
+    // one readback: overflow flags, items needed, total hits, job counts
+    QCP_TRY(read_counters(ws, s));
     if (ws->h_ctr[kCtrOverflow]) {
       size_t need = (size_t)ws->h_ctr[kCtrNeedItems];
       if (need < ws->items_cap * 2) need = ws->items_cap * 2;
@@ -1127,10 +1130,9 @@ qcp_status run_batched(qcp_index* ix, Workspace* ws, uint32_t q, bool counts_onl
     const uint64_t total = *ws->h_total;
     QCP_TRY(ws_reserve_out(ix, ws, (size_t)total));
     if (total) {
-      QCP_CUDA(cudaMemsetAsync(ws->qcursor, 0, sizeof(uint64_t) * q, s));
-      QCP_CUDA(cudaMemsetAsync(ctr + kCtrWork, 0, sizeof(uint32_t), s));
       ws->hist_G = 0;
-      if (sort) {  // the write pass counts ids per (query, sort window)
+      const bool windows = sort && ws->h_ctr[kCtrJobs1];
+      if (windows) {  // the write pass counts ids per (query, sort window)
         uint32_t wbits = 0, G = 0;
         sort_window_shape(ix, ws, &wbits, &G);
         if (G <= kHistMaxG) {
@@ -1142,16 +1144,9 @@ qcp_status run_batched(qcp_index* ix, Workspace* ws, uint32_t q, bool counts_onl
       }
       QCP_TRY(write_items(ix, ws, cur, s));
       mark(ws, kEvWrite, s);
-      if (sort) QCP_TRY(segmented_sort(ix, ws, q, s));
+      if (sort) QCP_TRY(segmented_sort(ix, ws, s));
       mark(ws, kEvSort, s);
-      // bounded waits of the window sort's bulk prefetch
-      QCP_CUDA(cudaMemcpyAsync(ws->h_ctr + kCtrTimeout, ctr + kCtrTimeout, sizeof(uint32_t),
-                               cudaMemcpyDeviceToHost, s));
-      QCP_CUDA(cudaStreamSynchronize(s));
-      if (ws->h_ctr[kCtrTimeout]) {
-        set_error("a bounded wait for a bulk copy ran out in the sort");
-        return QCP_ERR_TIMEOUT;
-      }
+      if (windows) QCP_TRY(check_timeout(ws, s));
     }
     // hit bits that did not fit this call were tested again by the write
     // pass; the next call gets room for them (after this call's passes)
@@ -1179,28 +1174,33 @@ qcp_status run_plain(qcp_index* ix, Workspace* ws, uint32_t q, bool counts_only,
   uint32_t grid = q ? q : 1;
   if (grid > (uint32_t)num_sms() * 64) grid = (uint32_t)num_sms() * 64;
   mark(ws, kEvStart, s);
+  QCP_CUDA(ws_zero(ws, 0, s));
   mark(ws, kEvExpand, s);
-  QCP_DISPATCH_D(D, launch_mprs<DD, kCount>(rect, grid, threads, s, t, ws->boxes, q, ws->qcount,
+  QCP_DISPATCH_D(D, launch_mprs<DD, kCount>(rect, grid, threads, s, t, ws->qboxes, q, ws->qcount,
                                             nullptr, nullptr));
   note_launch();
   QCP_TRY(check_launch("k_mprs<count>"));
   mark(ws, kEvCount, s);
+  if (counts_only) {
+    mark(ws, kEvScan, s);
+    return QCP_OK;
+  }
   QCP_TRY(exclusive_scan_counts(ws->qcount, ws->offsets, q, ix->pool, s));
+  QCP_TRY(classify_slices(ix, ws, q, sort, ~0ull, nullptr, s));
   mark(ws, kEvScan, s);
-  QCP_CUDA(cudaMemcpyAsync(ws->h_total, ws->offsets + q, sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
-  QCP_CUDA(cudaStreamSynchronize(s));
-  if (counts_only) return QCP_OK;
+  QCP_TRY(read_counters(ws, s));
   const uint64_t total = *ws->h_total;
   QCP_TRY(ws_reserve_out(ix, ws, (size_t)total));
   if (total) {
     ws->hist_G = 0;  // the sort counts its windows itself
-    QCP_DISPATCH_D(D, launch_mprs<DD, kWrite>(rect, grid, threads, s, t, ws->boxes, q, nullptr,
+    QCP_DISPATCH_D(D, launch_mprs<DD, kWrite>(rect, grid, threads, s, t, ws->qboxes, q, nullptr,
                                               ws->offsets, ws->out_ids));
     note_launch();
     QCP_TRY(check_launch("k_mprs<write>"));
     mark(ws, kEvWrite, s);
-    if (sort) QCP_TRY(segmented_sort(ix, ws, q, s));
+    if (sort) QCP_TRY(segmented_sort(ix, ws, s));
     mark(ws, kEvSort, s);
+    if (sort && ws->sort_msd_jobs) QCP_TRY(check_timeout(ws, s));
   }
   return QCP_OK;
 }
@@ -1260,8 +1260,11 @@ qcp_status run_batched_device(qcp_index* ix, Workspace* ws, uint32_t q, uint64_t
   uint32_t* ctr = ws->ctr;
   const uint32_t start = (ix->levels >= 2) ? ix->levels - 1 : 1;
   ws->use_hit_cache = ws->hmask != nullptr;
-  QCP_CUDA(cudaMemsetAsync(ctr, 0, sizeof(uint32_t) * kCtrCount, s));
-  QCP_CUDA(cudaMemsetAsync(ws->qcount, 0, sizeof(uint64_t) * q, s));
+  if (ws->hist_G) {  // needed by the write pass only: beside the traversal
+    QCP_CUDA(ws_branch(ws, 0, s, ws->side));
+    QCP_CUDA(cudaMemsetAsync(ws->qwhist, 0, sizeof(uint32_t) * q * ws->hist_G, ws->side));
+  }
+  QCP_CUDA(ws_zero(ws, q, s));
   int cur = 0;
   if (start == 1) QCP_TRY(init_items(ws, q, s));
   for (uint32_t l = start; l > 1; --l) {
@@ -1274,13 +1277,9 @@ qcp_status run_batched_device(qcp_index* ix, Workspace* ws, uint32_t q, uint64_t
   if (order_nodes(ix, q)) QCP_TRY(order_items(ix, ws, &cur, s));
   QCP_TRY(count_items(ix, ws, q, cur, false, s));
   QCP_TRY(exclusive_scan_counts(ws->qcount, ws->offsets, q, ix->pool, s, ws->scan_tmp, ws->scan_tmp_cap));
-  k_gate<<<1, 32, 0, s>>>((const unsigned long long*)ws->offsets, q, ids_cap, ctr + kCtrFrontier0 + cur,
-                          ctr + kCtrOverflow);
-  k_gate_zero<<<(q + 256) / 256, 256, 0, s>>>((unsigned long long*)ws->offsets, q, ctr + kCtrOverflow);
-  note_launch(2);
-  QCP_CUDA(cudaMemsetAsync(ws->qcursor, 0, sizeof(uint64_t) * q, s));
-  QCP_CUDA(cudaMemsetAsync(ctr + kCtrWork, 0, sizeof(uint32_t), s));
-  if (ws->hist_G) QCP_CUDA(cudaMemsetAsync(ws->qwhist, 0, sizeof(uint32_t) * q * ws->hist_G, s));
+  // a batch of more than ids_cap ids: flagged, nothing written or sorted
+  QCP_TRY(classify_slices(ix, ws, q, sort, ids_cap, ctr + kCtrFrontier0 + cur, s));
+  if (ws->hist_G) QCP_CUDA(ws_branch(ws, 1, ws->side, s));
   QCP_TRY(write_items(ix, ws, cur, s));
   if (sort) QCP_TRY(segmented_sort_device(ix, ws, q, sort_tables, s));
   return check_launch("batched pipeline (device counts)");

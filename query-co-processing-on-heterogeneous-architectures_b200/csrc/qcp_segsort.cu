@@ -536,12 +536,25 @@ __global__ void __launch_bounds__(kSmallThreads, 4) k_sort_small(const Job* __re
 // Window partition
 // ============================================================================
 // Job lists by slice size: slices of <= kTinyCap ids from the front of
-// `small` (count *ntiny), slices of <= kSmallCap ids from its back (small[cap -
-// 1 - k], count *nsmall), larger ones in `big`.  Slices of 0 or 1 ids are
-// sorted already.
-__global__ void k_classify(const unsigned long long* __restrict__ offsets, uint32_t q, Job* small,
-                           uint32_t* ntiny, uint32_t* nsmall, size_t cap, Job* big, uint32_t* nbig,
-                           unsigned long long* big_ids) {
+// `small` (count ctr[kCtrJobs0]), slices of <= kSmallCap ids from its back
+// (small[cap - 1 - k], count ctr[kCtrSmall]), larger ones in `big`
+// (ctr[kCtrJobs1]), each with the first of its tiles (tile_off, their number
+// in ctr[kCtrTiles]; any order of the slices does).  Slices of 0 or 1 ids are
+// sorted already.  The batch's total goes to ctr[kCtrTotal]; more than ids_cap
+// ids set bit 2 of ctr[kCtrOverflow], empty the write pass's item list and
+// list nothing.  small == nullptr: no lists.
+__global__ void k_classify(const unsigned long long* __restrict__ offsets, uint32_t q, Job* small, size_t cap,
+                           Job* big, uint32_t* tile_off, uint32_t* ctr, unsigned long long ids_cap,
+                           uint32_t* item_count, unsigned long long* big_ids) {
+  const unsigned long long total = offsets[q];
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    *reinterpret_cast<unsigned long long*>(ctr + kCtrTotal) = total;
+    if (total > ids_cap) {
+      atomicOr(ctr + kCtrOverflow, 2u);
+      if (item_count) *item_count = 0;
+    }
+  }
+  if (!small || total > ids_cap) return;
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < q; i += gridDim.x * blockDim.x) {
     const unsigned long long off = offsets[i];
     const unsigned long long sz = offsets[i + 1] - off;
@@ -551,29 +564,24 @@ __global__ void k_classify(const unsigned long long* __restrict__ offsets, uint3
     j.size = (uint32_t)sz;
     j.q = i;
     if (sz <= kTinyCap) {
-      small[atomicAdd(ntiny, 1u)] = j;
+      small[atomicAdd(ctr + kCtrJobs0, 1u)] = j;
     } else if (sz <= kSmallCap) {
-      small[cap - 1 - atomicAdd(nsmall, 1u)] = j;
+      small[cap - 1 - atomicAdd(ctr + kCtrSmall, 1u)] = j;
     } else {
-      big[atomicAdd(nbig, 1u)] = j;
+      const uint32_t at = atomicAdd(ctr + kCtrJobs1, 1u);
+      big[at] = j;
+      tile_off[at] = atomicAdd(ctr + kCtrTiles, (uint32_t)((sz + kTile - 1) / kTile));
       if (big_ids) atomicAdd(big_ids, sz);
     }
   }
 }
 
-// tiles[j] for j < nmax: tiles of job j, 0 past the job count
-__global__ void k_tiles_per_job(const Job* __restrict__ jobs, const uint32_t* __restrict__ njobs_p, uint32_t nmax,
-                                uint32_t* tiles) {
-  const uint32_t njobs = *njobs_p;
-  for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < nmax; j += gridDim.x * blockDim.x)
-    tiles[j] = j < njobs ? (jobs[j].size + kTile - 1) / kTile : 0u;
-}
-
-__global__ void k_tile_map(const uint32_t* __restrict__ tiles, const uint32_t* __restrict__ tile_off,
+// tile -> job
+__global__ void k_tile_map(const Job* __restrict__ jobs, const uint32_t* __restrict__ tile_off,
                            const uint32_t* __restrict__ njobs_p, uint32_t* map) {
   const uint32_t njobs = *njobs_p;
   for (uint32_t j = blockIdx.x; j < njobs; j += gridDim.x) {
-    const uint32_t t0 = tile_off[j], nt = tiles[j];
+    const uint32_t t0 = tile_off[j], nt = (jobs[j].size + kTile - 1) / kTile;
     for (uint32_t k = threadIdx.x; k < nt; k += blockDim.x) map[t0 + k] = j;
   }
 }
@@ -1076,18 +1084,24 @@ static void launch_win_sort_t(uint64_t max_pairs, uint32_t sms, const uint32_t* 
 
 // The windows of a call: k_win_split lists them (counts in ctr[kCtrWinBig],
 // ctr[kCtrWinSmall], zeroed by the caller), the bitmap sort takes the large
-// ones and one warp each the small ones.  lists holds 2 * max_pairs entries;
+// ones and one warp each the small ones, in a plan (ws->side) on its second
+// branch.  lists holds 2 * max_pairs entries;
 // max_pairs bounds the (job, window) pairs.
-static void launch_win_sort(Workspace* ws, uint64_t max_pairs, uint32_t sms, const uint32_t* njobs, uint32_t G,
-                            uint32_t wbits, const uint32_t* whist, const unsigned long long* wbase, uint32_t* lists,
-                            uint32_t* ctr, const int32_t* src, int32_t* out, uint32_t* err, cudaStream_t s,
-                            bool stats) {
+static qcp_status launch_win_sort(Workspace* ws, uint64_t max_pairs, uint32_t sms, const uint32_t* njobs, uint32_t G,
+                                  uint32_t wbits, const uint32_t* whist, const unsigned long long* wbase, uint32_t* lists,
+                                  uint32_t* ctr, const int32_t* src, int32_t* out, uint32_t* err, cudaStream_t s,
+                                  bool stats) {
   uint32_t* big = lists;
   uint32_t* small = lists + max_pairs;
   const uint64_t split_blocks = (max_pairs + 255) / 256;
   k_win_split<<<(uint32_t)(split_blocks < (uint64_t)sms * 8 ? split_blocks : (uint64_t)sms * 8), 256, 0, s>>>(
       njobs, G, whist, big, ctr + kCtrWinBig, small, ctr + kCtrWinSmall,
       stats && ws->timing ? ws->d_stats + kStatBitmapIds : nullptr);
+  cudaStream_t warp_s = s;
+  if (ws->side) {
+    warp_s = ws->side;
+    QCP_CUDA(ws_branch(ws, 3, s, warp_s));
+  }
   if (wbits >= 18) launch_win_sort_t<18>(max_pairs, sms, big, ctr + kCtrWinBig, G, wbits, whist, wbase, src, out, err, s);
   else if (wbits == 17) launch_win_sort_t<17>(max_pairs, sms, big, ctr + kCtrWinBig, G, wbits, whist, wbase, src, out, err, s);
   else launch_win_sort_t<16>(max_pairs, sms, big, ctr + kCtrWinBig, G, wbits, whist, wbase, src, out, err, s);
@@ -1095,7 +1109,8 @@ static void launch_win_sort(Workspace* ws, uint64_t max_pairs, uint32_t sms, con
   const uint64_t warp_blocks = (max_pairs + kTinyWarps - 1) / kTinyWarps;
   const uint64_t warp_cap = (uint64_t)sms * kWinWarpBlocks;
   k_win_sort_warp<<<(uint32_t)(warp_blocks < warp_cap ? warp_blocks : warp_cap), kTinyWarps * 32,
-                    sizeof(TinySmem<kWinWarpMax>), s>>>(small, ctr + kCtrWinSmall, G, wbits, whist, wbase, src, out);
+                    sizeof(TinySmem<kWinWarpMax>), warp_s>>>(small, ctr + kCtrWinSmall, G, wbits, whist, wbase, src, out);
+  return QCP_OK;
 }
 
 static qcp_status set_sort_attrs(const qcp_index* ix, size_t scatter_max) {
@@ -1120,27 +1135,80 @@ static qcp_status set_sort_attrs(const qcp_index* ix, size_t scatter_max) {
   return QCP_OK;
 }
 
-qcp_status sort_small_slices(qcp_index* ix, Workspace* ws, uint32_t q, cudaStream_t s,
-                             const SortJob** big_out, uint32_t* nbig_out) {
-  *big_out = nullptr;
-  *nbig_out = 0;
-  ws->sort_small_jobs = ws->sort_msd_jobs = 0;
-  if (q == 0) return QCP_OK;
+qcp_status classify_slices(qcp_index* ix, Workspace* ws, uint32_t q, bool sort, uint64_t cap, uint32_t* item_count,
+                           cudaStream_t s) {
+  if (sort) QCP_TRY(ws_reserve_sort(ix, ws, (size_t)q + 256, 0));
+  k_classify<<<(q + 255) / 256, 256, 0, s>>>((const unsigned long long*)ws->offsets, q,
+                                             sort ? reinterpret_cast<Job*>(ws->jobs[0]) : nullptr, ws->jobs_cap,
+                                             reinterpret_cast<Job*>(ws->jobs[1]), ws->job_tiles, ws->ctr, cap,
+                                             item_count, ws->timing ? ws->d_stats + kStatWindowIds : nullptr);
+  note_launch();
+  return check_launch("k_classify");
+}
+
+// The tables of the window partition for at most njobs slices: counts (u32),
+// bases and cursors (u64) per (slice, window), and the two window lists.
+struct SortTables {
+  uint32_t* whist;
+  unsigned long long *wbase, *wcur;
+  uint32_t* lists;
+  size_t bytes;
+  SortTables(void* p, size_t njobs, uint32_t G) {
+    const size_t nw = njobs * G;
+    const size_t hist_bytes = (nw * 4 + 15) & ~(size_t)15;
+    char* c = static_cast<char*>(p);
+    whist = reinterpret_cast<uint32_t*>(c);
+    wbase = reinterpret_cast<unsigned long long*>(c + hist_bytes);
+    wcur = wbase + nw;
+    lists = reinterpret_cast<uint32_t*>(wcur + nw);  // 2 * nw
+    bytes = hist_bytes + nw * 24 + 64;
+  }
+};
+
+// The windows of the larger slices: partition and sort, over at most njobs
+// slices and ntiles tiles.  stats: a call that reports phase times.
+static qcp_status sort_windows(qcp_index* ix, Workspace* ws, size_t njobs, uint64_t ntiles, const SortTables& t,
+                               uint32_t G, uint32_t wbits, cudaStream_t s, bool stats) {
+  const uint32_t sms = (uint32_t)num_sms();
+  const uint32_t nsets = (G <= kPerWarpMaxG) ? kTileWarps : 1u;
+  const size_t scatter_bytes = (size_t)G * (8 + 4 * nsets) + kTile * 4;
+  const size_t nw = njobs * G;
+  uint32_t* ctr = ws->ctr;
+  const Job* big = reinterpret_cast<const Job*>(ws->jobs[1]);
+  auto at_most = [](uint64_t a, uint64_t b) { return (uint32_t)(a < b ? a : b); };
+  k_tile_map<<<at_most(njobs, sms * 8), 256, 0, s>>>(big, ws->job_tiles, ctr + kCtrJobs1, ws->seg_hist);
+  // per-(job, window) counts: from the write pass when it gathered them
+  const bool have_counts = ws->hist_G == G && ws->hist_bits == wbits;
+  if (!have_counts) {
+    QCP_CUDA(cudaMemsetAsync(t.whist, 0, sizeof(uint32_t) * nw, s));
+    k_win_hist<<<at_most(ntiles, sms * 8), kTileThreads, sizeof(uint32_t) * G, s>>>(
+        big, ws->seg_hist, ws->job_tiles, ctr + kCtrTiles, ws->out_ids, G, wbits, t.whist);
+    note_launch();
+  }
+  k_win_scan<<<at_most(njobs, sms * 16), kTileThreads, 0, s>>>(big, ctr + kCtrJobs1, G, t.whist,
+                                                               have_counts ? ws->qwhist : nullptr, t.wbase, t.wcur);
+  k_win_scatter<<<at_most(ntiles, sms * scatter_blocks_per_sm(scatter_bytes)), kTileThreads, scatter_bytes, s>>>(
+      big, ws->seg_hist, ws->job_tiles, ctr + kCtrTiles, ws->out_ids, ws->tmp_ids, G, wbits, t.wcur);
+  if (stats) {
+    mark(ws, kEvSortPart, s);
+    ws->sort_part_marked = ws->timing;
+  }
+  // (the window lists' counters are zero since the call's start)
+  QCP_TRY(launch_win_sort(ws, nw, sms, ctr + kCtrJobs1, G, wbits, t.whist, t.wbase, t.lists, ctr, ws->tmp_ids,
+                          ws->out_ids, ctr + kCtrTimeout, s, stats));
+  note_launch(6);
+  return check_launch("segmented sort windows");
+}
+
+static constexpr size_t kScatterMax = (size_t)(1u << (31 - kWinBits)) * 16 + kTile * 4;
+
+qcp_status segmented_sort(qcp_index* ix, Workspace* ws, cudaStream_t s) {
+  ws->sort_part_marked = false;
   const uint32_t idbits = id_bits(ix->n);
   const uint32_t sms = (uint32_t)num_sms();
-  const size_t scatter_max = (size_t)(1u << (31 - kWinBits)) * 16 + kTile * 4;
-  QCP_TRY(set_sort_attrs(ix, scatter_max));
-  QCP_TRY(ws_reserve_sort(ix, ws, (size_t)q + 256, 0));
+  QCP_TRY(set_sort_attrs(ix, kScatterMax));
   uint32_t* ctr = ws->ctr;
-  QCP_CUDA(cudaMemsetAsync(ctr + kCtrJobs0, 0, sizeof(uint32_t) * 3, s));  // jobs0, jobs1, small
   Job* small = reinterpret_cast<Job*>(ws->jobs[0]);
-  Job* big = reinterpret_cast<Job*>(ws->jobs[1]);
-  k_classify<<<(q + 255) / 256, 256, 0, s>>>((const unsigned long long*)ws->offsets, q, small,
-                                             ctr + kCtrJobs0, ctr + kCtrSmall, ws->jobs_cap, big, ctr + kCtrJobs1,
-                                             ws->timing ? ws->d_stats + kStatWindowIds : nullptr);
-  note_launch();
-  QCP_CUDA(cudaMemcpyAsync(ws->h_ctr, ctr, sizeof(uint32_t) * kCtrCount, cudaMemcpyDeviceToHost, s));
-  QCP_CUDA(cudaStreamSynchronize(s));
   const uint32_t ntiny = ws->h_ctr[kCtrJobs0];
   const uint32_t nsmall = ws->h_ctr[kCtrSmall];
   const uint32_t nbig = ws->h_ctr[kCtrJobs1];
@@ -1148,104 +1216,24 @@ qcp_status sort_small_slices(qcp_index* ix, Workspace* ws, uint32_t q, cudaStrea
   ws->sort_msd_jobs = nbig;
   if (ntiny) {
     k_sort_tiny<<<min((ntiny + kTinyWarps - 1) / kTinyWarps, sms * kTinyBlocks), kTinyWarps * 32,
-                  sizeof(TinySmem<kTinyCap>), s>>>(
-        small, ctr + kCtrJobs0, ws->out_ids, idbits);
+                  sizeof(TinySmem<kTinyCap>), s>>>(small, ctr + kCtrJobs0, ws->out_ids, idbits);
     note_launch();
     QCP_TRY(check_launch("k_sort_tiny"));
   }
   if (nsmall) {
-    k_sort_small<<<min(nsmall, sms * 4), kSmallThreads, sizeof(BucketSmem), s>>>(small + ws->jobs_cap,
-                                                                                  ctr + kCtrSmall, ws->out_ids,
-                                                                                  idbits);
+    k_sort_small<<<min(nsmall, sms * 4), kSmallThreads, sizeof(BucketSmem), s>>>(
+        small + ws->jobs_cap, ctr + kCtrSmall, ws->out_ids, idbits);
     note_launch();
     QCP_TRY(check_launch("k_sort_small"));
   }
-  *big_out = big;
-  *nbig_out = nbig;
-  return QCP_OK;
-}
-
-qcp_status segmented_sort(qcp_index* ix, Workspace* ws, uint32_t q, cudaStream_t s) {
-  ws->sort_part_marked = false;
-  const Job* bigc = nullptr;
-  uint32_t nbig = 0;
-  QCP_TRY(sort_small_slices(ix, ws, q, s, &bigc, &nbig));
   mark(ws, kEvSortSmall, s);
   if (nbig == 0) return QCP_OK;
-  Job* big = const_cast<Job*>(bigc);
-  uint32_t* ctr = ws->ctr;
-  const uint32_t idbits = id_bits(ix->n);
-  // window bits of this call: at most kWinBits (the bitmap), at least what
-  // keeps the window count <= 8192 (the scatter's shared counters)
-  uint32_t wb = ws->win_bits ? ws->win_bits : kDefaultWinBits;
-  if (wb > kWinBits) wb = kWinBits;
-  if (idbits > 13 && wb < idbits - 13) wb = idbits - 13;
-  const uint32_t wbits = idbits < wb ? idbits : wb;
-  const uint32_t G = 1u << (idbits - wbits);
-  const uint32_t sms = (uint32_t)num_sms();
-  const uint32_t nsets = (G <= kPerWarpMaxG) ? kTileWarps : 1u;
-  const size_t scatter_bytes = (size_t)G * (8 + 4 * nsets) + kTile * 4;
-
-  // tables per (job, window): counts (u32), bases and cursors (u64); tiles
-  // and tile offsets per job
-  const size_t nw = (size_t)nbig * G;
-  const size_t hist_bytes = (nw * 4 + 15) & ~(size_t)15;
-  const size_t lists_off = (hist_bytes + nw * 16 + (size_t)nbig * 8 + 15) & ~(size_t)15;
-  const size_t bytes = lists_off + nw * 8 + 64;
-  void* tables = nullptr;
-  QCP_TRY(ix->pool.get(bytes, &tables));
-  uint32_t* whist = reinterpret_cast<uint32_t*>(tables);
-  unsigned long long* wbase = reinterpret_cast<unsigned long long*>(reinterpret_cast<char*>(tables) + hist_bytes);
-  unsigned long long* wcur = wbase + nw;
-  uint32_t* tiles = reinterpret_cast<uint32_t*>(wcur + nw);
-  uint32_t* tile_off = tiles + nbig;
-  uint32_t* lists = reinterpret_cast<uint32_t*>(reinterpret_cast<char*>(tables) + lists_off);  // 2 * nw
-  qcp_status st = QCP_OK;
-  do {
-    k_tiles_per_job<<<(nbig + 255) / 256, 256, 0, s>>>(big, ctr + kCtrJobs1, nbig, tiles);
-    note_launch();
-    st = exclusive_scan<uint32_t>(tiles, tile_off, nbig, ctr + kCtrWork2, ix->pool, s);
-    if (st != QCP_OK) break;
-    if (cudaMemcpyAsync(ws->h_ctr + kCtrWork2, ctr + kCtrWork2, sizeof(uint32_t), cudaMemcpyDeviceToHost, s) !=
-            cudaSuccess ||
-        cudaStreamSynchronize(s) != cudaSuccess) {
-      st = cuda_status(cudaGetLastError(), "segmented sort tiles");
-      break;
-    }
-    const uint32_t ntiles = ws->h_ctr[kCtrWork2];
-    st = ws_reserve_sort(ix, ws, 0, ntiles);
-    if (st != QCP_OK) break;
-    uint32_t* map = ws->seg_hist;
-    k_tile_map<<<min(nbig, sms * 8), 256, 0, s>>>(tiles, tile_off, ctr + kCtrJobs1, map);
-    // per-(job, window) counts: from the write pass when it gathered them
-    const bool have_counts = ws->hist_G == G && ws->hist_bits == wbits;
-    if (!have_counts) {
-      if (cudaMemsetAsync(whist, 0, sizeof(uint32_t) * nw, s) != cudaSuccess) {
-        st = cuda_status(cudaGetLastError(), "memset");
-        break;
-      }
-      k_win_hist<<<min(ntiles, sms * 8), kTileThreads, sizeof(uint32_t) * G, s>>>(
-          big, map, tile_off, ctr + kCtrWork2, ws->out_ids, G, wbits, whist);
-    }
-    k_win_scan<<<min(nbig, sms * 16), kTileThreads, 0, s>>>(big, ctr + kCtrJobs1, G, whist,
-                                                            have_counts ? ws->qwhist : nullptr, wbase, wcur);
-    k_win_scatter<<<min(ntiles, sms * scatter_blocks_per_sm(scatter_bytes)), kTileThreads, scatter_bytes, s>>>(
-        big, map, tile_off, ctr + kCtrWork2, ws->out_ids, ws->tmp_ids, G, wbits, wcur);
-    mark(ws, kEvSortPart, s);
-    ws->sort_part_marked = ws->timing;
-    if (cudaMemsetAsync(ctr + kCtrWinBig, 0, 2 * sizeof(uint32_t), s) != cudaSuccess) {
-      st = cuda_status(cudaGetLastError(), "memset");
-      break;
-    }
-    launch_win_sort(ws, nw, sms, ctr + kCtrJobs1, G, wbits, whist, wbase, lists, ctr, ws->tmp_ids, ws->out_ids,
-                    ctr + kCtrTimeout, s, true);
-    note_launch(7);
-    st = check_launch("segmented sort windows");
-    // the tables go back to the pool below: make sure the kernels are done
-    if (st == QCP_OK && cudaStreamSynchronize(s) != cudaSuccess) st = cuda_status(cudaGetLastError(), "sort");
-  } while (false);
-  ix->pool.put(bytes, tables);
-  return st;
+  uint32_t wbits = 0, G = 0;
+  sort_window_shape(ix, ws, &wbits, &G);
+  const uint32_t ntiles = ws->h_ctr[kCtrTiles];
+  QCP_TRY(ws_reserve_sort(ix, ws, 0, ntiles));
+  QCP_TRY(ws_reserve_tables(ws, SortTables(nullptr, nbig, G).bytes));
+  return sort_windows(ix, ws, nbig, ntiles, SortTables(ws->tables, nbig, G), G, wbits, s, true);
 }
 
 
@@ -1270,66 +1258,37 @@ void sort_window_shape(const qcp_index* ix, const Workspace* ws, uint32_t* wbits
 size_t sort_tables_bytes(const qcp_index* ix, const Workspace* ws, uint32_t q) {
   uint32_t wbits = 0, G = 0;
   window_shape(ix, ws, &wbits, &G);
-  const size_t nw = (size_t)q * G;
-  const size_t lists_off = ((((nw * 4 + 15) & ~(size_t)15) + nw * 16 + (size_t)q * 8) + 15) & ~(size_t)15;
-  return lists_off + nw * 8 + 64;
+  return SortTables(nullptr, q, G).bytes;
 }
 
-// segmented_sort without host readbacks: job and tile counts stay on the
-// device, every launch has a fixed grid and the kernels read the counts.
-// Tables (sort_tables_bytes) and the tile map (at least total/kSortTile + q
-// entries, ws->seg_hist) are the caller's.  Stream-capturable.
+// segmented_sort without host readbacks, for at most max_ids ids: job and tile
+// counts stay on the device, every launch has a fixed grid and the kernels
+// read the counts.  The slices and windows that single CTAs and warps sort run
+// on ws->side beside the window partition and the bitmap sort: each of the
+// kernels leaves most of the chip idle on a plan's small batch (a run of 64
+// boxes on 16 M points, 62 us of it sort kernels: 194 -> 153 us with this
+// branch and the tiles numbered by k_classify instead of a scan).
+// Tables (sort_tables_bytes) and the tile map (at least
+// max_ids / kSortTile + q entries, ws->seg_hist) are the caller's.
+// Stream-capturable.
 qcp_status segmented_sort_device(qcp_index* ix, Workspace* ws, uint32_t q, void* tables, cudaStream_t s) {
   if (q == 0) return QCP_OK;
   const uint32_t idbits = id_bits(ix->n);
   uint32_t wbits = 0, G = 0;
   window_shape(ix, ws, &wbits, &G);
   const uint32_t sms = (uint32_t)num_sms();
-  const size_t scatter_max = (size_t)(1u << (31 - kWinBits)) * 16 + kTile * 4;
-  QCP_TRY(set_sort_attrs(ix, scatter_max));
-  const uint32_t nsets = (G <= kPerWarpMaxG) ? kTileWarps : 1u;
-  const size_t scatter_bytes = (size_t)G * (8 + 4 * nsets) + kTile * 4;
+  QCP_TRY(set_sort_attrs(ix, kScatterMax));
   uint32_t* ctr = ws->ctr;
   Job* small = reinterpret_cast<Job*>(ws->jobs[0]);
-  Job* big = reinterpret_cast<Job*>(ws->jobs[1]);
-  const size_t nw = (size_t)q * G;
-  const size_t hist_bytes = (nw * 4 + 15) & ~(size_t)15;
-  uint32_t* whist = reinterpret_cast<uint32_t*>(tables);
-  unsigned long long* wbase = reinterpret_cast<unsigned long long*>(reinterpret_cast<char*>(tables) + hist_bytes);
-  unsigned long long* wcur = wbase + nw;
-  uint32_t* tiles = reinterpret_cast<uint32_t*>(wcur + nw);
-  uint32_t* tile_off = tiles + q;
-  const size_t lists_off = (hist_bytes + nw * 16 + (size_t)q * 8 + 15) & ~(size_t)15;
-  uint32_t* lists = reinterpret_cast<uint32_t*>(reinterpret_cast<char*>(tables) + lists_off);  // 2 * nw
-  QCP_CUDA(cudaMemsetAsync(ctr + kCtrJobs0, 0, sizeof(uint32_t) * 3, s));  // jobs0, jobs1, small
-  k_classify<<<(q + 255) / 256, 256, 0, s>>>((const unsigned long long*)ws->offsets, q, small, ctr + kCtrJobs0,
-                                             ctr + kCtrSmall, ws->jobs_cap,
-                                             big, ctr + kCtrJobs1, nullptr);
-  k_sort_tiny<<<sms * kTinyBlocks, kTinyWarps * 32, sizeof(TinySmem<kTinyCap>), s>>>(small, ctr + kCtrJobs0, ws->out_ids, idbits);
-  k_sort_small<<<sms * 4, kSmallThreads, sizeof(BucketSmem), s>>>(small + ws->jobs_cap, ctr + kCtrSmall,
-                                                                  ws->out_ids, idbits);
-  note_launch();
-  k_tiles_per_job<<<(q + 255) / 256, 256, 0, s>>>(big, ctr + kCtrJobs1, q, tiles);
-  note_launch(3);
-  QCP_TRY(exclusive_scan<uint32_t>(tiles, tile_off, q, ctr + kCtrWork2, ix->pool, s, ws->scan_tmp,
-                                   ws->scan_tmp_cap));
-  k_tile_map<<<sms * 8, 256, 0, s>>>(tiles, tile_off, ctr + kCtrJobs1, ws->seg_hist);
-  const bool have_counts = ws->hist_G == G && ws->hist_bits == wbits;
-  if (!have_counts) {
-    QCP_CUDA(cudaMemsetAsync(whist, 0, sizeof(uint32_t) * nw, s));
-    k_win_hist<<<sms * 8, kTileThreads, sizeof(uint32_t) * G, s>>>(big, ws->seg_hist, tile_off, ctr + kCtrWork2,
-                                                                   ws->out_ids, G, wbits, whist);
-  }
-  k_win_scan<<<sms * 16, kTileThreads, 0, s>>>(big, ctr + kCtrJobs1, G, whist, have_counts ? ws->qwhist : nullptr,
-                                               wbase, wcur);
-  k_win_scatter<<<sms * scatter_blocks_per_sm(scatter_bytes), kTileThreads, scatter_bytes, s>>>(
-      big, ws->seg_hist, tile_off, ctr + kCtrWork2,
-                                                             ws->out_ids, ws->tmp_ids, G, wbits, wcur);
-  QCP_CUDA(cudaMemsetAsync(ctr + kCtrWinBig, 0, 2 * sizeof(uint32_t), s));
-  launch_win_sort(ws, nw, sms, ctr + kCtrJobs1, G, wbits, whist, wbase, lists, ctr, ws->tmp_ids, ws->out_ids,
-                  ctr + kCtrTimeout, s, false);
-  note_launch(7);
-  return check_launch("segmented sort (device counts)");
+  QCP_CUDA(ws_branch(ws, 2, s, ws->side));
+  k_sort_tiny<<<sms * kTinyBlocks, kTinyWarps * 32, sizeof(TinySmem<kTinyCap>), ws->side>>>(
+      small, ctr + kCtrJobs0, ws->out_ids, idbits);
+  k_sort_small<<<sms * 4, kSmallThreads, sizeof(BucketSmem), ws->side>>>(small + ws->jobs_cap, ctr + kCtrSmall,
+                                                                         ws->out_ids, idbits);
+  note_launch(2);
+  QCP_TRY(sort_windows(ix, ws, q, ~0ull, SortTables(tables, q, G), G, wbits, s, false));
+  QCP_CUDA(ws_branch(ws, 4, ws->side, s));
+  return QCP_OK;
 }
 
 }  // namespace qcp
