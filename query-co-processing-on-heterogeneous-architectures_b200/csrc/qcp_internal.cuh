@@ -13,6 +13,7 @@
 namespace qcp {
 
 constexpr int kMaxLevels = 16;
+constexpr uint32_t kMaxFanout = 256;
 constexpr int kMaxDims = 8;
 constexpr uint32_t kWarp = 32;
 
