@@ -318,6 +318,14 @@ qcp_status ws_reserve_qwhist(Workspace* ws, size_t n) {
   return QCP_OK;
 }
 
+// The second branch's stream and events, made by the first call that needs them.
+qcp_status ws_reserve_side(Workspace* ws) {
+  if (!ws->side) QCP_CUDA(cudaStreamCreateWithFlags(&ws->side, cudaStreamNonBlocking));
+  for (cudaEvent_t& e : ws->side_ev)
+    if (!e) QCP_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  return QCP_OK;
+}
+
 qcp_status ws_reserve_tables(Workspace* ws, size_t bytes) { return grow(&ws->tables, &ws->tables_cap, bytes, 4096); }
 
 // Counts and cursors per level-1 node and the scratch of their scan.
@@ -654,6 +662,7 @@ static qcp_status run_query(qcp_index* ix, const float* boxes, uint32_t q, const
   }
   if (st != QCP_OK) {
     cudaStreamSynchronize(s);
+    if (ws->side) cudaStreamSynchronize(ws->side);
     ws_release(ix, ws);
     return st;
   }

@@ -139,7 +139,7 @@ struct Workspace {
   uint4* jobs[2] = {nullptr, nullptr};
   uint32_t* job_tiles = nullptr; // first tile of every larger slice
   size_t jobs_cap = 0;
-  cudaStream_t side = nullptr;   // plans: the captured pipeline's second branch
+  cudaStream_t side = nullptr;   // second branch of the sort (and of a plan's pipeline)
   cudaEvent_t side_ev[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
   char* tables = nullptr;        // the window partition's tables
   size_t tables_cap = 0;
@@ -498,6 +498,7 @@ constexpr size_t kMaxMaskWords = 0xc0000000u;        // hit-bit words (32-bit of
 qcp_status ws_reserve_hitcache(Workspace* ws, size_t recs, size_t mask_words);
 qcp_status ws_reserve_nodes(Workspace* ws, size_t nodes);
 qcp_status ws_reserve_tables(Workspace* ws, size_t bytes);
+qcp_status ws_reserve_side(Workspace* ws);
 // Workspace construction and buffer reservation (qcp_capi.cu).
 qcp_status ws_reserve_queries(qcp_index* ix, Workspace* ws, uint32_t q);
 qcp_status ws_reserve_items(qcp_index* ix, Workspace* ws, size_t items);

@@ -132,14 +132,7 @@ extern "C" qcp_status qcp_plan_create(qcp_index* ix, uint32_t max_queries, uint6
       st = cuda_status(cudaGetLastError(), "qcp_plan_create");
       break;
     }
-    if (cudaStreamCreateWithFlags(&ws->side, cudaStreamNonBlocking) != cudaSuccess) {
-      st = cuda_status(cudaGetLastError(), "qcp_plan_create");
-      break;
-    }
-    for (cudaEvent_t& e : ws->side_ev)
-      if (st == QCP_OK && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess)
-        st = cuda_status(cudaGetLastError(), "qcp_plan_create");
-    if (st != QCP_OK) break;
+    if ((st = ws_reserve_side(ws)) != QCP_OK) break;
     // one plain run first: kernel attributes are set up outside the capture
     if ((st = run_batched_device(ix, ws, max_queries, max_hits, p->sort, p->tables, p->capture)) != QCP_OK) break;
     if (cudaStreamSynchronize(p->capture) != cudaSuccess) {
