@@ -477,10 +477,13 @@ __device__ __forceinline__ bool whole_items(uint32_t nitems, uint32_t G, uint32_
 // no barriers.  Few items share a node, so nothing is staged: the box sits in
 // registers, a group's MBRs are tested one per lane, and the partially covered
 // leaves one after the other.  Bound by the latency of its dependent reads
-// (item, box and MBRs, objects).  1,000 boxes over 1 M points: 18.9 (a warp
-// per item) -> 12.4 us; 64 boxes over 16 M points 36.7 -> 14.8 us.
+// (item, box and MBRs, objects); the CTAs per SM are what the registers of a
+// box, its MBRs and four objects allow without spills (61,000 8-D points, 7,768
+// boxes: 110 -> 45 us with three instead of four and no MBRs ahead).  1,000
+// boxes over 1 M points: 18.9 (a warp per item) -> 12.4 us; 64 boxes over 16 M
+// points 36.7 -> 14.8 us.
 template <int D, bool RECT>
-__global__ void __launch_bounds__(256, (RECT ? 2 * D : D) > 8 ? 2 : 4)
+__global__ void __launch_bounds__(256, (RECT ? 2 * D : D) > 8 ? 2 : (RECT ? 2 * D : D) > 3 ? 3 : 4)
     k_count(TreeView t, const float* __restrict__ boxes, const uint2* __restrict__ items,
             const uint32_t* __restrict__ item_count, unsigned long long* qcount, uint64_t item_cap,
             uint64_t nodes, unsigned long long* stats, HitCache hc) {
@@ -509,7 +512,8 @@ __global__ void __launch_bounds__(256, (RECT ? 2 * D : D) > 8 ? 2 : 4)
     }
     uint32_t total = 0;  // hits of the unit
     const uint32_t ga = whole ? 0u : (uint32_t)(u % G), gb = whole ? G : ga + 1;
-    float mlo[D], mhi[D];  // the next group's MBRs, loaded one group ahead
+    float mlo[D], mhi[D];  // a group's MBRs, with few dimensions loaded one group ahead
+    constexpr bool kMbrAhead = D <= 4;
     auto load_mbrs = [&](uint32_t g) {
       const uint64_t at = (uint64_t)it.y * F + g * 32 + lane;
 #pragma unroll
@@ -518,8 +522,9 @@ __global__ void __launch_bounds__(256, (RECT ? 2 * D : D) > 8 ? 2 : 4)
         mhi[d] = __ldg(lmbr + (D + d) * lpad + at);
       }
     };
-    load_mbrs(ga);
+    if (kMbrAhead) load_mbrs(ga);
     for (uint32_t g = ga; g < gb; ++g) {
+      if (!kMbrAhead) load_mbrs(g);
       const uint64_t l0 = (uint64_t)it.y * F + g * 32;  // the group's first leaf
       bool ov = l0 + lane < nleaves, in = true;
 #pragma unroll
@@ -527,7 +532,7 @@ __global__ void __launch_bounds__(256, (RECT ? 2 * D : D) > 8 ? 2 : 4)
         ov &= overlaps1(-b[2 * d], b[2 * d + 1], mlo[d], mhi[d]);
         in &= inside1(-b[2 * d], b[2 * d + 1], mlo[d], mhi[d]);
       }
-      if (g + 1 < gb) load_mbrs(g + 1);
+      if (kMbrAhead && g + 1 < gb) load_mbrs(g + 1);
       const uint32_t mov = __ballot_sync(0xffffffffu, ov), mcov = __ballot_sync(0xffffffffu, ov && in);
       const uint32_t part = mov & ~mcov;
       // room for the hit bits; the objects' reads do not wait for it
