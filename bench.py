@@ -117,7 +117,8 @@ def dist_setup(n_gpus):
 
 def algorithmic_bytes(st: dict, dims: int, fanout: int, is_rect: bool = False, hit_cache: bool = True) -> dict:
     """Bytes each kernel must move at minimum for the work it did, per launch
-    (one launch of each per step):
+    (one launch of each per step; k_leafscan<count> and <write> name the count
+    and the write pass, whose kernels are k_join or k_count, and k_leafwrite):
     k_leafscan<count>  leaf-MBR reads of every (query, leaf-parent) item +
                        coordinates of partially covered leaves (+ with the hit
                        cache, its records written: 12 B per item and 32-leaf
@@ -956,7 +957,7 @@ def main():
     ap.add_argument("--lanes-per-item", type=int, default=0,
                     help="lanes per (query, node) item of the level expansion with --no-tune (0: 32)")
     ap.add_argument("--leaf-prefetch", type=int, default=0,
-                    help="leaf prefetch buffers per warp with --no-tune (0: default 2, 1: none)")
+                    help="accepted by the library, without effect")
     ap.add_argument("--plain-steps", type=int, default=2)
     ap.add_argument("--e2e-steps", type=int, default=4)
     ap.add_argument("--e2e-streams", type=int, default=2,

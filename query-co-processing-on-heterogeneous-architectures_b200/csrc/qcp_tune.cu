@@ -5,17 +5,15 @@
 // The reference fixes its node size at compile time (NODE_SIZE,
 // src/common/config.h) and has no tuner.  Here the fan-out is a build option
 // and two query knobs are exposed through qcp_query_opts:
-//   blocks_per_sm  grid of the traversal kernels (k_expand, k_leafscan) in
+//   blocks_per_sm  grid of the traversal kernels (k_expand, k_leafwrite) in
 //                  256-thread blocks per SM; their work is fetched from a
 //                  device counter, so the grid sets only how many items are
 //                  in flight per SM;
 //   win_bits       id window of the per-query sort (2^win_bits ids per
 //                  bitmap), which trades partition fan-out against the
 //                  density of the window bitmaps;
-//   leaf_prefetch  the leaf tile of the traversal's leaf passes: how many
-//                  partially covered leaves each warp keeps in flight in its
-//                  shared-memory ring (bulk copies), or none, which trades
-//                  latency hiding against CTAs per SM;
+//   leaf_prefetch  accepted by the query, without effect: its trials only keep
+//                  their place in the list;
 //   lanes_per_item queries per warp of the level expansion: 32, 16 or 8
 //                  lanes per (query, node) item;
 //   hit_cache      the count pass's leaf masks and hit bits replayed by the
@@ -166,7 +164,7 @@ extern "C" qcp_status qcp_autotune(const float* objs, uint64_t n, uint32_t dims,
       }
     }
     if (st != QCP_OK) break;
-    // 4. leaf tile: no ring (1), or 3 buffers per warp instead of 2
+    // 4. leaf_prefetch (without effect)
     for (uint32_t lp : {1u, 3u}) {
       const Trial tr = time_batch(best_ix, (const float*)d_boxes, q, s, best_b, best_w, lp, best_lpi, best_hc, repeats, e0, e1);
       if ((st = tr.st) != QCP_OK) break;
