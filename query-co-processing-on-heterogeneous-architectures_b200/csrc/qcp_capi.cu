@@ -37,6 +37,19 @@ qcp_status check_launch(const char* what) {
   return QCP_OK;
 }
 
+// Calls that allocate and synchronise are refused on a stream that is being
+// captured, before they touch anything: an allocation on such a stream becomes
+// a node of the caller's graph, whose address backs nothing until that graph
+// runs, and a workspace that kept it would hand it to a later call.
+static qcp_status refuse_capture(cudaStream_t s) {
+  cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+  cudaError_t e = cudaStreamIsCapturing(s, &c);
+  if (e == cudaSuccess && c != cudaStreamCaptureStatusNone) e = cudaErrorStreamCaptureUnsupported;
+  if (e == cudaSuccess) return QCP_OK;
+  cudaGetLastError();
+  return cuda_status(e, "stream");
+}
+
 // ---------------------------------------------------------------------------
 // Pools
 // ---------------------------------------------------------------------------
@@ -489,6 +502,7 @@ static qcp_status build_impl(const float* objs, uint64_t n, uint32_t dims, uint3
     return QCP_ERR_NO_DEVICE;
   }
   cudaStream_t s = (cudaStream_t)o.stream;
+  QCP_TRY(refuse_capture(s));
   AllocOn on(s);
   qcp_index* ix = new (std::nothrow) qcp_index();
   if (!ix) return QCP_ERR_OOM;
@@ -600,6 +614,7 @@ static qcp_status run_query(qcp_index* ix, const float* boxes, uint32_t q, const
     return QCP_ERR_BAD_ARG;
   }
   cudaStream_t s = (cudaStream_t)o.stream;
+  QCP_TRY(refuse_capture(s));
   AllocOn on(s);
   Workspace* ws = ws_acquire(ix);
   if (!ws) return QCP_ERR_OOM;
