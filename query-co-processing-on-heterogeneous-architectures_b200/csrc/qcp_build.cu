@@ -146,18 +146,21 @@ __global__ void __launch_bounds__(256) k_keys(const float* __restrict__ objs, ui
 // ---------------------------------------------------------------------------
 constexpr int RS_THREADS = 256;
 constexpr int RS_WARPS = RS_THREADS / 32;
-#ifndef RSI
-#define RSI 12
-#define RSB 4
-#endif
-constexpr int RS_ITEMS = RSI;
+constexpr int RS_ITEMS = 12;
 constexpr int RS_TILE = RS_THREADS * RS_ITEMS;
 constexpr int RS_PER_WARP = RS_TILE / RS_WARPS;
 constexpr uint32_t RS_MAX_PASSES = 8;
 constexpr uint32_t RS_TOP = 4;          // sweeps over the top bits
 constexpr uint32_t kRunSort = 2048;     // pairs of a run that a CTA sorts in shared memory
 constexpr uint32_t kRunCap = 1u << 18;  // longest run of equal top bits that is ordered in place
-constexpr uint32_t RS_SPIN = 1u << 22;  // polls of the earlier tiles' statuses before a tile gives up
+constexpr uint32_t RS_POLLS = 1u << 22; // polls of the earlier tiles' statuses before a tile gives up
+constexpr uint32_t kSortTimeout = 2;    // error bit of a tile that did
+
+// The build's kernels from the sort on return at once where the bit is set: the
+// pairs are then incomplete, and nothing of them may be used as an index.
+__device__ __forceinline__ bool sort_timed_out(const uint32_t* err) {
+  return *reinterpret_cast<const volatile uint32_t*>(err) & kSortTimeout;
+}
 
 // Scratch: digit counts (then offsets) and tile tickets of every sweep, the
 // largest key, the flag, and per tile and digit a status word: (2 sweep + 1 or
@@ -275,13 +278,13 @@ __device__ __forceinline__ uint32_t block_excl_scan256(uint32_t v, uint32_t* war
 // run is written contiguously.  The slots past a short last tile's end count
 // as its last pairs of digit 255 and are not written.  Tiles are taken by
 // ticket, so every tile that one waits for is running or done; a wait is
-// bounded all the same (RS_SPIN polls, then *err |= 2 and a prefix that is too
-// low: in bounds, wrong order).  vals_in == nullptr: the values are the
-// positions.
+// bounded all the same: after `polls` polls the tile sets kSortTimeout in *err
+// and its CTA leaves without writing the tile.  vals_in == nullptr: the values
+// are the positions.
 __global__ void __launch_bounds__(RS_THREADS, 3) k_rs_sweep(
     const uint64_t* __restrict__ keys_in, const uint32_t* __restrict__ vals_in, uint64_t* __restrict__ keys_out,
     uint32_t* __restrict__ vals_out, uint64_t n, uint32_t ntiles, uint32_t sweep, RsScratch* rs, uint64_t* status,
-    uint32_t* err) {
+    uint32_t polls, uint32_t* err) {
   __shared__ uint64_t skeys[RS_TILE];
   __shared__ uint32_t svals[RS_TILE];
   __shared__ uint32_t gofs[256];  // output position of the digit's first pair minus its slot in the tile
@@ -292,6 +295,7 @@ __global__ void __launch_bounds__(RS_THREADS, 3) k_rs_sweep(
   uint32_t* wcnt = reinterpret_cast<uint32_t*>(skeys);
   static_assert(RS_WARPS * 256 <= 2 * RS_TILE, "the counters fit the stage");
   const uint32_t tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  if (__syncthreads_or(tid == 0 && sort_timed_out(err))) return;  // (another CTA may be setting it)
   const uint32_t shift = rs_shift(rs, sweep);
   const uint32_t digit0 = rs->hist[sweep][tid];  // first output position of this thread's digit
   const uint32_t partial = 2 * sweep + 1, inclusive = 2 * sweep + 2;
@@ -371,6 +375,7 @@ __global__ void __launch_bounds__(RS_THREADS, 3) k_rs_sweep(
     }
     // look-back: counts of the digit in the earlier tiles, four statuses at a time
     uint32_t before = 0;
+    bool gave_up = false;
     if (tile) {
       int64_t t = (int64_t)tile - 1;
       uint32_t spins = 0;
@@ -387,15 +392,15 @@ __global__ void __launch_bounds__(RS_THREADS, 3) k_rs_sweep(
           done = (uint32_t)(st[j] >> 32) == inclusive;
           --t;
         }
-        if (!done && ++spins > RS_SPIN) {
-          atomicOr(err, 2u);
-          done = true;
+        if (!done && ++spins > polls) {
+          atomicOr(err, kSortTimeout);
+          done = gave_up = true;
         }
       }
-      st_status(mine, (uint64_t)inclusive << 32 | (before + real));
+      if (!gave_up) st_status(mine, (uint64_t)inclusive << 32 | (before + real));
     }
     gofs[tid] = digit0 + before - ex;
-    __syncthreads();
+    if (__syncthreads_or(gave_up)) return;
 #pragma unroll 4
     for (uint32_t i = tid; i < tile_n; i += RS_THREADS) {
       const uint64_t key = skeys[i];
@@ -412,7 +417,9 @@ __global__ void __launch_bounds__(RS_THREADS, 3) k_rs_sweep(
 // k_rs_runs.  Other threads only compare their key with the one before.
 // (Insertion by one thread up to 32 keys took 148 us on 16 M clustered points:
 // a chain of dependent reads per step.)
-__global__ void k_rs_ties(uint64_t* keys, uint32_t* vals, uint64_t n, RsScratch* rs, uint2* runs, uint64_t cap) {
+__global__ void k_rs_ties(uint64_t* keys, uint32_t* vals, uint64_t n, RsScratch* rs, uint2* runs, uint64_t cap,
+                          const uint32_t* err) {
+  if (sort_timed_out(err)) return;
   const uint32_t shift = rs_shift(rs, 0);
   if (shift == 0) return;  // the top bits were all of them
   for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i + 1 < n;
@@ -486,7 +493,9 @@ __device__ __forceinline__ void sort_in_smem(uint64_t* sk, uint32_t* sv, uint32_
 //   Where they are not few the flag is set instead.
 __global__ void __launch_bounds__(RS_THREADS) k_rs_runs(uint64_t* keys, uint32_t* vals, uint64_t* ktmp,
                                                         uint32_t* vtmp, RsScratch* rs,
-                                                        const uint2* __restrict__ runs, uint64_t cap) {
+                                                        const uint2* __restrict__ runs, uint64_t cap,
+                                                        const uint32_t* err) {
+  if (sort_timed_out(err)) return;
   __shared__ uint64_t sk[kRunSort];
   __shared__ uint32_t sv[kRunSort];
   __shared__ uint32_t warp_tot[RS_WARPS];
@@ -701,7 +710,7 @@ __global__ void __launch_bounds__(1024) k_scan_one(const T* __restrict__ in, T* 
 }
 
 // objs -> sorted SoA arrays and the leaves' MBRs; flags non-finite coordinates
-// in *bad.  A block packs blockDim.x / fanout whole leaves at a time, one
+// in *bad (bit 1) and does nothing where the sort timed out.  A block packs blockDim.x / fanout whole leaves at a time, one
 // object per thread, so a leaf's MBR comes from registers: every warp reduces
 // its 32 objects (as order-preserving integers), the leaf's warps meet in
 // shared memory.  Bound by the gather of whole rows in key order; the separate
@@ -737,6 +746,7 @@ __global__ void __launch_bounds__(256) k_pack(const float* __restrict__ objs, co
                                               uint64_t pad0, float* __restrict__ coords, int32_t* __restrict__ ids,
                                               float* __restrict__ mbr, uint32_t* bad) {
   constexpr int NC = RECT ? 2 * D : D;
+  if (sort_timed_out(bad)) return;
   __shared__ uint32_t wlo[8][D], whi[8][D];
   const uint32_t tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   const uint32_t per = blockDim.x / fanout;  // leaves per block and round
@@ -1022,6 +1032,13 @@ qcp_status build_keys(const float* objs, uint64_t n, uint32_t dims, uint32_t is_
   return st;
 }
 
+namespace {
+thread_local uint32_t t_sort_polls = RS_POLLS;
+}
+// For tests: most polls of a wait in the sorts that this host thread launches
+// (negative: the default).  Not part of the ABI.
+extern "C" void qcp_test_sort_polls(int polls) { t_sort_polls = polls < 0 ? RS_POLLS : (uint32_t)polls; }
+
 static uint64_t rs_run_cap(uint64_t n) { return n / 3 + 1; }  // runs of three pairs at least
 
 size_t radix_scratch_bytes(uint64_t n) {
@@ -1071,7 +1088,7 @@ qcp_status radix_sort_pairs(uint64_t* keys, uint32_t* vals, uint64_t* keys_tmp, 
     k_rs_offsets<<<1, np * 32, 0, s>>>(rs, p0);
     note_launch(2);
     for (uint32_t p = p0; p < p0 + np; ++p) {
-      k_rs_sweep<<<grid, RS_THREADS, 0, s>>>(kin, vin, kout, vout, n, ntiles, p, rs, status, err);
+      k_rs_sweep<<<grid, RS_THREADS, 0, s>>>(kin, vin, kout, vout, n, ntiles, p, rs, status, t_sort_polls, err);
       note_launch();
       kin = kout;
       vin = vout;
@@ -1084,8 +1101,9 @@ qcp_status radix_sort_pairs(uint64_t* keys, uint32_t* vals, uint64_t* keys_tmp, 
     if (key_bits > 32) {
       cudaMemcpyAsync(&rs->max_key, max_key, sizeof(uint64_t), cudaMemcpyDeviceToDevice, s);
       sweeps(0, RS_TOP);
-      k_rs_ties<<<grid_for(n, 256, sms * 16), 256, 0, s>>>(keys, vals, n, rs, runs, rs_run_cap(n));
-      k_rs_runs<<<sms * 4, RS_THREADS, 0, s>>>(keys, vals, keys_tmp, vals_tmp, rs, runs, rs_run_cap(n));
+      k_rs_ties<<<grid_for(n, 256, sms * 16), 256, 0, s>>>(keys, vals, n, rs, runs, rs_run_cap(n), err);
+      k_rs_runs<<<sms * 4, RS_THREADS, 0, s>>>(keys, vals, keys_tmp, vals_tmp, rs, runs, rs_run_cap(n),
+                                                 err);
       note_launch(2);
       // all digits, if a run was too long; an even number of sweeps, so that
       // the result is where it is without them
