@@ -139,10 +139,15 @@ __global__ void __launch_bounds__(256) k_keys(const float* __restrict__ objs, ui
 // k_rs_ties and k_rs_runs then order every run of equal top bits by the
 // rest, in place (a thread, a warp or a CTA per run); a run that cannot be
 // sets a flag, and only then do the sweeps over all digits
-// that follow do anything.  Bound by issue (ranking a pair) and the
+// that follow do anything.  Where objects lie close to one another many share
+// their top bits and the ties cost more than the four sweeps they save (16 M
+// objects in 64 clusters of deviation 0.005: 0.66 ms, 0.002: all twelve
+// sweeps), so large sorts sample the keys first and leave such to the sweeps
+// over all digits.  Bound by issue (ranking a pair) and the
 // pairs' traffic, 24 bytes per pair and sweep.  16 M pairs of 63 bits: an
 // upsweep, table scan and downsweep per digit, 8 digits, 1,284 us; this
-// 750-860 us (150 us a sweep), 2.2 ms where the flag is set.
+// 750-860 us (150 us a sweep), 1.3 ms over all digits, 2.2 ms where a run too
+// long for its place was not seen by the sample.
 // ---------------------------------------------------------------------------
 constexpr int RS_THREADS = 256;
 constexpr int RS_WARPS = RS_THREADS / 32;
@@ -156,13 +161,7 @@ constexpr uint32_t kRunCap = 1u << 18;  // longest run of equal top bits that is
 constexpr uint32_t RS_POLLS = 1u << 22; // polls of the earlier tiles' statuses before a tile gives up
 constexpr uint32_t kSortTimeout = 2;    // error bit of a tile that did
 
-// The build's kernels from the sort on return at once where the bit is set: the
-// pairs are then incomplete, and nothing of them may be used as an index.
-__device__ __forceinline__ bool sort_timed_out(const uint32_t* err) {
-  return *reinterpret_cast<const volatile uint32_t*>(err) & kSortTimeout;
-}
-
-// Scratch: digit counts (then offsets) and tile tickets of every sweep, the
+// Scratch: digit counts and tile tickets of every sweep, the
 // largest key, the flag, and per tile and digit a status word: (2 sweep + 1 or
 // 2) << 32 | count, odd = the tile's own count, even = the inclusive prefix.
 // Statuses of earlier sweeps (and the zeros before the first) are lower than
@@ -172,9 +171,22 @@ struct RsScratch {
   uint32_t ticket[RS_TOP + RS_MAX_PASSES];
   uint32_t long_run;  // nonzero: a run of equal top bits was too long
   uint32_t nruns, nlong;  // runs listed for k_rs_runs: of up to 32 pairs, longer
+  uint32_t shared;    // sampled keys that share their top bits with another one's
+  uint32_t failed;    // nonzero: a tile's wait ran out
   uint32_t pad_;
   unsigned long long max_key;
 };
+
+// Whether so many objects share their top bits that the sweeps over all digits
+// are the cheaper way from the start (tight: of more than this many sampled).
+__device__ __forceinline__ bool rs_tight(const RsScratch* rs, uint32_t tight) { return rs->shared > tight; }
+
+// Whether sweep p does anything: those over the top bits unless the keys are
+// tight, those over all digits if they are or a run turned out too long.
+__device__ __forceinline__ bool rs_runs(const RsScratch* rs, uint32_t p, uint32_t tight) {
+  const bool t = rs_tight(rs, tight);
+  return p < RS_TOP ? !t : t || rs->long_run;
+}
 
 // Lowest bit of sweep p's digit: p < RS_TOP: of the top 32 bits; otherwise
 // digit p - RS_TOP of the whole key.
@@ -189,17 +201,55 @@ __device__ __forceinline__ uint32_t rs_digit(uint64_t k, uint32_t shift) {
   return (shift < 32 ? __funnelshift_r(lo, hi, shift) : hi >> (shift - 32)) & 255u;
 }
 
-// Counts of the digits of sweeps [p0, p0 + np).
+// Samples m keys, one at a scattered place of each n / m, and counts those
+// whose top bits another sampled key has too, the rest of it being different
+// (equal keys cost the ties nothing), by a hash table of 2 m zeroed words.
+// Thread t of the m takes one.
+__device__ __forceinline__ void rs_sample(const uint64_t* keys, uint64_t n, uint32_t m, uint32_t t, RsScratch* rs,
+                                          unsigned long long* slots) {
+  const uint32_t mask = 2 * m - 1;
+  const uint32_t shift = rs_shift(rs, 0);
+  bool shares = false;
+  if (shift) {
+    const uint64_t step = n / m;
+    const unsigned long long k = keys[t * step + (t * 0x9e3779b1u >> 8) % step];
+    const unsigned long long top = k >> shift;
+    uint32_t at = (uint32_t)((top * 0x9e3779b97f4a7c15ull) >> 40) & mask;
+    // (a zero word is free, so the key 0 is not counted)
+    for (int probe = 0; k && probe < 16; ++probe, at = (at + 1) & mask) {
+      const unsigned long long old = atomicCAS(slots + at, 0ull, k);
+      if (old == 0) break;
+      if (old >> shift == top) {
+        shares = old != k;
+        break;
+      }
+    }
+  }
+  const uint32_t c = __popc(__ballot_sync(0xffffffffu, shares));
+  if ((threadIdx.x & 31) == 0 && c) atomicAdd(&rs->shared, c);
+}
+
+// Counts of the digits of sweeps [p0, p0 + np).  The first samples / kSampleBlock
+// blocks of the first pass take the sample instead, beside it (a kernel of its
+// own: 6 to 11 us), so the pass is made whatever the sample says.
+constexpr uint32_t kSampleBlock = 4 * RS_THREADS;  // keys that a block samples
 __global__ void __launch_bounds__(RS_THREADS) k_rs_hist(const uint64_t* __restrict__ keys, uint64_t n, uint32_t p0,
-                                                        uint32_t np, RsScratch* rs) {
+                                                        uint32_t np, uint32_t tight, uint32_t samples, RsScratch* rs,
+                                                        unsigned long long* slots) {
   __shared__ uint32_t h[RS_MAX_PASSES][256];
-  if (p0 >= RS_TOP && !rs->long_run) return;
+  if (p0 >= RS_TOP && !rs_runs(rs, p0, tight)) return;
+  const uint32_t sblocks = samples / kSampleBlock;
+  if (blockIdx.x < sblocks) {
+    for (uint32_t t = blockIdx.x * RS_THREADS + threadIdx.x; t < samples; t += sblocks * RS_THREADS)
+      rs_sample(keys, n, samples, t, rs, slots);
+    return;
+  }
   const uint32_t tid = threadIdx.x, lane = tid & 31;
   for (uint32_t i = tid; i < np * 256; i += RS_THREADS) (&h[0][0])[i] = 0;
   __syncthreads();
   const uint32_t shift0 = rs_shift(rs, p0);
-  const uint64_t stride = (uint64_t)gridDim.x * RS_THREADS;
-  for (uint64_t i0 = (uint64_t)blockIdx.x * RS_THREADS; i0 < n; i0 += 4 * stride) {
+  const uint64_t stride = (uint64_t)(gridDim.x - sblocks) * RS_THREADS;
+  for (uint64_t i0 = (uint64_t)(blockIdx.x - sblocks) * RS_THREADS; i0 < n; i0 += 4 * stride) {
     uint64_t k[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
@@ -226,25 +276,6 @@ __global__ void __launch_bounds__(RS_THREADS) k_rs_hist(const uint64_t* __restri
   __syncthreads();
   for (uint32_t p = 0; p < np; ++p)
     if (h[p][tid]) atomicAdd(&rs->hist[p0 + p][tid], h[p][tid]);
-}
-
-// Digit counts -> exclusive digit offsets, a warp per sweep.
-__global__ void k_rs_offsets(RsScratch* rs, uint32_t p0) {
-  if (p0 >= RS_TOP && !rs->long_run) return;
-  const uint32_t lane = threadIdx.x & 31, p = p0 + (threadIdx.x >> 5);
-  uint32_t c[8], t = 0;
-#pragma unroll
-  for (int k = 0; k < 8; ++k) {
-    c[k] = rs->hist[p][lane * 8 + k];
-    t += c[k];
-  }
-  uint32_t tot;
-  uint32_t run = warp_excl_sum(t, &tot);
-#pragma unroll
-  for (int k = 0; k < 8; ++k) {
-    rs->hist[p][lane * 8 + k] = run;
-    run += c[k];
-  }
 }
 
 __device__ __forceinline__ uint64_t ld_status(const uint64_t* p) {
@@ -279,29 +310,32 @@ __device__ __forceinline__ uint32_t block_excl_scan256(uint32_t v, uint32_t* war
 // as its last pairs of digit 255 and are not written.  Tiles are taken by
 // ticket, so every tile that one waits for is running or done; a wait is
 // bounded all the same: after `polls` polls the tile sets kSortTimeout in *err
-// and its CTA leaves without writing the tile.  vals_in == nullptr: the values
-// are the positions.
+// and its CTA leaves without writing the tile; the sweeps that follow then do
+// nothing.
 __global__ void __launch_bounds__(RS_THREADS, 3) k_rs_sweep(
     const uint64_t* __restrict__ keys_in, const uint32_t* __restrict__ vals_in, uint64_t* __restrict__ keys_out,
     uint32_t* __restrict__ vals_out, uint64_t n, uint32_t ntiles, uint32_t sweep, RsScratch* rs, uint64_t* status,
-    uint32_t polls, uint32_t* err) {
+    uint32_t tight, uint32_t polls, uint32_t* err) {
   __shared__ uint64_t skeys[RS_TILE];
   __shared__ uint32_t svals[RS_TILE];
   __shared__ uint32_t gofs[256];  // output position of the digit's first pair minus its slot in the tile
   __shared__ uint32_t warp_tot[RS_WARPS];
   __shared__ uint32_t s_tile;
-  if (sweep >= RS_TOP && !rs->long_run) return;
+  if (!rs_runs(rs, sweep, tight)) return;
+  // the first sweep that runs: the values are the positions
+  const bool first = sweep == 0 || (sweep == RS_TOP && rs_tight(rs, tight));
   // ranking counters [warp][digit], in the stage until the pairs go there
   uint32_t* wcnt = reinterpret_cast<uint32_t*>(skeys);
   static_assert(RS_WARPS * 256 <= 2 * RS_TILE, "the counters fit the stage");
   const uint32_t tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-  if (__syncthreads_or(tid == 0 && sort_timed_out(err))) return;  // (another CTA may be setting it)
   const uint32_t shift = rs_shift(rs, sweep);
-  const uint32_t digit0 = rs->hist[sweep][tid];  // first output position of this thread's digit
+  // first output position of this thread's digit
+  const uint32_t digit0 = block_excl_scan256(rs->hist[sweep][tid], warp_tot);
   const uint32_t partial = 2 * sweep + 1, inclusive = 2 * sweep + 2;
   const uint32_t lt = lane_lt_mask();
   for (;;) {
-    if (tid == 0) s_tile = atomicAdd(&rs->ticket[sweep], 1u);
+    // (after an expired wait the pairs are incomplete: no sweep may rank them)
+    if (tid == 0) s_tile = *(volatile uint32_t*)&rs->failed ? ntiles : atomicAdd(&rs->ticket[sweep], 1u);
     for (uint32_t i = tid; i < RS_WARPS * 256; i += RS_THREADS) wcnt[i] = 0;
     __syncthreads();
     const uint32_t tile = s_tile;
@@ -318,14 +352,14 @@ __global__ void __launch_bounds__(RS_THREADS, 3) k_rs_sweep(
       for (int r = 0; r < RS_ITEMS; ++r) k[r] = __ldcs(keys_in + base + l0 + r * 32);
 #pragma unroll
       for (int r = 0; r < RS_ITEMS; ++r)
-        v[r] = vals_in ? __ldcs(vals_in + base + l0 + r * 32) : (uint32_t)base + l0 + r * 32;
+        v[r] = first ? (uint32_t)base + l0 + r * 32 : __ldcs(vals_in + base + l0 + r * 32);
     } else {
 #pragma unroll
       for (int r = 0; r < RS_ITEMS; ++r) {
         const uint32_t li = l0 + r * 32;
         k[r] = li < tile_n ? __ldcs(keys_in + base + li) : ~0ull;
         v[r] = (uint32_t)base + li;
-        if (vals_in && li < tile_n) v[r] = __ldcs(vals_in + base + li);
+        if (!first && li < tile_n) v[r] = __ldcs(vals_in + base + li);
       }
     }
     uint32_t* wc = wcnt + w * 256;
@@ -393,6 +427,7 @@ __global__ void __launch_bounds__(RS_THREADS, 3) k_rs_sweep(
           --t;
         }
         if (!done && ++spins > polls) {
+          rs->failed = 1;
           atomicOr(err, kSortTimeout);
           done = gave_up = true;
         }
@@ -418,8 +453,8 @@ __global__ void __launch_bounds__(RS_THREADS, 3) k_rs_sweep(
 // (Insertion by one thread up to 32 keys took 148 us on 16 M clustered points:
 // a chain of dependent reads per step.)
 __global__ void k_rs_ties(uint64_t* keys, uint32_t* vals, uint64_t n, RsScratch* rs, uint2* runs, uint64_t cap,
-                          const uint32_t* err) {
-  if (sort_timed_out(err)) return;
+                          uint32_t tight) {
+  if (rs_tight(rs, tight)) return;
   const uint32_t shift = rs_shift(rs, 0);
   if (shift == 0) return;  // the top bits were all of them
   for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i + 1 < n;
@@ -493,9 +528,7 @@ __device__ __forceinline__ void sort_in_smem(uint64_t* sk, uint32_t* sv, uint32_
 //   Where they are not few the flag is set instead.
 __global__ void __launch_bounds__(RS_THREADS) k_rs_runs(uint64_t* keys, uint32_t* vals, uint64_t* ktmp,
                                                         uint32_t* vtmp, RsScratch* rs,
-                                                        const uint2* __restrict__ runs, uint64_t cap,
-                                                        const uint32_t* err) {
-  if (sort_timed_out(err)) return;
+                                                        const uint2* __restrict__ runs, uint64_t cap) {
   __shared__ uint64_t sk[kRunSort];
   __shared__ uint32_t sv[kRunSort];
   __shared__ uint32_t warp_tot[RS_WARPS];
@@ -710,7 +743,8 @@ __global__ void __launch_bounds__(1024) k_scan_one(const T* __restrict__ in, T* 
 }
 
 // objs -> sorted SoA arrays and the leaves' MBRs; flags non-finite coordinates
-// in *bad (bit 1) and does nothing where the sort timed out.  A block packs blockDim.x / fanout whole leaves at a time, one
+// in *bad (bit 1).  The permutation of a sort that timed out holds anything,
+// so positions are bounded.  A block packs blockDim.x / fanout whole leaves at a time, one
 // object per thread, so a leaf's MBR comes from registers: every warp reduces
 // its 32 objects (as order-preserving integers), the leaf's warps meet in
 // shared memory.  Bound by the gather of whole rows in key order; the separate
@@ -746,7 +780,6 @@ __global__ void __launch_bounds__(256) k_pack(const float* __restrict__ objs, co
                                               uint64_t pad0, float* __restrict__ coords, int32_t* __restrict__ ids,
                                               float* __restrict__ mbr, uint32_t* bad) {
   constexpr int NC = RECT ? 2 * D : D;
-  if (sort_timed_out(bad)) return;
   __shared__ uint32_t wlo[8][D], whi[8][D];
   const uint32_t tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   const uint32_t per = blockDim.x / fanout;  // leaves per block and round
@@ -758,7 +791,7 @@ __global__ void __launch_bounds__(256) k_pack(const float* __restrict__ objs, co
     if (i < npad) {
       float x[NC];
       if (i < n) {
-        const uint32_t id = __ldcs(perm + i);
+        const uint32_t id = min(__ldcs(perm + i), (uint32_t)n - 1);
         load_row<NC, V>(x, objs + (uint64_t)id * NC);
         bool finite = true;
 #pragma unroll
@@ -1041,9 +1074,26 @@ extern "C" void qcp_test_sort_polls(int polls) { t_sort_polls = polls < 0 ? RS_P
 
 static uint64_t rs_run_cap(uint64_t n) { return n / 3 + 1; }  // runs of three pairs at least
 
+// Objects from which the sort of long keys samples them first, and how many it
+// takes (of 1 M objects 65,536 cost a rebuild of 202 us 14, 16,384 two).
+constexpr uint64_t kSampleMin = 1u << 19;
+static uint32_t rs_samples(uint64_t n) { return n < kSampleMin ? 0u : (n < (1u << 23) ? 1u << 14 : 1u << 16); }
+
+// The sample's limit: what it counts where every object shares its top bits
+// with x n / m others (m samples in cells of x each).  From 2^21 objects 1.6
+// others: rebuilds of 16 M objects with 1, 2 and 4 of them take 1.94, 2.20 and
+// 2.29 ms by top bits and ties, 2.01 by all digits, of 4 M 0.55, 0.60 and 0.63
+// against 0.60.  Fewer objects leave the sweeps launch-bound, and only long
+// runs cost more than they do: 1 M objects with 4 and 1,000 others 0.25 and
+// 0.34 ms against 0.27.
+static uint32_t rs_tight_limit(uint64_t n) {
+  const double m = rs_samples(n), x = (n < (1u << 21) ? 16 : 1.6) * m / (double)n;
+  return m ? (uint32_t)(m * (1 + std::expm1(-x) / x)) : 0xffffffffu;
+}
+
 size_t radix_scratch_bytes(uint64_t n) {
   return sizeof(RsScratch) + sizeof(uint64_t) * 256 * (size_t)((n + RS_TILE - 1) / RS_TILE) +
-         sizeof(uint2) * (size_t)rs_run_cap(n);
+         sizeof(uint64_t) * 2 * rs_samples(n) + sizeof(uint2) * (size_t)rs_run_cap(n);
 }
 
 qcp_status radix_sort_pairs(uint64_t* keys, uint32_t* vals, uint64_t* keys_tmp, uint32_t* vals_tmp,
@@ -1069,7 +1119,9 @@ qcp_status radix_sort_pairs(uint64_t* keys, uint32_t* vals, uint64_t* keys_tmp, 
   }
   RsScratch* rs = static_cast<RsScratch*>(scratch);
   uint64_t* status = reinterpret_cast<uint64_t*>(rs + 1);
-  uint2* runs = reinterpret_cast<uint2*>(status + (size_t)ntiles * 256);
+  uint64_t* slots = status + (size_t)ntiles * 256;
+  uint2* runs = reinterpret_cast<uint2*>(slots + 2 * rs_samples(n));
+  const uint32_t tight = rs_tight_limit(n);
   const size_t clear = reinterpret_cast<char*>(runs) - static_cast<char*>(scratch);
   const uint32_t sms = num_sms();
   int fit = 1;
@@ -1079,16 +1131,18 @@ qcp_status radix_sort_pairs(uint64_t* keys, uint32_t* vals, uint64_t* keys_tmp, 
     st = cuda_status(cudaGetLastError(), "radix scratch");
   const uint32_t grid = ntiles < sms * fit ? ntiles : sms * fit;
   uint64_t* kin = keys;
-  uint32_t* vin = nullptr;  // the first sweep's values are the positions
+  uint32_t* vin = vals;  // (the first sweep's are the positions)
   uint64_t* kout = keys_tmp;
   uint32_t* vout = vals_tmp;
   // sweeps [p0, p0 + np)
   auto sweeps = [&](uint32_t p0, uint32_t np) {
-    k_rs_hist<<<grid_for(n, RS_THREADS * 8, sms * 8), RS_THREADS, 0, s>>>(kin, n, p0, np, rs);
-    k_rs_offsets<<<1, np * 32, 0, s>>>(rs, p0);
-    note_launch(2);
+    const uint32_t m = p0 == 0 && key_bits > 32 ? rs_samples(n) : 0, sb = m / kSampleBlock;
+    k_rs_hist<<<sb + grid_for(n, RS_THREADS * 8, sms * 8 - sb), RS_THREADS, 0, s>>>(
+        kin, n, p0, np, tight, m, rs, reinterpret_cast<unsigned long long*>(slots));
+    note_launch();
     for (uint32_t p = p0; p < p0 + np; ++p) {
-      k_rs_sweep<<<grid, RS_THREADS, 0, s>>>(kin, vin, kout, vout, n, ntiles, p, rs, status, t_sort_polls, err);
+      k_rs_sweep<<<grid, RS_THREADS, 0, s>>>(kin, vin, kout, vout, n, ntiles, p, rs, status, tight, t_sort_polls,
+                                             err);
       note_launch();
       kin = kout;
       vin = vout;
@@ -1101,9 +1155,8 @@ qcp_status radix_sort_pairs(uint64_t* keys, uint32_t* vals, uint64_t* keys_tmp, 
     if (key_bits > 32) {
       cudaMemcpyAsync(&rs->max_key, max_key, sizeof(uint64_t), cudaMemcpyDeviceToDevice, s);
       sweeps(0, RS_TOP);
-      k_rs_ties<<<grid_for(n, 256, sms * 16), 256, 0, s>>>(keys, vals, n, rs, runs, rs_run_cap(n), err);
-      k_rs_runs<<<sms * 4, RS_THREADS, 0, s>>>(keys, vals, keys_tmp, vals_tmp, rs, runs, rs_run_cap(n),
-                                                 err);
+      k_rs_ties<<<grid_for(n, 256, sms * 16), 256, 0, s>>>(keys, vals, n, rs, runs, rs_run_cap(n), tight);
+      k_rs_runs<<<sms * 4, RS_THREADS, 0, s>>>(keys, vals, keys_tmp, vals_tmp, rs, runs, rs_run_cap(n));
       note_launch(2);
       // all digits, if a run was too long; an even number of sweeps, so that
       // the result is where it is without them

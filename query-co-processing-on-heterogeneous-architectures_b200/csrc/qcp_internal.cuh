@@ -455,7 +455,7 @@ qcp_status build_keys(const float* objs, uint64_t n, uint32_t dims, uint32_t is_
 // vals_tmp are output only).  With `scratch` (at least radix_scratch_bytes(n))
 // nothing is allocated, so the sort can be captured into a graph.  *err |= 2
 // on the device when a bounded wait ran out; the pairs are then incomplete and
-// what follows has to leave them alone (build_pack does).
+// hold anything (build_pack stays in bounds).
 qcp_status radix_sort_pairs(uint64_t* keys, uint32_t* vals, uint64_t* keys_tmp, uint32_t* vals_tmp,
                             uint64_t n, uint32_t key_bits, const uint64_t* max_key, uint32_t* err, cudaStream_t s,
                             bool* result_in_tmp, void* scratch = nullptr, size_t scratch_bytes = 0);
