@@ -18,9 +18,6 @@
 #include <cfloat>
 #include <cmath>
 
-#include <mutex>
-#include <unordered_set>
-
 #include "qcp_internal.cuh"
 #include "qcp_tree.cuh"
 
@@ -894,110 +891,6 @@ int num_sms() {
       sms = 148;
   }
   return sms;
-}
-
-namespace {
-thread_local cudaStream_t t_alloc_stream = nullptr;
-
-// The current device's pool, created on first use.
-cudaError_t device_pool(cudaMemPool_t* out) {
-  static std::mutex mu;
-  static cudaMemPool_t pools[64] = {};
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
-  if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
-  std::lock_guard<std::mutex> g(mu);
-  if (!pools[dev]) {
-    cudaMemPoolProps props = {};
-    props.allocType = cudaMemAllocationTypePinned;
-    props.location.type = cudaMemLocationTypeDevice;
-    props.location.id = dev;
-    cudaMemPool_t p = nullptr;
-    if ((e = cudaMemPoolCreate(&p, &props)) != cudaSuccess) return e;
-    uint64_t keep = kPoolKeeps;
-    if ((e = cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep)) != cudaSuccess) {
-      cudaMemPoolDestroy(p);
-      return e;
-    }
-    pools[dev] = p;
-  }
-  *out = pools[dev];
-  return cudaSuccess;
-}
-
-// The pool keeps at most kPoolKeeps bytes beyond what is in use (the release
-// threshold counts both).  If it holds more than that although something had
-// to be added, what it keeps does not fit what is asked for now: all of it is
-// given back, or every synchronisation would release what the next call needs.
-void bound_pool(cudaMemPool_t pool) {
-  uint64_t reserved = 0, used = 0;
-  if (cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved) != cudaSuccess ||
-      cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess)
-    return;
-  uint64_t threshold = used + kPoolKeeps;
-  cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &threshold);
-  if (reserved > threshold) cudaMemPoolTrimTo(pool, used);
-}
-
-cudaError_t pool_malloc(void** p, size_t bytes, cudaStream_t s) {
-  cudaMemPool_t pool;
-  cudaError_t e = device_pool(&pool);
-  if (e != cudaSuccess) return e;
-  e = cudaMallocFromPoolAsync(p, bytes ? bytes : 1, pool, s);
-  if (e == cudaErrorMemoryAllocation) {
-    // once more without what the pool keeps
-    cudaGetLastError();
-    cudaStreamSynchronize(s);
-    cudaMemPoolTrimTo(pool, 0);
-    e = cudaMallocFromPoolAsync(p, bytes ? bytes : 1, pool, s);
-  }
-  if (e == cudaSuccess) bound_pool(pool);
-  return e;
-}
-}  // namespace
-
-namespace {
-std::mutex direct_mu;
-std::unordered_set<void*> direct;  // live allocations that are not the pool's
-thread_local bool t_lasting = false;
-}  // namespace
-
-cudaError_t dev_malloc_bytes(void** p, size_t bytes) {
-  if (bytes <= (t_lasting ? kPoolLargestLasting : kPoolLargest)) return pool_malloc(p, bytes, t_alloc_stream);
-  const cudaError_t e = cudaMalloc(p, bytes);
-  if (e == cudaSuccess) {
-    std::lock_guard<std::mutex> g(direct_mu);
-    direct.insert(*p);
-  }
-  return e;
-}
-void dev_free(void* p) {
-  if (!p) return;
-  bool is_direct;
-  {
-    std::lock_guard<std::mutex> g(direct_mu);
-    is_direct = direct.erase(p) != 0;
-  }
-  if (is_direct) cudaFree(p);
-  else cudaFreeAsync(p, t_alloc_stream);
-}
-AllocOn::AllocOn(cudaStream_t s) : before_(t_alloc_stream) { t_alloc_stream = s; }
-AllocOn::~AllocOn() { t_alloc_stream = before_; }
-AllocLasting::AllocLasting() { t_lasting = true; }
-AllocLasting::~AllocLasting() { t_lasting = false; }
-
-// Temporaries freed before the work that uses them has run: a buffer freed on
-// one stream is handed to another stream only after the freeing stream has
-// reached the free, so calls that run concurrently on different streams never
-// share one.
-qcp_status temp_alloc(size_t bytes, cudaStream_t s, void** out) {
-  QCP_CUDA(pool_malloc(out, bytes, s));
-  return QCP_OK;
-}
-
-void temp_free(void* p, cudaStream_t s) {
-  if (p) cudaFreeAsync(p, s);
 }
 
 size_t scan_scratch_bytes(uint64_t n) {

@@ -87,7 +87,7 @@ qcp_status DevPool::get(size_t bytes, void** out) {
   cudaError_t e = dev_malloc(&p, sz);
   if (e == cudaErrorMemoryAllocation) {
     cudaGetLastError();
-    trim();
+    trim();  // (dev_malloc then gives back what the pool got from it)
     e = dev_malloc(&p, sz);
   }
   if (e != cudaSuccess) return cuda_status(e, "cudaMalloc");
@@ -422,6 +422,7 @@ static void index_release(qcp_index* ix) {
   dev_free(ix->keys);
   for (int l = 0; l < kMaxLevels; ++l) dev_free(ix->mbr[l]);
   ix->pool.trim();
+  dev_give_back(ix->device);
   delete ix;
 }
 

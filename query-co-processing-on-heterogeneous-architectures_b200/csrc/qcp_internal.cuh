@@ -42,9 +42,10 @@ void note_launch(uint32_t k = 1);
 qcp_status check_launch(const char* what);
 
 // ---------------------------------------------------------------------------
-// Device memory: stream-ordered, from one pool per device that keeps at most
-// kPoolKeeps bytes that are not in use (more is given back to the device at
-// the next synchronisation, all of it when an allocation fails).  cudaMalloc
+// Device memory (qcp_mem.cu): stream-ordered, from one pool per device that
+// keeps at most kPoolKeeps bytes that are not in use (more is given back to the
+// device at the next synchronisation and when an index is freed, all of it when
+// an allocation, from the pool or not, finds no room).  cudaMalloc
 // and cudaFree per buffer were most of a one-shot build: 5 M 4-D rectangles
 // and 1,000 queries 8.0 -> 0.83 ms.  Allocations and frees are ordered on the
 // calling thread's AllocOn stream (the legacy stream outside any); whoever
@@ -60,6 +61,10 @@ constexpr uint64_t kPoolLargest = 256ull << 20;
 constexpr uint64_t kPoolLargestLasting = 4ull << 20;
 cudaError_t dev_malloc_bytes(void** p, size_t bytes);
 void dev_free(void* p);
+// Gives the device what the pool holds beyond kPoolKeeps, after freeing much.
+void dev_give_back(int device);
+qcp_status temp_alloc(size_t bytes, cudaStream_t s, void** out);
+void temp_free(void* p, cudaStream_t s);
 template <class T>
 cudaError_t dev_malloc(T** p, size_t bytes) {
   return dev_malloc_bytes(reinterpret_cast<void**>(p), bytes);
