@@ -936,6 +936,7 @@ qcp_status qcp_build_plan_run(qcp_build_plan* p, const float* objs, uint32_t obj
 qcp_status qcp_build_plan_free(qcp_build_plan* p) {
   clear_error();
   if (!p) return QCP_OK;
+  const OnDevice on(p->ix->device);
   cudaDeviceSynchronize();
   build_plan_destroy(p);
   return QCP_OK;
@@ -966,6 +967,7 @@ qcp_status qcp_index_build(const float* objs, uint64_t n, uint32_t dims, uint32_
 qcp_status qcp_index_free(qcp_index* index) {
   clear_error();
   if (!index) return QCP_OK;
+  const OnDevice on(index->device);
   cudaDeviceSynchronize();
   index_release(index);
   return QCP_OK;

@@ -49,7 +49,8 @@ qcp_status check_launch(const char* what);
 // and cudaFree per buffer were most of a one-shot build: 5 M 4-D rectangles
 // and 1,000 queries 8.0 -> 0.83 ms.  Allocations and frees are ordered on the
 // calling thread's AllocOn stream (the legacy stream outside any); whoever
-// frees has made sure that work on other streams is done with the buffer.
+// frees has made sure that work on other streams is done with the buffer.  A
+// buffer is freed on its own device, whichever is the current one.
 // The pool maps new memory more slowly than cudaMalloc (6 ms per GB), so
 // buffers of more than kPoolLargest bytes, and those of plans (AllocLasting),
 // which come and go rarely, of more than kPoolLargestLasting, are allocated
@@ -78,6 +79,26 @@ class AllocOn {
 
  private:
   cudaStream_t before_;
+};
+
+// The given device is the current one while this lives.
+class OnDevice {
+ public:
+  explicit OnDevice(int device) {
+    if (cudaGetDevice(&before_) != cudaSuccess) before_ = device;
+    switched_ = before_ != device;
+    if (switched_) cudaSetDevice(device);
+  }
+  ~OnDevice() {
+    if (switched_) cudaSetDevice(before_);
+  }
+  OnDevice(const OnDevice&) = delete;
+  OnDevice& operator=(const OnDevice&) = delete;
+  bool switched() const { return switched_; }
+
+ private:
+  int before_ = 0;
+  bool switched_ = false;
 };
 
 class AllocLasting {

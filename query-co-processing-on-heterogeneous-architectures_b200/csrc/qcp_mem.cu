@@ -134,11 +134,16 @@ void dev_free(void* p) {
     b = it->second;
     m.blocks.erase(it);
   }
+  // (the calling thread's stream is one of the current device's)
+  const OnDevice on(b.device);
   if (!b.pooled) {
     cudaFree(p);
     return;
   }
-  cudaFreeAsync(p, t_alloc_stream);
+  if (cudaFreeAsync(p, on.switched() ? nullptr : t_alloc_stream) != cudaSuccess) {
+    cudaGetLastError();
+    cudaFree(p);
+  }
   std::lock_guard<std::mutex> g(m.mu);
   m.pools[b.device].live -= b.bytes;
   follow(m.pools[b.device]);
@@ -150,8 +155,9 @@ void dev_give_back(int device) {
   std::lock_guard<std::mutex> g(m.mu);
   Pool& p = m.pools[device];
   if (!p.pool) return;
+  const OnDevice on(device);
   if (reserved(p) <= p.live + kPoolKeeps) return;
-  cudaStreamSynchronize(t_alloc_stream);
+  cudaStreamSynchronize(on.switched() ? nullptr : t_alloc_stream);
   cudaMemPoolTrimTo(p.pool, p.live + kPoolKeeps);
 }
 

@@ -243,6 +243,7 @@ extern "C" qcp_status qcp_plan_run(qcp_plan* p, const float* boxes, uint32_t q, 
 extern "C" qcp_status qcp_plan_free(qcp_plan* p) {
   qcp::clear_error();
   if (!p) return QCP_OK;
+  const qcp::OnDevice on(p->ix->device);
   cudaDeviceSynchronize();
   plan_destroy(p);
   return QCP_OK;

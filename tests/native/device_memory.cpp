@@ -191,6 +191,32 @@ static void lasting_and_small() {
   CHECK(g_taken[0] <= kRoom);
 }
 
+// A buffer is freed on its device, in an order of its device's, whichever is
+// current, and the current one stays so.
+static void other_device() {
+  g_device = 1;
+  void* pooled = get(10 * MB);
+  void* large = get(1 * GB);
+  g_device = 0;
+  {
+    const AllocOn on(reinterpret_cast<cudaStream_t>(0x1000));  // a stream of device 0
+    dev_free(pooled);
+    dev_free(large);
+    dev_free(get(10 * MB));
+  }
+  CHECK(g_device == 0);
+  CHECK(g_wrong_device == 0);
+  CHECK(g_blocks.empty());
+}
+
+// A refused stream-ordered free is not a leak.
+static void refused_free() {
+  void* p = get(10 * MB);
+  g_refuse_async_free = true;
+  dev_free(p);
+  CHECK(g_blocks.empty());
+}
+
 int main(int, char** argv) {
   const struct {
     const char* name;
@@ -198,7 +224,9 @@ int main(int, char** argv) {
   } all[] = {{"idle_after_frees", idle_after_frees},
              {"give_back", give_back},
              {"large_gets_the_rest", large_gets_the_rest},
-             {"lasting_and_small", lasting_and_small}};
+             {"lasting_and_small", lasting_and_small},
+             {"other_device", other_device},
+             {"refused_free", refused_free}};
   for (const auto& t : all)
     if (!strcmp(argv[1], t.name)) return t.run(), 0;
   return 2;

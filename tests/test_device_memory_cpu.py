@@ -24,7 +24,8 @@ def exe(tmp_path_factory):
     return out
 
 
-@pytest.mark.parametrize("what", ["idle_after_frees", "give_back", "large_gets_the_rest", "lasting_and_small"])
+@pytest.mark.parametrize("what", ["idle_after_frees", "give_back", "large_gets_the_rest", "lasting_and_small",
+                                  "other_device", "refused_free"])
 def test_rule(exe, what):
     r = subprocess.run([str(exe), what], capture_output=True, text=True, timeout=60)
     assert r.returncode == 0, r.stderr
