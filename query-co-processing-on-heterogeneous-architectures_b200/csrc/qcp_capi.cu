@@ -84,11 +84,14 @@ qcp_status DevPool::get(size_t bytes, void** out) {
   }
   const size_t sz = round_alloc(bytes);
   void* p = nullptr;
-  cudaError_t e = dev_malloc(&p, sz);
+  auto alloc = [&] { return shared ? dev_malloc_shared(&p, sz) : dev_malloc(&p, sz); };
+  cudaError_t e = alloc();
   if (e == cudaErrorMemoryAllocation) {
     cudaGetLastError();
-    trim();  // (dev_malloc then gives back what the pool got from it)
-    e = dev_malloc(&p, sz);
+    // (the allocation then gives back what is kept of it)
+    trim();
+    if (beside) beside->trim();
+    e = alloc();
   }
   if (e != cudaSuccess) return cuda_status(e, "cudaMalloc");
   // remember the real size through the free list protocol: callers hand the
@@ -235,11 +238,11 @@ qcp_status ws_reserve_queries(qcp_index* ix, Workspace* ws, uint32_t q) {
     ws->q_cap = n;
   }
   if (!ws->offsets || ws->offsets_cap < need) {
-    if (ws->offsets) ix->pool.put(0, ws->offsets);
+    if (ws->offsets) ix->results.put(0, ws->offsets);
     ws->offsets = nullptr;
     ws->offsets_cap = 0;
     void* p = nullptr;
-    QCP_TRY(ix->pool.get(sizeof(uint64_t) * need, &p));
+    QCP_TRY(ix->results.get(sizeof(uint64_t) * need, &p));
     ws->offsets = (uint64_t*)p;
     ws->offsets_cap = need;
   }
@@ -262,16 +265,16 @@ qcp_status ws_reserve_queries(qcp_index* ix, Workspace* ws, uint32_t q) {
 qcp_status ws_reserve_out(qcp_index* ix, Workspace* ws, size_t ids) {
   if (ws->out_ids && ws->out_cap >= ids) return QCP_OK;
   size_t n = ids + (ids >> 3) + 1024;
-  if (ws->out_ids) ix->pool.put(sizeof(int32_t) * ws->out_cap, ws->out_ids);
+  if (ws->out_ids) ix->results.put(sizeof(int32_t) * ws->out_cap, ws->out_ids);
   if (ws->tmp_ids) ix->pool.put(sizeof(int32_t) * ws->out_cap, ws->tmp_ids);
   ws->out_ids = ws->tmp_ids = nullptr;
   ws->out_cap = 0;
   void* a = nullptr;
   void* b = nullptr;
-  QCP_TRY(ix->pool.get(sizeof(int32_t) * n, &a));
+  QCP_TRY(ix->results.get(sizeof(int32_t) * n, &a));
   qcp_status st = ix->pool.get(sizeof(int32_t) * n, &b);
   if (st != QCP_OK) {
-    ix->pool.put(sizeof(int32_t) * n, a);
+    ix->results.put(sizeof(int32_t) * n, a);
     return st;
   }
   ws->out_ids = (int32_t*)a;
@@ -369,8 +372,8 @@ void ws_destroy(Workspace* ws, qcp_index* ix) {
   if (ws->side) cudaStreamDestroy(ws->side);
   for (cudaEvent_t e : ws->side_ev)
     if (e) cudaEventDestroy(e);
-  if (ws->offsets) ix->pool.put(0, ws->offsets);
-  if (ws->out_ids) ix->pool.put(0, ws->out_ids);
+  if (ws->offsets) ix->results.put(0, ws->offsets);
+  if (ws->out_ids) ix->results.put(0, ws->out_ids);
   if (ws->tmp_ids) ix->pool.put(0, ws->tmp_ids);
   dev_free(ws->jobs[0]);
   dev_free(ws->jobs[1]);
@@ -422,6 +425,7 @@ static void index_release(qcp_index* ix) {
   dev_free(ix->keys);
   for (int l = 0; l < kMaxLevels; ++l) dev_free(ix->mbr[l]);
   ix->pool.trim();
+  ix->results.trim();
   dev_give_back(ix->device);
   delete ix;
 }
@@ -859,7 +863,7 @@ qcp_status qcp_build_plan_create(uint64_t n, uint32_t dims, uint32_t is_rect, co
   qcp_status st = index_alloc(ix);
   cudaStream_t cap = nullptr;
   if (st == QCP_OK) {
-    if (dev_malloc(&p->d_in, sizeof(float) * p->ncoord * n) != cudaSuccess ||
+    if (dev_malloc_shared(reinterpret_cast<void**>(&p->d_in), sizeof(float) * p->ncoord * n) != cudaSuccess ||
         dev_malloc(&p->keys_tmp, sizeof(uint64_t) * n) != cudaSuccess ||
         dev_malloc(&p->vals, sizeof(uint32_t) * n) != cudaSuccess ||
         dev_malloc(&p->vals_tmp, sizeof(uint32_t) * n) != cudaSuccess ||
@@ -1089,8 +1093,8 @@ qcp_status qcp_result_release(qcp_result* r) {
   if (!r || !r->owner_) return QCP_OK;
   ResultArena* a = (ResultArena*)r->owner_;
   if (a->host) host_pool().put(a->host_bytes, a->host);
-  if (a->d_offsets && a->ix) a->ix->pool.put(0, a->d_offsets);
-  if (a->d_ids && a->ix) a->ix->pool.put(0, a->d_ids);
+  if (a->d_offsets && a->ix) a->ix->results.put(0, a->d_offsets);
+  if (a->d_ids && a->ix) a->ix->results.put(0, a->d_ids);
   if (a->d_tmp && a->ix) a->ix->pool.put(0, a->d_tmp);
   delete a;
   memset(r, 0, sizeof(*r));

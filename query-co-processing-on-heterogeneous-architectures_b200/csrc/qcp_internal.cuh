@@ -57,10 +57,19 @@ qcp_status check_launch(const char* what);
 // on their own: an index of 32 M 8-D rectangles takes 35 ms with cudaMalloc,
 // 110 from the pool.
 // ---------------------------------------------------------------------------
+//
+// What the caller sees -- results, a plan's outputs, a build plan's input -- is
+// cudaMalloc memory at any size: pool memory has no interprocess handle, and
+// enabling peer access does not map it.  Up to kSharedKeeps bytes of such
+// buffers are kept per device when they are freed (without it a one-shot build
+// and its queries take 1.0 ms, 0.75 with it), and given back when an allocation
+// finds no room.
 constexpr uint64_t kPoolKeeps = 2ull << 30;
+constexpr uint64_t kSharedKeeps = 256ull << 20;
 constexpr uint64_t kPoolLargest = 256ull << 20;
 constexpr uint64_t kPoolLargestLasting = 4ull << 20;
 cudaError_t dev_malloc_bytes(void** p, size_t bytes);
+cudaError_t dev_malloc_shared(void** p, size_t bytes);
 void dev_free(void* p);
 // Gives the device what the pool holds beyond kPoolKeeps, after freeing much.
 void dev_give_back(int device);
@@ -114,6 +123,9 @@ class AllocLasting {
 // so that repeated query batches do not call cudaMalloc each time.
 // ---------------------------------------------------------------------------
 struct DevPool {
+  explicit DevPool(bool shared_buffers = false) : shared(shared_buffers) {}
+  const bool shared;           // of dev_malloc_shared buffers
+  DevPool* beside = nullptr;   // trimmed too when an allocation finds no room
   std::mutex mu;
   std::vector<std::pair<size_t, void*>> free_list;  // (bytes, ptr) ready for reuse
   std::vector<std::pair<void*, size_t>> sizes;      // every live allocation's size
@@ -155,7 +167,7 @@ struct Workspace {
   void* zeroed = nullptr;        // ctr, qcount and qcursor in one block, cleared by one memset
   uint64_t* qcount = nullptr;    // per-query counts, q
   uint64_t* qcursor = nullptr;   // per-query write cursors, q
-  uint64_t* offsets = nullptr;   // q + 1, from the index's pool
+  uint64_t* offsets = nullptr;   // q + 1, from the index's results
   size_t offsets_cap = 0;
   size_t q_cap = 0;
   int32_t* out_ids = nullptr;    // unsorted then sorted ids
@@ -262,6 +274,7 @@ enum CtrSlot : uint32_t {
 }  // namespace qcp
 
 struct qcp_index {
+  qcp_index() { pool.beside = &results, results.beside = &pool; }
   int device = 0;
   uint64_t n = 0;
   uint32_t dims = 0, is_rect = 0, fanout = 128, levels = 0;
@@ -282,6 +295,7 @@ struct qcp_index {
   uint64_t device_bytes = 0;
 
   qcp::DevPool pool;
+  qcp::DevPool results{true};  // offsets and ids
   std::mutex ws_mu;
   std::vector<qcp::Workspace*> ws_free;
   std::vector<qcp::Workspace*> ws_all;

@@ -3,6 +3,7 @@
 // only.
 #include <mutex>
 #include <unordered_map>
+#include <vector>
 
 #include "qcp_internal.cuh"
 
@@ -20,15 +21,18 @@ struct Pool {
   uint64_t live = 0;       // bytes allocated from it and not freed
   uint64_t threshold = 0;  // its release threshold
 };
+enum Kind { kPooled, kDirect, kShared };
 struct Block {
   size_t bytes;
   int device;
-  bool pooled;
+  Kind kind;
 };
 struct Memory {
   std::mutex mu;
   Pool pools[kMaxDevices];
-  std::unordered_map<void*, Block> blocks;  // every live allocation
+  std::unordered_map<void*, Block> blocks;       // every live allocation
+  std::vector<std::pair<void*, Block>> idle;     // shared blocks that are kept, oldest first
+  uint64_t idle_bytes[kMaxDevices] = {};
 };
 Memory& memory() {
   static Memory* m = new Memory();  // lives until exit
@@ -73,16 +77,52 @@ uint64_t reserved(const Pool& p) {
   return bytes;
 }
 
-cudaError_t allocate(void** p, size_t bytes, bool pooled, cudaStream_t s) {
+// Takes the kept shared blocks of a device off the list, the oldest first,
+// until it keeps at most `keep` bytes (m.mu is held; the caller frees them).
+std::vector<void*> drop_idle(Memory& m, int device, uint64_t keep) {
+  std::vector<void*> out;
+  for (size_t i = 0; i < m.idle.size() && m.idle_bytes[device] > keep;) {
+    if (m.idle[i].second.device != device) {
+      ++i;
+      continue;
+    }
+    out.push_back(m.idle[i].first);
+    m.idle_bytes[device] -= m.idle[i].second.bytes;
+    m.idle.erase(m.idle.begin() + i);
+  }
+  return out;
+}
+
+// A kept shared block of the device for `bytes`, the smallest of at most twice
+// as many.
+bool take_idle(Memory& m, int device, size_t bytes, void** p) {
+  std::lock_guard<std::mutex> g(m.mu);
+  size_t best = m.idle.size();
+  for (size_t i = 0; i < m.idle.size(); ++i) {
+    const Block& b = m.idle[i].second;
+    if (b.device == device && b.bytes >= bytes && b.bytes <= 2 * bytes + (1u << 20) &&
+        (best == m.idle.size() || b.bytes < m.idle[best].second.bytes))
+      best = i;
+  }
+  if (best == m.idle.size()) return false;
+  *p = m.idle[best].first;
+  m.blocks[*p] = m.idle[best].second;
+  m.idle_bytes[device] -= m.idle[best].second.bytes;
+  m.idle.erase(m.idle.begin() + best);
+  return true;
+}
+
+cudaError_t allocate(void** p, size_t bytes, Kind kind, cudaStream_t s) {
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
   if (!bytes) bytes = 1;
   Memory& m = memory();
-  if (!pooled) {
+  if (kind != kPooled) {
+    if (kind == kShared && take_idle(m, dev, bytes, p)) return cudaSuccess;
     if ((e = cudaMalloc(p, bytes)) != cudaSuccess) return e;
     std::lock_guard<std::mutex> g(m.mu);
-    m.blocks[*p] = Block{bytes, dev, false};
+    m.blocks[*p] = Block{bytes, dev, kind};
     return cudaSuccess;
   }
   Pool* pool = nullptr;
@@ -92,7 +132,7 @@ cudaError_t allocate(void** p, size_t bytes, bool pooled, cudaStream_t s) {
   }
   if ((e = cudaMallocFromPoolAsync(p, bytes, pool->pool, s)) != cudaSuccess) return e;
   std::lock_guard<std::mutex> g(m.mu);
-  m.blocks[*p] = Block{bytes, dev, true};
+  m.blocks[*p] = Block{bytes, dev, kPooled};
   pool->live += bytes;
   follow(*pool);
   // If the pool holds more than the threshold although something had to be
@@ -102,26 +142,33 @@ cudaError_t allocate(void** p, size_t bytes, bool pooled, cudaStream_t s) {
   return cudaSuccess;
 }
 
-// As allocate; once more, without what the pool keeps, where there is no room.
-cudaError_t allocate_or_trim(void** p, size_t bytes, bool pooled, cudaStream_t s) {
-  cudaError_t e = allocate(p, bytes, pooled, s);
+// As allocate; once more, without what is kept, where there is no room.
+cudaError_t allocate_or_trim(void** p, size_t bytes, Kind kind, cudaStream_t s) {
+  cudaError_t e = allocate(p, bytes, kind, s);
   if (e != cudaErrorMemoryAllocation) return e;
   cudaGetLastError();
   cudaStreamSynchronize(s);  // what was freed on it is free then
   int dev = 0;
   Memory& m = memory();
   if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < kMaxDevices) {
-    std::lock_guard<std::mutex> g(m.mu);
-    if (m.pools[dev].pool) cudaMemPoolTrimTo(m.pools[dev].pool, 0);
+    std::vector<void*> old;
+    {
+      std::lock_guard<std::mutex> g(m.mu);
+      if (m.pools[dev].pool) cudaMemPoolTrimTo(m.pools[dev].pool, 0);
+      old = drop_idle(m, dev, 0);
+    }
+    for (void* q : old) cudaFree(q);
   }
-  return allocate(p, bytes, pooled, s);
+  return allocate(p, bytes, kind, s);
 }
 
 }  // namespace
 
 cudaError_t dev_malloc_bytes(void** p, size_t bytes) {
-  return allocate_or_trim(p, bytes, bytes <= (t_lasting ? kPoolLargestLasting : kPoolLargest), t_alloc_stream);
+  const bool pooled = bytes <= (t_lasting ? kPoolLargestLasting : kPoolLargest);
+  return allocate_or_trim(p, bytes, pooled ? kPooled : kDirect, t_alloc_stream);
 }
+cudaError_t dev_malloc_shared(void** p, size_t bytes) { return allocate_or_trim(p, bytes, kShared, t_alloc_stream); }
 
 void dev_free(void* p) {
   if (!p) return;
@@ -136,7 +183,18 @@ void dev_free(void* p) {
   }
   // (the calling thread's stream is one of the current device's)
   const OnDevice on(b.device);
-  if (!b.pooled) {
+  if (b.kind == kShared && b.bytes <= kSharedKeeps) {
+    std::vector<void*> old;
+    {
+      std::lock_guard<std::mutex> g(m.mu);
+      old = drop_idle(m, b.device, kSharedKeeps - b.bytes);
+      m.idle.emplace_back(p, b);
+      m.idle_bytes[b.device] += b.bytes;
+    }
+    for (void* q : old) cudaFree(q);
+    return;
+  }
+  if (b.kind != kPooled) {
     cudaFree(p);
     return;
   }
@@ -171,7 +229,7 @@ AllocLasting::~AllocLasting() { t_lasting = false; }
 // reached the free, so calls that run concurrently on different streams never
 // share one.
 qcp_status temp_alloc(size_t bytes, cudaStream_t s, void** out) {
-  QCP_CUDA(allocate_or_trim(out, bytes, true, s));
+  QCP_CUDA(allocate_or_trim(out, bytes, kPooled, s));
   return QCP_OK;
 }
 

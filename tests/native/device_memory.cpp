@@ -217,6 +217,40 @@ static void refused_free() {
   CHECK(g_blocks.empty());
 }
 
+// Buffers that callers see come from cudaMalloc, are kept up to a bound when
+// they are freed, and serve the next such buffer of their device.
+static void shared_buffers() {
+  auto share = [](size_t bytes) {
+    void* p = nullptr;
+    CHECK(dev_malloc_shared(&p, bytes) == cudaSuccess);
+    CHECK(!g_blocks[p].pool);
+    return p;
+  };
+  void* a = share(10 * MB);
+  dev_free(a);
+  CHECK(share(9 * MB) == a);
+  CHECK(share(9 * MB) != a);  // (in use)
+  dev_free(a);
+  CHECK(share(1 * MB) != a);  // not for much less
+  g_device = 1;
+  CHECK(share(9 * MB) != a);  // nor on another device
+  g_device = 0;
+  std::vector<void*> v;
+  for (int i = 0; i < 60; ++i) v.push_back(share(10 * MB));
+  for (void* p : v) dev_free(p);
+  dev_free(share(1 * GB));
+  CHECK(g_taken[0] <= kSharedKeeps + 10 * MB);
+  // no room: what is kept goes first
+  dev_free(share(kRoom - 15 * MB));
+  CHECK(g_taken[0] <= 10 * MB);
+  v.assign(1, share(200 * MB));
+  dev_free(v[0]);
+  {
+    AllocLasting lasting;
+    get(kRoom - 15 * MB);
+  }
+}
+
 int main(int, char** argv) {
   const struct {
     const char* name;
@@ -226,7 +260,8 @@ int main(int, char** argv) {
              {"large_gets_the_rest", large_gets_the_rest},
              {"lasting_and_small", lasting_and_small},
              {"other_device", other_device},
-             {"refused_free", refused_free}};
+             {"refused_free", refused_free},
+             {"shared_buffers", shared_buffers}};
   for (const auto& t : all)
     if (!strcmp(argv[1], t.name)) return t.run(), 0;
   return 2;

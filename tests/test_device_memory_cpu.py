@@ -25,7 +25,7 @@ def exe(tmp_path_factory):
 
 
 @pytest.mark.parametrize("what", ["idle_after_frees", "give_back", "large_gets_the_rest", "lasting_and_small",
-                                  "other_device", "refused_free"])
+                                  "other_device", "refused_free", "shared_buffers"])
 def test_rule(exe, what):
     r = subprocess.run([str(exe), what], capture_output=True, text=True, timeout=60)
     assert r.returncode == 0, r.stderr
