@@ -741,7 +741,7 @@ __global__ void __launch_bounds__(1024) k_scan_one(const T* __restrict__ in, T* 
 
 // objs -> sorted SoA arrays and the leaves' MBRs; flags non-finite coordinates
 // in *bad (bit 1).  The permutation of a sort that timed out holds anything,
-// so positions are bounded.  A block packs blockDim.x / fanout whole leaves at a time, one
+// so positions are bounded.  *inverted: see qcp_index.  A block packs blockDim.x / fanout whole leaves at a time, one
 // object per thread, so a leaf's MBR comes from registers: every warp reduces
 // its 32 objects (as order-preserving integers), the leaf's warps meet in
 // shared memory.  Bound by the gather of whole rows in key order; the separate
@@ -775,7 +775,7 @@ template <int D, bool RECT, int V>
 __global__ void __launch_bounds__(256) k_pack(const float* __restrict__ objs, const uint32_t* __restrict__ perm,
                                               uint64_t n, uint64_t npad, uint32_t fanout, uint64_t nleaves,
                                               uint64_t pad0, float* __restrict__ coords, int32_t* __restrict__ ids,
-                                              float* __restrict__ mbr, uint32_t* bad) {
+                                              float* __restrict__ mbr, uint32_t* bad, uint32_t* inverted) {
   constexpr int NC = RECT ? 2 * D : D;
   __shared__ uint32_t wlo[8][D], whi[8][D];
   const uint32_t tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
@@ -794,6 +794,12 @@ __global__ void __launch_bounds__(256) k_pack(const float* __restrict__ objs, co
 #pragma unroll
         for (int c = 0; c < NC; ++c) finite &= isfinite(x[c]);
         if (!finite) atomicOr(bad, 1u);
+        if constexpr (RECT) {
+          bool inv = false;
+#pragma unroll
+          for (int d = 0; d < D; ++d) inv |= x[d] > x[D + d];
+          if (inv) *inverted = 1;
+        }
         ids[i] = (int32_t)id;
 #pragma unroll
         for (int d = 0; d < D; ++d) {
@@ -829,6 +835,15 @@ __global__ void __launch_bounds__(256) k_pack(const float* __restrict__ objs, co
       mbr[(uint64_t)c * pad0 + j] = m;
     }
     __syncthreads();
+  }
+}
+
+__global__ void k_find_inverted(const float* __restrict__ coords, uint64_t n, uint64_t npad, uint32_t dims,
+                                uint32_t* inverted) {
+  for (uint32_t d = 0; d < dims; ++d) {
+    const float *lo = coords + d * npad, *hi = coords + (dims + d) * npad;
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
+      if (lo[i] > hi[i]) *inverted = 1;
   }
 }
 
@@ -1073,15 +1088,27 @@ static void launch_pack(qcp_index* ix, const float* objs, const uint32_t* perm, 
   const bool wide = reinterpret_cast<uintptr_t>(objs) % (sizeof(float) * V) == 0;
   auto* kern = wide ? k_pack<D, RECT, V> : k_pack<D, RECT, 1>;
   kern<<<grid, per * F, 0, s>>>(objs, perm, ix->n, ix->npad, F, ix->level_nodes[0], ix->level_pad[0], ix->coords,
-                                ix->ids, ix->mbr[0], d_bad);
+                                ix->ids, ix->mbr[0], d_bad, ix->inverted);
 }
 
 qcp_status build_pack(qcp_index* ix, const float* objs, const uint32_t* perm, cudaStream_t s,
                       uint32_t* d_bad) {
+  if (ix->is_rect) QCP_CUDA(cudaMemsetAsync(ix->inverted, 0, sizeof(uint32_t), s));
   QCP_DISPATCH_D(ix->dims, if (ix->is_rect) launch_pack<DD, true>(ix, objs, perm, s, d_bad);
                  else launch_pack<DD, false>(ix, objs, perm, s, d_bad));
   note_launch();
   return check_launch("k_pack");
+}
+
+qcp_status find_inverted(qcp_index* ix, cudaStream_t s) {
+  if (!ix->is_rect) return QCP_OK;
+  QCP_CUDA(cudaMemsetAsync(ix->inverted, 0, sizeof(uint32_t), s));
+  k_find_inverted<<<grid_for(ix->n, 256, num_sms() * 8), 256, 0, s>>>(ix->coords, ix->n, ix->npad, ix->dims,
+                                                                      ix->inverted);
+  note_launch();
+  QCP_TRY(check_launch("k_find_inverted"));
+  QCP_CUDA(cudaStreamSynchronize(s));
+  return QCP_OK;
 }
 
 qcp_status build_levels(qcp_index* ix, cudaStream_t s) {

@@ -423,6 +423,7 @@ static void index_release(qcp_index* ix) {
   dev_free(ix->coords);
   dev_free(ix->ids);
   dev_free(ix->keys);
+  dev_free(ix->inverted);
   for (int l = 0; l < kMaxLevels; ++l) dev_free(ix->mbr[l]);
   ix->pool.trim();
   ix->results.trim();
@@ -451,6 +452,7 @@ static qcp_status index_alloc(qcp_index* ix) {
   QCP_CUDA(dev_malloc(&ix->coords, sizeof(float) * ix->ncoord * ix->npad));
   QCP_CUDA(dev_malloc(&ix->ids, sizeof(int32_t) * ix->npad));
   QCP_CUDA(dev_malloc(&ix->keys, sizeof(uint64_t) * ix->n));
+  if (ix->is_rect) QCP_CUDA(dev_malloc(&ix->inverted, sizeof(uint32_t)));
   ix->device_bytes += sizeof(float) * ix->ncoord * ix->npad + sizeof(int32_t) * ix->npad;
   for (uint32_t l = 0; l < L; ++l) {
     QCP_CUDA(dev_malloc(&ix->mbr[l], sizeof(float) * 2 * ix->dims * ix->level_pad[l]));
@@ -1218,6 +1220,7 @@ qcp_status qcp_index_load(const char* path, void* stream, qcp_index** out) {
   load(ix->coords, sizeof(float) * ix->ncoord * ix->npad);
   for (uint32_t l = 0; l < ix->levels && ok; ++l) load(ix->mbr[l], sizeof(float) * 2 * ix->dims * ix->level_pad[l]);
   fclose(f);
+  if (ok && (st = find_inverted(ix, nullptr)) != QCP_OK) ok = false;
   if (!ok) {
     if (st == QCP_OK) {
       set_error(std::string("failed reading ") + path);

@@ -61,8 +61,8 @@ qcp_status check_launch(const char* what);
 // What the caller sees -- results, a plan's outputs, a build plan's input -- is
 // cudaMalloc memory at any size: pool memory has no interprocess handle, and
 // enabling peer access does not map it.  Up to kSharedKeeps bytes of such
-// buffers are kept per device when they are freed (without it a one-shot build
-// and its queries take 1.0 ms, 0.75 with it), and given back when an allocation
+// buffers are kept per device when they are freed (without it building 5 M
+// rectangles and asking 1,000 boxes takes 1.6 ms, 0.77 with it), and given back when an allocation
 // finds no room.
 constexpr uint64_t kPoolKeeps = 2ull << 30;
 constexpr uint64_t kSharedKeeps = 256ull << 20;
@@ -292,6 +292,10 @@ struct qcp_index {
   std::mutex host_mbr_mu;
   std::vector<float> host_mbr[qcp::kMaxLevels];
   bool host_mbr_ready = false;
+  // rectangles only: nonzero where one has lo > hi in some dimension.  Such an
+  // object can miss a box that covers its leaf's MBR, so no leaf of the index is
+  // then counted whole.
+  uint32_t* inverted = nullptr;
   uint64_t device_bytes = 0;
 
   qcp::DevPool pool;
@@ -314,7 +318,7 @@ __host__ __device__ __forceinline__ bool overlaps1(float qlo, float qhi, float l
 }
 // Entry [lo, hi] lies inside the query box in one dimension.  Only used to
 // skip the per-entry test of leaves whose MBR is covered by the query: every
-// finite entry inside such an MBR passes overlaps1.
+// finite entry with lo <= hi inside such an MBR passes overlaps1.
 __host__ __device__ __forceinline__ bool inside1(float qlo, float qhi, float lo, float hi) {
   return qlo <= lo && hi <= qhi;
 }
@@ -507,6 +511,8 @@ uint32_t kmeans_rank_bits(uint32_t K);
 qcp_status build_pack(qcp_index* ix, const float* objs, const uint32_t* perm, cudaStream_t s,
                       uint32_t* d_bad);
 qcp_status build_levels(qcp_index* ix, cudaStream_t s);
+// *ix->inverted of packed coordinates that were read from a file.
+qcp_status find_inverted(qcp_index* ix, cudaStream_t s);
 
 // Query
 qcp_status run_batched(qcp_index* ix, Workspace* ws, uint32_t q, bool counts_only, bool sort,

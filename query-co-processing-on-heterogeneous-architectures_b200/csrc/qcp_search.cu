@@ -341,6 +341,7 @@ __global__ void __launch_bounds__(kJoinThreads, (RECT ? 2 * D : D) > 8 ? 4 : ((R
 #pragma unroll
             for (int d = 0; d < D; ++d) in &= inside1(-b.v[2 * d], b.v[2 * d + 1], lo[d], hi[d]);
             mcov = __ballot_sync(0xffffffffu, in);
+            if (RECT && mcov && __ldg(t.inverted)) mcov = 0;
             if (mcov) {
               h = __popc(mcov) * F;
               // the tree's last leaf may hold fewer than F objects
@@ -533,7 +534,9 @@ __global__ void __launch_bounds__(256, (RECT ? 2 * D : D) > 8 ? 2 : (RECT ? 2 * 
         in &= inside1(-b[2 * d], b[2 * d + 1], mlo[d], mhi[d]);
       }
       if (kMbrAhead && g + 1 < gb) load_mbrs(g + 1);
-      const uint32_t mov = __ballot_sync(0xffffffffu, ov), mcov = __ballot_sync(0xffffffffu, ov && in);
+      const uint32_t mov = __ballot_sync(0xffffffffu, ov);
+      uint32_t mcov = __ballot_sync(0xffffffffu, ov && in);
+      if (RECT && mcov && __ldg(t.inverted)) mcov = 0;
       const uint32_t part = mov & ~mcov;
       // room for the hit bits; the objects' reads do not wait for it
       uint32_t off = kNoMask;

@@ -9,6 +9,7 @@ namespace qcp {
 struct TreeView {
   const float* coords;
   const int32_t* ids;
+  const uint32_t* inverted;  // qcp_index::inverted
   uint64_t n, npad;
   uint32_t fanout, levels;
   const float* mbr[kMaxLevels];
@@ -20,6 +21,7 @@ inline TreeView view_of(const qcp_index* ix) {
   TreeView v;
   v.coords = ix->coords;
   v.ids = ix->ids;
+  v.inverted = ix->inverted;
   v.n = ix->n;
   v.npad = ix->npad;
   v.fanout = ix->fanout;
