@@ -1260,6 +1260,7 @@ qcp_status run_plain(qcp_index* ix, Workspace* ws, uint32_t q, bool counts_only,
   if (grid > (uint32_t)num_sms() * 64) grid = (uint32_t)num_sms() * 64;
   mark(ws, kEvStart, s);
   QCP_CUDA(ws_zero(ws, 0, s));
+  if (ws->timing) QCP_CUDA(cudaMemsetAsync(ws->d_stats, 0, sizeof(unsigned long long) * kStatCount, s));
   mark(ws, kEvExpand, s);
   QCP_DISPATCH_D(D, launch_mprs<DD, kCount>(rect, grid, s, t, ws->qboxes, q, ws->qcount,
                                             nullptr, nullptr));
