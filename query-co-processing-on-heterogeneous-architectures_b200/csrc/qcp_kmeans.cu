@@ -34,6 +34,7 @@
 #include <vector>
 
 #include "qcp_internal.cuh"
+#include "qcp_kmeans.cuh"
 #include "qcp_tree.cuh"
 
 namespace qcp {
@@ -214,16 +215,7 @@ __global__ void __launch_bounds__(kAssignThreads) k_assign(const float* __restri
     int32_t arg = 0;
     if (grp[j] >= 0) {
       const uint32_t ka = (uint32_t)grp[j] * kCentreGroup, kb = min(ka + kCentreGroup, K);
-      arg = -1;
-      for (uint32_t k = ka; k < kb && arg < 0; ++k) {
-        float dist = 0.f;
-#pragma unroll
-        for (int d = 0; d < D; ++d) {
-          const float t = __fsub_rn(x[d], __ldg(centres + (uint64_t)d * K + k));
-          dist = __fadd_rn(dist, __fmul_rn(t, t));
-        }
-        if (dist == best[j]) arg = (int32_t)k;
-      }
+      arg = (int32_t)first_at_distance<D>(x, centres, K, ka, kb, best[j]);
     }
     const int32_t old = member[i];
     if (old == arg) continue;
