@@ -562,7 +562,8 @@ qcp_status classify_slices(qcp_index* ix, Workspace* ws, uint32_t q, bool sort, 
 qcp_status segmented_sort(qcp_index* ix, Workspace* ws, cudaStream_t s);
 
 qcp_status run_batched_counts_into(qcp_index* ix, const float* boxes, uint32_t q, uint64_t* counts,
-                                   uint2* items0, uint2* items1, size_t item_cap, uint32_t* ctr, cudaStream_t s);
+                                   uint2* items0, uint2* items1, size_t item_cap, uint32_t* ctr, uint32_t* hist,
+                                   size_t max_nodes, void* scan, size_t scan_bytes, cudaStream_t s);
 qcp_status exclusive_scan_counts(const uint64_t* counts, uint64_t* offsets, uint32_t q,
                                  DevPool& pool, cudaStream_t s, void* scratch = nullptr,
                                  size_t scratch_bytes = 0);

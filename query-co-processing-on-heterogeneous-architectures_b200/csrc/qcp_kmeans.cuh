@@ -16,7 +16,9 @@ __host__ __device__ __forceinline__ uint32_t first_at_distance(const float (&x)[
                                                                uint32_t ka, uint32_t kb, float best) {
   for (uint32_t k = ka; k < kb; ++k) {
     float dist = 0.f;
+#ifdef __CUDA_ARCH__
 #pragma unroll
+#endif
     for (int d = 0; d < D; ++d) {
 #ifdef __CUDA_ARCH__
       const float t = __fsub_rn(x[d], __ldg(centres + (uint64_t)d * K + k));

@@ -6,7 +6,7 @@
 // device-wide synchronisation cudaMalloc/cudaFree imply, or code that has
 // finished all allocation at start-up by policy.  For them this entry point
 // runs the batched traversal's counting pass with its scratch (the query
-// frontier, per-item counts and counters) in one fixed array of device
+// frontier, counts per node and counters) in one fixed array of device
 // memory that is part of this library's image, so a call allocates nothing;
 // the caller passes the query boxes and receives the counts in its own
 // device buffers.
@@ -27,8 +27,14 @@ namespace {
 constexpr size_t kNoAllocMaxItems = size_t(1) << 20;     // (query, node) items per frontier level
 constexpr uint32_t kNoAllocMaxQueries = 1u << 18;         // queries per call
 
+// level-1 nodes of an index whose large batches are put in node order (at
+// fan-out 128, 4,295 M objects; at 32, 268 M)
+constexpr size_t kNoAllocMaxNodes = size_t(1) << 18;
+
 struct NoAllocScratch {
   uint2 items[2][kNoAllocMaxItems];
+  uint32_t hist[2 * kNoAllocMaxNodes];
+  uint64_t scan[kNoAllocMaxNodes / 4096 + 2];
   uint32_t ctr[kCtrCount];
 };
 
@@ -107,5 +113,6 @@ extern "C" qcp_status qcp_query_counts_noalloc(qcp_index* index, const float* d_
   NoAllocScratch* sc = nullptr;
   QCP_TRY(scratch_on_current_device(&sc));
   return run_batched_counts_into(index, d_boxes, q, d_counts, sc->items[0], sc->items[1],
-                                 kNoAllocMaxItems, sc->ctr, (cudaStream_t)stream);
+                                 kNoAllocMaxItems, sc->ctr, sc->hist, kNoAllocMaxNodes, sc->scan, sizeof(sc->scan),
+                                 (cudaStream_t)stream);
 }

@@ -1075,23 +1075,26 @@ static uint64_t order_nodes(const qcp_index* ix, uint32_t q) {
   return may ? ix->level_nodes[1] : 0;
 }
 
-// The level-1 items in items[*cur] in node order, into the other buffer.
-static qcp_status order_items(qcp_index* ix, Workspace* ws, int* cur, cudaStream_t s) {
+// The level-1 items in items[*cur] in node order, into the other buffer.  hist:
+// twice as many words as there are level-1 nodes; scan: scan_scratch_bytes of
+// their number.
+static qcp_status order_items(qcp_index* ix, uint2* const* items, size_t item_cap, uint32_t* ctr, uint32_t* hist,
+                              void* scan, size_t scan_bytes, int* cur, cudaStream_t s) {
   const uint32_t grid = (uint32_t)num_sms() * 8;
   const int nxt = *cur ^ 1;
   const uint64_t nodes = ix->level_nodes[1];
-  uint32_t* ctr = ws->ctr;
-  QCP_CUDA(cudaMemsetAsync(ws->node_hist, 0, sizeof(uint32_t) * nodes, s));
-  k_node_hist<<<grid, 256, 0, s>>>(ws->items[*cur], ctr + kCtrFrontier0 + *cur, ws->items_cap, nodes,
-                                   ws->node_hist);
-  uint32_t* cursor = ws->node_hist + nodes;
-  QCP_TRY(exclusive_scan<uint32_t>(ws->node_hist, cursor, nodes, nullptr, ix->pool, s, ws->scan_tmp,
-                                   ws->scan_tmp_cap));
-  k_node_scatter<<<grid, 256, 0, s>>>(ws->items[*cur], ctr + kCtrFrontier0 + *cur, ws->items_cap, nodes, cursor,
-                                      ws->items[nxt], ctr + kCtrFrontier0 + nxt);
+  QCP_CUDA(cudaMemsetAsync(hist, 0, sizeof(uint32_t) * nodes, s));
+  k_node_hist<<<grid, 256, 0, s>>>(items[*cur], ctr + kCtrFrontier0 + *cur, item_cap, nodes, hist);
+  uint32_t* cursor = hist + nodes;
+  QCP_TRY(exclusive_scan<uint32_t>(hist, cursor, nodes, nullptr, ix->pool, s, scan, scan_bytes));
+  k_node_scatter<<<grid, 256, 0, s>>>(items[*cur], ctr + kCtrFrontier0 + *cur, item_cap, nodes, cursor, items[nxt],
+                                      ctr + kCtrFrontier0 + nxt);
   note_launch(2);
   *cur = nxt;
   return check_launch("order_items");
+}
+static qcp_status order_items(qcp_index* ix, Workspace* ws, int* cur, cudaStream_t s) {
+  return order_items(ix, ws->items, ws->items_cap, ws->ctr, ws->node_hist, ws->scan_tmp, ws->scan_tmp_cap, cur, s);
 }
 
 // What the count pass of this call records for its write pass.
@@ -1293,10 +1296,12 @@ qcp_status run_plain(qcp_index* ix, Workspace* ws, uint32_t q, bool counts_only,
 
 // Batched per-query hit counts into caller-provided device buffers (boxes,
 // counts) with scratch supplied by the caller as well: two frontier buffers
-// of item_cap items and kCtrCount counters.  Nothing is allocated.  Returns
+// of item_cap items, kCtrCount counters, and for up to max_nodes level-1 nodes
+// what order_items needs (more are counted as they come).  Nothing is allocated.  Returns
 // QCP_ERR_OUTPUT_OVERFLOW when the batch's frontier exceeds item_cap.
 qcp_status run_batched_counts_into(qcp_index* ix, const float* boxes, uint32_t q, uint64_t* counts,
-                                   uint2* items0, uint2* items1, size_t item_cap, uint32_t* ctr, cudaStream_t s) {
+                                   uint2* items0, uint2* items1, size_t item_cap, uint32_t* ctr, uint32_t* hist,
+                                   size_t max_nodes, void* scan, size_t scan_bytes, cudaStream_t s) {
   const TreeView t = view_of(ix);
   const uint32_t D = ix->dims;
   const bool rect = ix->is_rect != 0;
@@ -1320,8 +1325,11 @@ qcp_status run_batched_counts_into(qcp_index* ix, const float* boxes, uint32_t q
     note_launch();
     cur = nxt;
   }
+  uint64_t nodes = order_nodes(ix, q);
+  if (nodes > max_nodes) nodes = 0;
+  if (nodes) QCP_TRY(order_items(ix, items, item_cap, ctr, hist, scan, scan_bytes, &cur, s));
   qcp_status st = QCP_OK;
-  QCP_DISPATCH_D(D, st = launch_count<DD>(rect, 0, 8, s, t, boxes, items[cur], ctr + kCtrFrontier0 + cur,
+  QCP_DISPATCH_D(D, st = launch_count<DD>(rect, nodes, 8, s, t, boxes, items[cur], ctr + kCtrFrontier0 + cur,
                                          ctr + kCtrWork, counts, item_cap, nullptr, HitCache{}));
   QCP_TRY(st);
   uint32_t overflow = 0;  // pageable host word: no pinned buffer is allocated
