@@ -116,9 +116,14 @@ def dist_setup(n_gpus):
 
 
 def algorithmic_bytes(st: dict, dims: int, fanout: int, is_rect: bool = False, hit_cache: bool = True) -> dict:
-    """Bytes each kernel must move at minimum for the work it did, per launch
-    (one launch of each per step; k_leafscan<count> and <write> name the count
-    and the write pass, whose kernels are k_join or k_count, and k_leafwrite):
+    """Bytes charged to each kernel for the work it did, per launch (one launch
+    of each per step).  For the sorts these are what the kernel must move.
+    k_leafscan<count> and <write> name the count and the write pass and are
+    charged what a kernel moves that reads leaves once per (query, node) item
+    and keeps 12 B per group and 16 B per chunk.  Their kernels, k_join or
+    k_count and k_leafwrite, read a leaf once per run of boxes and keep 16 and
+    32 B, so the rates of these two are work per time in a unit of bytes, not
+    a share of the memory's, and may pass it:
     k_leafscan<count>  leaf-MBR reads of every (query, leaf-parent) item +
                        coordinates of partially covered leaves (+ with the hit
                        cache, its records written: 12 B per item and 32-leaf

@@ -190,7 +190,16 @@ typedef struct qcp_result {
 
 /* Build the index.  objs: n rows of dims floats (points, is_rect = 0) or of
  * 2*dims floats [lo0..lo(D-1), hi0..hi(D-1)] (rectangles, is_rect = 1).
- * Coordinates must be finite; 1 <= dims <= 8; 1 <= n < 2^31. */
+ * Coordinates must be finite; 1 <= dims <= 8; 1 <= n < 2^31.  A rectangle with
+ * lo > hi in some dimension is indexed and answered by the same predicate; an
+ * index that holds one tests every object of every leaf that a box overlaps.
+ *
+ * Builds and queries allocate device memory and wait for their stream, so they
+ * are refused (QCP_ERR_CUDA) on a stream that is being captured.  Results, a
+ * plan's outputs and a build plan's input are cudaMalloc memory; everything
+ * else comes from a stream-ordered pool of the library's own.  Of what is freed
+ * the library keeps at most 2 GiB per device in the pool and 256 MiB of buffers
+ * like the results', until an allocation of its own needs the room. */
 qcp_status qcp_index_build(const float* objs, uint64_t n, uint32_t dims, uint32_t is_rect,
                            const qcp_build_opts* opts, qcp_index** out);
 
@@ -307,8 +316,8 @@ qcp_status qcp_autotune(const float* objs, uint64_t n, uint32_t dims, uint32_t i
  * most max_queries boxes and max_hits ids per batch, captured once into a
  * CUDA graph and replayed per batch.  qcp_query_batch sizes its buffers and
  * launches from host readbacks between its phases; a plan fixes them at
- * creation (device memory for max_queries boxes, the frontier, max_hits ids
- * twice, the sort's tables) so every phase runs from device-resident counts,
+ * creation (device memory for max_queries boxes, the frontier and what is
+ * kept of it between the passes, max_hits ids twice, the sort's tables) so every phase runs from device-resident counts,
  * and one graph launch replaces its ~20 kernel launches and 3 host round
  * trips.  opts: blocks_per_sm, win_bits, leaf_prefetch, lanes_per_item and
  * unsorted are used (algo must be

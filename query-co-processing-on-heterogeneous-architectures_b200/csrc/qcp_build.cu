@@ -97,15 +97,15 @@ __global__ void __launch_bounds__(256) k_keys(const float* __restrict__ objs, ui
         key = (key << IB) | (e & ((1u << IB) - 1u));
         state = e >> IB;
       }
-      if constexpr (true) {  // bits % L levels
-        uint32_t rot = state / (D + 1), f = state % (D + 1);
-        uint64_t flip = f ? (1ull << (f - 1)) : 0ull;
-        for (--lvl; lvl >= 0; --lvl) {
-          uint32_t g = 0;
+      // bits % L levels
+      uint32_t rot = state / (D + 1);
+      const uint32_t f = state % (D + 1);
+      uint64_t flip = f ? (1ull << (f - 1)) : 0ull;
+      for (--lvl; lvl >= 0; --lvl) {
+        uint32_t g = 0;
 #pragma unroll
-          for (int d = 0; d < D; ++d) g |= ((c[d] >> lvl) & 1u) << d;
-          key = (key << D) | hilbert_step<D>(g, rot, flip);
-        }
+        for (int d = 0; d < D; ++d) g |= ((c[d] >> lvl) & 1u) << d;
+        key = (key << D) | hilbert_step<D>(g, rot, flip);
       }
       // hilbert_finish; shifts past the key's top bit change nothing
       key ^= low_bits;

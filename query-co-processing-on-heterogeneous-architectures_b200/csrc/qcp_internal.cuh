@@ -539,7 +539,6 @@ constexpr uint32_t kHistMaxG = 256;
 // Default log2 of the per-query sort's id windows (qcp_query_opts.win_bits).
 constexpr uint32_t kDefaultWinBits = 17;
 qcp_status ws_reserve_qwhist(Workspace* ws, size_t n);
-constexpr uint32_t kMaxGroups = 8;                    // 32-leaf groups per item (fan-out <= 256)
 constexpr uint32_t kNoMask = 0xffffffffu;            // group without cached hit masks
 constexpr size_t kMaxMaskWords = 0xc0000000u;        // hit-bit words (32-bit offsets)
 qcp_status ws_reserve_hitcache(Workspace* ws, size_t recs, size_t mask_words);

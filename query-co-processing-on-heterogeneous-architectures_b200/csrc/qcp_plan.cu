@@ -222,7 +222,7 @@ extern "C" qcp_status qcp_plan_run(qcp_plan* p, const float* boxes, uint32_t q, 
   QCP_CUDA(cudaMemcpyAsync(ws->h_total, ws->offsets + q, sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
   QCP_CUDA(cudaStreamSynchronize(s));
   if (ws->h_ctr[kCtrTimeout]) {
-    set_error("qcp_plan_run: a bounded wait for a leaf's bulk copy ran out");
+    set_error("qcp_plan_run: a bounded wait for a bulk copy ran out in the sort");
     return QCP_ERR_TIMEOUT;
   }
   const uint32_t flags = ws->h_ctr[kCtrOverflow];

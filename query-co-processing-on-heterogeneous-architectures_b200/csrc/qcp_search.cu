@@ -5,22 +5,25 @@
 //      (query, node) item of level l becomes the (query, child) items of the
 //      children whose MBR overlaps the query (warp per item, ballot
 //      compaction, one atomic per 32 items written).
-//   2. k_join: the (query, level-1 node) items, in large batches ordered by
-//      node (k_node_hist, a scan, k_node_scatter), are counted by one CTA per
-//      run of items: the node's leaf MBRs and the queries' boxes are staged in
-//      shared memory, leaves whose MBR lies inside a box are counted without
-//      touching their objects, and each other leaf that some box of the run
-//      overlaps is loaded once and tested against all of them.
+//   2. the (query, level-1 node) items are counted.  k_join, for large batches,
+//      which are ordered by node first (k_node_hist, a scan, k_node_scatter):
+//      one CTA per run of items, the queries' boxes in shared memory, the
+//      node's leaf MBRs in registers, and each partially covered leaf that some
+//      box of the run overlaps loaded once and tested against all of them.
+//      k_count, for the others: a warp per item or per 32-leaf group of one.
+//      Both count leaves whose MBR lies inside a box without touching their
+//      objects (unless the index holds a rectangle with lo > hi).
 //   3. exclusive scan of the per-query counts -> CSR offsets.
 //   4. k_leafwrite: a warp per item reserves its item's slice of the query's
 //      output with one atomic and writes ids (whole id runs for covered
 //      leaves, the hit bits k_join recorded, or a test of the leaf's objects).
 //   5. per-query sort of the ids (qcp_segsort.cu).
 //
-// Plain traversal (QCP_ALGO_PLAIN): k_mprs, one query per CUDA block,
-// restart scanning + parent check as the reference's
-// global_RestartScanning_and_ParentCheck (src/tree/mphr.cpp:303-438) does,
-// over the implicit node layout, run twice (count, then write).
+// Plain traversal (QCP_ALGO_PLAIN): k_mprs, one query per CUDA block as the
+// reference's global_RestartScanning_and_ParentCheck
+// (src/tree/mphr.cpp:303-438), but depth first over the implicit node layout
+// with the path's overlap masks in shared memory instead of a restart from the
+// root after every run of leaves; run twice (count, then write).
 //
 // The hit predicate everywhere is the reference's closed-interval test
 // (src/node/node_soa.cpp:94-113).
@@ -478,9 +481,12 @@ __device__ __forceinline__ bool whole_items(uint32_t nitems, uint32_t G, uint32_
 // no barriers.  Few items share a node, so nothing is staged: the box sits in
 // registers, a group's MBRs are tested one per lane, and the partially covered
 // leaves one after the other.  Bound by the latency of its dependent reads
-// (item, box and MBRs, objects); the CTAs per SM are what the registers of a
-// box, its MBRs and four objects allow without spills (61,000 8-D points, 7,768
-// boxes: 110 -> 45 us with three instead of four and no MBRs ahead).  1,000
+// (item, box and MBRs, objects); more CTAs per SM hide it until the registers
+// of a box, its MBRs and four objects spill too much (61,000 8-D points, 7,768
+// boxes: 110 -> 45 us with three instead of four and no MBRs ahead).  What is
+// left spills up to 88 bytes (3-D points, 64 registers) where a split without
+// was no faster: 20,000 boxes over 16 M points counted in this form 598 us,
+// with three CTAs 611, with one chunk ahead 600.  1,000
 // boxes over 1 M points: 18.9 (a warp per item) -> 12.4 us; 64 boxes over 16 M
 // points 36.7 -> 14.8 us.
 template <int D, bool RECT>
