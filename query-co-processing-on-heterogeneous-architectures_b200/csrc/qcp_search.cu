@@ -467,32 +467,60 @@ __global__ void __launch_bounds__(kJoinThreads, (RECT ? 2 * D : D) > 8 ? 4 : ((R
   }
 }
 
-// Whether a warp takes whole items: where their 32-leaf groups would be more
-// than eight rounds of the grid's warps.  15,000 items over 16 M points, six
-// rounds: the groups one by one 59 us to count and 59 to write, whole items 65
-// and 87; 10,000 items of tiny boxes at fan-out 256, nine rounds: 66 and 40,
-// whole items 44 and 23.
-__device__ __forceinline__ bool whole_items(uint32_t nitems, uint32_t G, uint32_t warps) {
-  return (uint64_t)nitems * G >= 8ull * warps;
+// Leaves that an item overlaps, about, from 32 items: the share of its node's
+// extent that the box covers and a leaf more, per dimension.
+template <int D>
+__device__ __forceinline__ float leaves_per_item(const TreeView& t, const float* boxes, const uint2* items,
+                                                 uint32_t nitems) {
+  if (t.levels < 2) return 1.f;
+  const uint2 it = items[(uint64_t)(threadIdx.x & 31) * nitems / 32];
+  const float leaf = exp2f(-log2f((float)t.fanout) / D);
+  float part = (float)t.fanout;
+#pragma unroll 1
+  for (int d = 0; d < D; ++d) {
+    const float lo = __ldg(t.mbr[1] + d * t.pad[1] + it.y), hi = __ldg(t.mbr[1] + (D + d) * t.pad[1] + it.y);
+    const float* q = boxes + (uint64_t)it.x * 2 * D + d;
+    const float common = fminf(__ldg(q + D), hi) - fmaxf(__ldg(q), lo);
+    part *= fminf(1.f, (hi > lo ? common / (hi - lo) : 1.f) + leaf);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
+  return part * (1.f / 32);
 }
 
-// Counts of batches that are not in node order: a warp per item, or per
-// 32-leaf group of one where there are too few items to keep the warps busy;
-// no barriers.  Few items share a node, so nothing is staged: the box sits in
-// registers, a group's MBRs are tested one per lane, and the partially covered
-// leaves one after the other.  Bound by the latency of its dependent reads
-// (item, box and MBRs, objects); more CTAs per SM hide it until the registers
-// of a box, its MBRs and four objects spill too much (61,000 8-D points, 7,768
-// boxes: 110 -> 45 us with three instead of four and no MBRs ahead).  What is
-// left spills up to 88 bytes (3-D points, 64 registers) where a split without
-// was no faster: 20,000 boxes over 16 M points counted in this form 598 us,
-// with three CTAs 611, with one chunk ahead 600.  1,000
-// boxes over 1 M points: 18.9 (a warp per item) -> 12.4 us; 64 boxes over 16 M
-// points 36.7 -> 14.8 us.
+// How the warps of k_count and k_leafwrite share the items: their 32-leaf groups
+// in turn where those are fewer than eight rounds of the grid's warps (15,000
+// items over 16 M points, six rounds: 59 us to count and 59 to write, whole items
+// 65 and 87); above that whole items where an item has few leaves (10,000 items
+// of tiny boxes at fan-out 256, nine rounds: the groups 66 and 40, whole items 44
+// and 23), and groups again, each to the next free warp, where it has many: whole
+// items then leave most warps waiting for the last ones.
+enum Share { kGroups, kItems, kGroupsByNeed };
+template <int D>
+__device__ __forceinline__ Share share_items(const TreeView& t, const float* boxes, const uint2* items,
+                                             uint32_t nitems, uint32_t G, uint32_t warps) {
+  const uint64_t groups = (uint64_t)nitems * G;
+  if (groups < 8ull * warps) return kGroups;
+  if (groups >= 1u << 31) return kItems;  // (units are counted in 32 bits)
+  return leaves_per_item<D>(t, boxes, items, nitems) < 2.f * G ? kItems : kGroupsByNeed;
+}
+
+// Counts of batches that are not in node order: a warp per item or per 32-leaf
+// group of one (share_items); no barriers.  Few items share a node, so nothing
+// is staged: the box sits in registers, a group's MBRs are tested one per lane,
+// and the partially covered leaves one after the other.  Bound by the latency
+// of its dependent reads (item, box and MBRs, objects); more CTAs per SM hide it
+// until the registers of a box, its MBRs and four objects spill too much
+// (61,000 8-D points, 7,768 boxes: 110 -> 45 us with three instead of four;
+// MBRs read one group ahead only up to two dimensions: 4 M 4-D rectangles 665 ->
+// 626 us; 3-D points still spill 72 bytes, three CTAs were slower).  1,000 boxes
+// over 1 M points: 18.9 (a warp per item) -> 12.4 us; 64 boxes over 16 M points
+// 36.7 -> 14.8 us; 3,000 boxes with 34 leaves per item over 4 M 4-D rectangles
+// at fan-out 256, by whole items in turn 900, by need 626.
 template <int D, bool RECT>
 __global__ void __launch_bounds__(256, (RECT ? 2 * D : D) > 8 ? 2 : (RECT ? 2 * D : D) > 3 ? 3 : 4)
     k_count(TreeView t, const float* __restrict__ boxes, const uint2* __restrict__ items,
-            const uint32_t* __restrict__ item_count, unsigned long long* qcount, uint64_t item_cap,
+            const uint32_t* __restrict__ item_count, uint32_t* work, unsigned long long* qcount, uint64_t item_cap,
             uint64_t nodes, unsigned long long* stats, HitCache hc) {
   const uint32_t lane = threadIdx.x & 31;
   const uint32_t F = t.fanout, G = F >> 5;
@@ -502,13 +530,29 @@ __global__ void __launch_bounds__(256, (RECT ? 2 * D : D) > 8 ? 2 : (RECT ? 2 * 
   const float* lmbr = t.mbr[0];
   const uint32_t chunks = (F + 127u) >> 7, wpl = chunks * kChunkWords;
   const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
-  const bool whole = whole_items(nitems, G, warps);
-  const uint64_t units = whole ? nitems : (uint64_t)nitems * G;
-  uint64_t u = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  uint2 next = u < units ? items[whole ? u : u / G] : make_uint2(0, 0);
-  for (; u < units; u += warps) {
-    const uint2 it = next;
-    if (u + warps < units) next = items[whole ? u + warps : (u + warps) / G];
+  const Share share = share_items<D>(t, boxes, items, nitems, G, warps);
+  const bool whole = share == kItems;
+  const uint32_t units = whole ? nitems : nitems * G;
+  // the next unit is known while this one is counted, so that its item is read
+  // ahead: by need it has been asked for a unit earlier
+  uint32_t asked = 0;  // lane 0's
+  auto ask = [&]() {
+    if (share == kGroupsByNeed && lane == 0) asked = atomicAdd(work, 1u);
+  };
+  auto after = [&](uint32_t u) {
+    if (share == kGroupsByNeed) return __shfl_sync(0xffffffffu, asked, 0);
+    return units - u > warps ? u + warps : units;
+  };
+  ask();
+  uint32_t u = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (share == kGroupsByNeed) u = after(u);
+  if (u >= units) return;
+  ask();
+  uint2 it = items[whole ? u : u / G];
+  for (uint32_t un = after(u);;) {
+    ask();
+    uint2 next = it;
+    if (un < units) next = items[whole ? un : un / G];
     float b[2 * D];  // -lo, hi per dimension, zeros as +0
     const float* q = boxes + (uint64_t)it.x * 2 * D;
 #pragma unroll
@@ -518,9 +562,9 @@ __global__ void __launch_bounds__(256, (RECT ? 2 * D : D) > 8 ? 2 : (RECT ? 2 * 
       b[2 * d + 1] = hi == 0.f ? 0.f : hi;
     }
     uint32_t total = 0;  // hits of the unit
-    const uint32_t ga = whole ? 0u : (uint32_t)(u % G), gb = whole ? G : ga + 1;
+    const uint32_t ga = whole ? 0u : u % G, gb = whole ? G : ga + 1;
     float mlo[D], mhi[D];  // a group's MBRs, with few dimensions loaded one group ahead
-    constexpr bool kMbrAhead = D <= 4;
+    constexpr bool kMbrAhead = D <= 2;
     auto load_mbrs = [&](uint32_t g) {
       const uint64_t at = (uint64_t)it.y * F + g * 32 + lane;
 #pragma unroll
@@ -596,7 +640,7 @@ __global__ void __launch_bounds__(256, (RECT ? 2 * D : D) > 8 ? 2 : (RECT ? 2 * 
       if (last < 32 && ((mcov >> last) & 1u)) chits -= (uint32_t)(nleaves * F - t.n);
       hits += chits;
       if (lane == 0) {
-        if (hc.rec) hc.rec[whole ? u * G + g : u] = make_uint4(mov, mcov, off, hits);
+        if (hc.rec) hc.rec[whole ? (size_t)u * G + g : u] = make_uint4(mov, mcov, off, hits);
         if (stats) {
           if (mcov) atomicAdd(stats + kStatCovered, (unsigned long long)__popc(mcov));
           if (part) atomicAdd(stats + kStatPartial, (unsigned long long)__popc(part));
@@ -606,6 +650,10 @@ __global__ void __launch_bounds__(256, (RECT ? 2 * D : D) > 8 ? 2 : (RECT ? 2 * 
       total += hits;
     }
     if (lane == 0 && total) atomicAdd(qcount + it.x, (unsigned long long)total);
+    if (un >= units) break;
+    u = un;
+    un = after(u);
+    it = next;
   }
 }
 
@@ -645,7 +693,9 @@ __global__ void __launch_bounds__(256) k_leafwrite(TreeView t, const float* __re
   // first one by its index, more as the warps get free (all in turn, without
   // the atomic: 59 -> 87 us on the 15,000 items, a heavy item's groups follow
   // one another; all by the atomic: 13 -> 18 us for 1,000 boxes over 1 M points)
-  const bool whole = whole_items(nitems, G, warps);
+  // (from eight items per warp on whole ones leave no warp waiting for long: 16 M
+  // points, 10,000 boxes of 10^9 ids 1.1 ms, by need 1.2)
+  const bool whole = nitems >= 8 * warps || share_items<D>(t, boxes, items, nitems, G, warps) == kItems;
   const uint32_t per = whole ? G : 1u;
   const uint32_t nfetch = whole ? nitems : nitems * G;
   for (uint32_t turn = 0;; ++turn) {
@@ -999,8 +1049,8 @@ qcp_status launch_count(bool rect, uint64_t nodes, uint32_t blocks_per_sm, cudaS
                         const float* boxes, const uint2* items, const uint32_t* item_count, uint32_t* work,
                         uint64_t* qcount, uint64_t item_cap, unsigned long long* stats, HitCache hc) {
   auto* count = rect ? k_count<D, true> : k_count<D, false>;
-  count<<<(uint32_t)num_sms() * blocks_per_sm, 256, 0, s>>>(t, boxes, items, item_count, (unsigned long long*)qcount,
-                                                            item_cap, nodes, stats, hc);
+  count<<<(uint32_t)num_sms() * blocks_per_sm, 256, 0, s>>>(t, boxes, items, item_count, work,
+                                                            (unsigned long long*)qcount, item_cap, nodes, stats, hc);
   note_launch();
   QCP_TRY(check_launch("k_count"));
   if (!nodes) return QCP_OK;
