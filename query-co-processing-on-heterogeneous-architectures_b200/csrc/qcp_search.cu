@@ -489,20 +489,24 @@ __device__ __forceinline__ float leaves_per_item(const TreeView& t, const float*
 }
 
 // How the warps of k_count and k_leafwrite share the items: their 32-leaf groups
-// in turn where those are fewer than eight rounds of the grid's warps (15,000
-// items over 16 M points, six rounds: 59 us to count and 59 to write, whole items
-// 65 and 87); above that whole items where an item has few leaves (10,000 items
-// of tiny boxes at fan-out 256, nine rounds: the groups 66 and 40, whole items 44
-// and 23), and groups again, each to the next free warp, where it has many: whole
-// items then leave most warps waiting for the last ones.
+// in turn where those are fewer than four rounds of the grid's warps; above that
+// whole items where an item has few leaves (10,000 items of tiny boxes at fan-out
+// 256, nine rounds: the groups 66 us to count and 40 to write, whole items 44 and
+// 23; a plan of 4,096 tiny boxes 201 -> 164 us with four rounds instead of
+// eight), and groups again, each to the next free warp, where it has kManyLeaves
+// or more: whole items then leave most warps waiting for the last ones.  (By need
+// an atomic on one address per group is paid, about 1 ns each: with 10 leaves per
+// item 9,000 boxes over 2 M points take 187 us by items, 212 by need, with 22
+// 6,000 over 1 M 233 and 217.)
+constexpr float kManyLeaves = 24.f;
 enum Share { kGroups, kItems, kGroupsByNeed };
 template <int D>
 __device__ __forceinline__ Share share_items(const TreeView& t, const float* boxes, const uint2* items,
                                              uint32_t nitems, uint32_t G, uint32_t warps) {
   const uint64_t groups = (uint64_t)nitems * G;
-  if (groups < 8ull * warps) return kGroups;
+  if (groups < 4ull * warps) return kGroups;
   if (groups >= 1u << 31) return kItems;  // (units are counted in 32 bits)
-  return leaves_per_item<D>(t, boxes, items, nitems) < 2.f * G ? kItems : kGroupsByNeed;
+  return leaves_per_item<D>(t, boxes, items, nitems) < kManyLeaves ? kItems : kGroupsByNeed;
 }
 
 // Counts of batches that are not in node order: a warp per item or per 32-leaf

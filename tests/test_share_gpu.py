@@ -1,5 +1,5 @@
 """Batches that are not in node order and have more 32-leaf groups than the
-grid's warps take in eight rounds: items of few leaves, of many, and around the
+grid's warps take in four rounds: items of few leaves, of many, and around the
 line between them, trees of one level up, ragged last leaves, inverted and
 infinite boxes -- ids and counts equal the oracle's, with and without recorded
 hit bits and in a captured plan."""
@@ -13,7 +13,7 @@ pytestmark = pytest.mark.gpu
 WARPS = 148 * 8 * 8  # of the default grid
 
 
-# (every batch has at least 8 WARPS / (fanout / 32) boxes, and an item or more each)
+# (every batch has at least 8 WARPS / (fanout / 32) boxes, an item or more each: twice that)
 @pytest.mark.parametrize("dims,rect,fanout,n,q,side", [
     (3, False, 256, 255, 10_000, 0.2), (2, False, 256, 60_001, 10_000, 0.1),  # one and two levels
     (3, False, 256, 150_001, 9_700, 0.01), (3, False, 256, 70_001, 12_000, 0.3), (3, False, 256, 70_001, 12_000, 0.15),
