@@ -467,46 +467,61 @@ __global__ void __launch_bounds__(kJoinThreads, (RECT ? 2 * D : D) > 8 ? 4 : ((R
   }
 }
 
-// Leaves that an item overlaps, about, from 32 items: the share of its node's
-// extent that the box covers and a leaf more, per dimension.
+// Leaves that an item overlaps and those that it covers partially, from one
+// 32-leaf group each of eight items, a warp of the CTA each (every CTA takes the
+// same ones, so all agree).  All threads call it.  With 32 groups the CTAs, which
+// all pay for it, took 4 us of a call in 3-D and 12 in 8-D; with eight, 1 to 2.
+struct Leaves {
+  float overlapped, partial;
+};
+constexpr uint32_t kSampled = 8;
 template <int D>
-__device__ __forceinline__ float leaves_per_item(const TreeView& t, const float* boxes, const uint2* items,
-                                                 uint32_t nitems) {
-  if (t.levels < 2) return 1.f;
-  const uint2 it = items[(uint64_t)(threadIdx.x & 31) * nitems / 32];
-  const float leaf = exp2f(-log2f((float)t.fanout) / D);
-  float part = (float)t.fanout;
-#pragma unroll 1
-  for (int d = 0; d < D; ++d) {
-    const float lo = __ldg(t.mbr[1] + d * t.pad[1] + it.y), hi = __ldg(t.mbr[1] + (D + d) * t.pad[1] + it.y);
-    const float* q = boxes + (uint64_t)it.x * 2 * D + d;
-    const float common = fminf(__ldg(q + D), hi) - fmaxf(__ldg(q), lo);
-    part *= fminf(1.f, (hi > lo ? common / (hi - lo) : 1.f) + leaf);
+__device__ __forceinline__ Leaves leaves_per_item(const TreeView& t, const float* boxes, const uint2* items,
+                                                  uint32_t nitems) {
+  __shared__ uint32_t s_leaves[2];
+  if (threadIdx.x < 2) s_leaves[threadIdx.x] = 0;
+  __syncthreads();
+  const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5, G = t.fanout >> 5;
+  const uint2 it = items[(uint64_t)w * nitems / kSampled];
+  const uint64_t c = (uint64_t)it.y * t.fanout + w % G * 32 + lane;
+  bool ov = false, in = false;
+  if (c < t.nodes[0]) test_node<D>(load_box<D>(boxes, it.x), t.mbr[0], t.pad[0], c, ov, in);
+  const uint32_t overlapped = __popc(__ballot_sync(0xffffffffu, ov));
+  const uint32_t partial = __popc(__ballot_sync(0xffffffffu, ov && !in));
+  if (lane == 0 && overlapped) {
+    atomicAdd(&s_leaves[0], overlapped);
+    atomicAdd(&s_leaves[1], partial);
   }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-  return part * (1.f / 32);
+  __syncthreads();
+  const float each = (float)G / kSampled;
+  return {s_leaves[0] * each, s_leaves[1] * each};
 }
 
 // How the warps of k_count and k_leafwrite share the items: their 32-leaf groups
-// in turn where those are fewer than four rounds of the grid's warps; above that
-// whole items where an item has few leaves (10,000 items of tiny boxes at fan-out
-// 256, nine rounds: the groups 66 us to count and 40 to write, whole items 44 and
-// 23; a plan of 4,096 tiny boxes 201 -> 164 us with four rounds instead of
-// eight), and groups again, each to the next free warp, where it has kManyLeaves
-// or more: whole items then leave most warps waiting for the last ones.  (By need
-// an atomic on one address per group is paid, about 1 ns each: with 10 leaves per
-// item 9,000 boxes over 2 M points take 187 us by items, 212 by need, with 22
-// 6,000 over 1 M 233 and 217.)
-constexpr float kManyLeaves = 24.f;
+// in turn where those are fewer than four rounds of the grid's warps, up to eight
+// where an item has many leaves that it covers; groups by need, each to the next
+// free warp, where it has many that it covers partially; whole items otherwise.
+//   few leaves: 10,000 items of tiny boxes at fan-out 256, nine rounds: the
+//   groups 66 us to count and 40 to write, whole items 44 and 23; a plan of 4,096
+//   tiny boxes, two rounds of items: 201 and 164 us;
+//   many covered ones: 1,500 8-D boxes of 75 leaves, five rounds: the groups 126
+//   us to count, whole items 150;
+//   many partially covered ones: whole items leave most warps waiting for the
+//   last ones.  By need an atomic on one address per group is paid, about 1 ns
+//   each: with 10 such leaves per item 9,000 boxes over 2 M points take 187 us by
+//   items, 212 by need, with 22 6,000 over 1 M 233 and 217.
 enum Share { kGroups, kItems, kGroupsByNeed };
+static_assert(kSampled == 256 / 32, "a warp per sampled group");
+constexpr float kManyPartial = 16.f, kManyLeaves = 16.f;
 template <int D>
 __device__ __forceinline__ Share share_items(const TreeView& t, const float* boxes, const uint2* items,
                                              uint32_t nitems, uint32_t G, uint32_t warps) {
   const uint64_t groups = (uint64_t)nitems * G;
   if (groups < 4ull * warps) return kGroups;
   if (groups >= 1u << 31) return kItems;  // (units are counted in 32 bits)
-  return leaves_per_item<D>(t, boxes, items, nitems) < kManyLeaves ? kItems : kGroupsByNeed;
+  const Leaves l = leaves_per_item<D>(t, boxes, items, nitems);
+  if (l.partial >= kManyPartial) return kGroupsByNeed;
+  return l.overlapped >= kManyLeaves && groups < 8ull * warps ? kGroups : kItems;
 }
 
 // Counts of batches that are not in node order: a warp per item or per 32-leaf
