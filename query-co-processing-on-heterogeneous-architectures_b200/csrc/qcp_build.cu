@@ -226,16 +226,14 @@ __device__ __forceinline__ void rs_sample(const uint64_t* keys, uint64_t n, uint
   if ((threadIdx.x & 31) == 0 && c) atomicAdd(&rs->shared, c);
 }
 
-// Counts of the digits of sweeps [p0, p0 + np).  The first samples / kSampleBlock
+// Counts of the digits of sweeps [p0, p0 + np).  The first sblocks
 // blocks of the first pass take the sample instead, beside it (a kernel of its
 // own: 6 to 11 us), so the pass is made whatever the sample says.
-constexpr uint32_t kSampleBlock = 4 * RS_THREADS;  // keys that a block samples
 __global__ void __launch_bounds__(RS_THREADS) k_rs_hist(const uint64_t* __restrict__ keys, uint64_t n, uint32_t p0,
-                                                        uint32_t np, uint32_t tight, uint32_t samples, RsScratch* rs,
-                                                        unsigned long long* slots) {
+                                                        uint32_t np, uint32_t tight, uint32_t samples,
+                                                        uint32_t sblocks, RsScratch* rs, unsigned long long* slots) {
   __shared__ uint32_t h[RS_MAX_PASSES][256];
   if (p0 >= RS_TOP && !rs_runs(rs, p0, tight)) return;
-  const uint32_t sblocks = samples / kSampleBlock;
   if (blockIdx.x < sblocks) {
     for (uint32_t t = blockIdx.x * RS_THREADS + threadIdx.x; t < samples; t += sblocks * RS_THREADS)
       rs_sample(keys, n, samples, t, rs, slots);
@@ -1044,9 +1042,11 @@ qcp_status radix_sort_pairs(uint64_t* keys, uint32_t* vals, uint64_t* keys_tmp, 
   uint32_t* vout = vals_tmp;
   // sweeps [p0, p0 + np)
   auto sweeps = [&](uint32_t p0, uint32_t np) {
-    const uint32_t m = p0 == 0 && key_bits > 32 ? rs_samples(n) : 0, sb = m / kSampleBlock;
+    // a key per thread where the histogram is short (four in turn took twice its
+    // 12 us on 1 M keys), four where the blocks are missed more (16 M)
+    const uint32_t m = p0 == 0 && key_bits > 32 ? rs_samples(n) : 0, sb = m > 16384 ? m / 1024 : m / RS_THREADS;
     k_rs_hist<<<sb + grid_for(n, RS_THREADS * 8, sms * 8 - sb), RS_THREADS, 0, s>>>(
-        kin, n, p0, np, tight, m, rs, reinterpret_cast<unsigned long long*>(slots));
+        kin, n, p0, np, tight, m, sb, rs, reinterpret_cast<unsigned long long*>(slots));
     note_launch();
     for (uint32_t p = p0; p < p0 + np; ++p) {
       k_rs_sweep<<<grid, RS_THREADS, 0, s>>>(kin, vin, kout, vout, n, ntiles, p, rs, status, tight, t_sort_polls,
