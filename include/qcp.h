@@ -265,7 +265,7 @@ qcp_status qcp_build_plan_free(qcp_build_plan* plan);
  * and d_counts (q entries) are device memory the caller owns, on the
  * index's device (or managed memory); device memory of another GPU is
  * refused with QCP_ERR_BAD_ARG.  The traversal's scratch is one fixed array
- * of about 20 MiB in the library's device image, held by every GPU that
+ * of 18 MiB in the library's device image, held by every GPU that
  * loads the library until exit and shared by all calls: calls that overlap
  * on the GPU race and must be serialised by the caller.  The first call on a
  * device looks up the array's device address and keeps it for the life of

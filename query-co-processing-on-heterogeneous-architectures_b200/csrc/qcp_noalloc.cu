@@ -11,7 +11,7 @@
 // the caller passes the query boxes and receives the counts in its own
 // device buffers.
 //
-// The fixed scratch costs kNoAllocScratchBytes (about 20 MiB) on every GPU
+// The fixed scratch costs kNoAllocScratchBytes (18 MiB) on every GPU
 // that loads the library, for as long as the process runs.  It is shared by
 // every call: calls that overlap on the GPU (several streams or host threads
 // at once) race on it and must be serialised by the caller.  The counters a
