@@ -694,6 +694,7 @@ __global__ void __launch_bounds__(256) k_leafwrite(TreeView t, const float* __re
                                                    const uint2* __restrict__ items,
                                                    const uint32_t* __restrict__ item_count, uint32_t* work,
                                                    const uint4* __restrict__ rec, const uint32_t* __restrict__ hmask,
+                                                   const unsigned long long* __restrict__ mask_words,
                                                    const unsigned long long* __restrict__ offsets,
                                                    unsigned long long* qcursor, int32_t* __restrict__ out,
                                                    uint64_t item_cap, uint32_t* qwhist, uint32_t hist_G,
@@ -716,7 +717,15 @@ __global__ void __launch_bounds__(256) k_leafwrite(TreeView t, const float* __re
   // one another; all by the atomic: 13 -> 18 us for 1,000 boxes over 1 M points)
   // (from eight items per warp on whole ones leave no warp waiting for long: 16 M
   // points, 10,000 boxes of 10^9 ids 1.1 ms, by need 1.2)
-  const bool whole = nitems >= 8 * warps || share_items<D>(t, boxes, items, nitems, G, warps) == kItems;
+  bool whole = nitems >= 8 * warps;
+  if (!whole) {
+    // the count pass asked for cpl * kChunkWords words per partially covered
+    // leaf: from eight rounds of groups on that decides, without the sample
+    if (hmask && (uint64_t)nitems * G >= 8ull * warps)
+      whole = (float)*mask_words < kManyPartial * nitems * (cpl * kChunkWords);
+    else
+      whole = share_items<D>(t, boxes, items, nitems, G, warps) == kItems;
+  }
   const uint32_t per = whole ? G : 1u;
   const uint32_t nfetch = whole ? nitems : nitems * G;
   for (uint32_t turn = 0;; ++turn) {
@@ -1091,7 +1100,7 @@ void launch_leafwrite(bool rect, uint32_t grid, cudaStream_t s, const TreeView& 
                       const uint64_t* offsets, uint64_t* qcursor, int32_t* out, uint64_t item_cap, uint32_t* qwhist,
                       uint32_t hist_G, uint32_t hist_bits) {
   auto* kern = rect ? k_leafwrite<D, true> : k_leafwrite<D, false>;
-  kern<<<grid, 256, 0, s>>>(t, boxes, items, item_count, work, hc.rec, hc.mask, (const unsigned long long*)offsets,
+  kern<<<grid, 256, 0, s>>>(t, boxes, items, item_count, work, hc.rec, hc.mask, hc.cursor, (const unsigned long long*)offsets,
                             (unsigned long long*)qcursor, out, item_cap, qwhist, hist_G, hist_bits);
 }
 
