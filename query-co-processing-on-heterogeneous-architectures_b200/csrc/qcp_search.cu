@@ -499,8 +499,9 @@ __device__ __forceinline__ Leaves leaves_per_item(const TreeView& t, const float
 
 // How the warps of k_count and k_leafwrite share the items: their 32-leaf groups
 // in turn where those are fewer than four rounds of the grid's warps, up to eight
-// where an item has many leaves that it covers; groups by need, each to the next
-// free warp, where it has many that it covers partially; whole items otherwise.
+// unless an item has few leaves; from eight rounds on groups by need, each to the
+// next free warp, where an item has many that it covers partially; whole items
+// otherwise.
 //   few leaves: 10,000 items of tiny boxes at fan-out 256, nine rounds: the
 //   groups 66 us to count and 40 to write, whole items 44 and 23; a plan of 4,096
 //   tiny boxes, two rounds of items: 201 and 164 us;
@@ -512,7 +513,7 @@ __device__ __forceinline__ Leaves leaves_per_item(const TreeView& t, const float
 //   items, 212 by need, with 22 6,000 over 1 M 233 and 217.
 enum Share { kGroups, kItems, kGroupsByNeed };
 static_assert(kSampled == 256 / 32, "a warp per sampled group");
-constexpr float kManyPartial = 16.f, kManyLeaves = 16.f;
+constexpr float kManyPartial = 16.f, kFewLeaves = 8.f;
 template <int D>
 __device__ __forceinline__ Share share_items(const TreeView& t, const float* boxes, const uint2* items,
                                              uint32_t nitems, uint32_t G, uint32_t warps) {
@@ -522,8 +523,8 @@ __device__ __forceinline__ Share share_items(const TreeView& t, const float* box
   if (groups < (D > 4 ? 8ull : 4ull) * warps) return kGroups;
   if (groups >= 1u << 31) return kItems;  // (units are counted in 32 bits)
   const Leaves l = leaves_per_item<D>(t, boxes, items, nitems);
-  if (l.partial >= kManyPartial) return kGroupsByNeed;
-  return l.overlapped >= kManyLeaves && groups < 8ull * warps ? kGroups : kItems;
+  if (groups < 8ull * warps) return l.overlapped < kFewLeaves ? kItems : kGroups;
+  return l.partial >= kManyPartial ? kGroupsByNeed : kItems;
 }
 
 // Counts of batches that are not in node order: a warp per item or per 32-leaf
@@ -695,6 +696,7 @@ __global__ void __launch_bounds__(256) k_leafwrite(TreeView t, const float* __re
                                                    const uint32_t* __restrict__ item_count, uint32_t* work,
                                                    const uint4* __restrict__ rec, const uint32_t* __restrict__ hmask,
                                                    const unsigned long long* __restrict__ mask_words,
+                                                   const unsigned long long* __restrict__ total_ids,
                                                    const unsigned long long* __restrict__ offsets,
                                                    unsigned long long* qcursor, int32_t* __restrict__ out,
                                                    uint64_t item_cap, uint32_t* qwhist, uint32_t hist_G,
@@ -719,12 +721,19 @@ __global__ void __launch_bounds__(256) k_leafwrite(TreeView t, const float* __re
   // points, 10,000 boxes of 10^9 ids 1.1 ms, by need 1.2)
   bool whole = nitems >= 8 * warps;
   if (!whole) {
-    // the count pass asked for cpl * kChunkWords words per partially covered
-    // leaf: from eight rounds of groups on that decides, without the sample
-    if (hmask && (uint64_t)nitems * G >= 8ull * warps)
-      whole = (float)*mask_words < kManyPartial * nitems * (cpl * kChunkWords);
-    else
+    // the rule of share_items, without its sample where the count pass has
+    // recorded hit bits: it asked for cpl * kChunkWords words per partially
+    // covered leaf, and the ids make up F per covered one at least (the sample
+    // comes out differently from call to call: 1.1 M points, 3,000 boxes, 19
+    // partially covered leaves per item, 115 us one time and 170 the next)
+    const uint64_t groups = (uint64_t)nitems * G;
+    if (!hmask || groups < 4ull * warps) {
       whole = share_items<D>(t, boxes, items, nitems, G, warps) == kItems;
+    } else {
+      const float partial = (float)*mask_words / (float)(cpl * kChunkWords);
+      whole = groups < 8ull * warps ? D <= 4 && partial + (float)*total_ids / (float)F < kFewLeaves * nitems
+                                    : partial < kManyPartial * nitems;
+    }
   }
   const uint32_t per = whole ? G : 1u;
   const uint32_t nfetch = whole ? nitems : nitems * G;
@@ -1097,10 +1106,11 @@ qcp_status launch_count(bool rect, uint64_t nodes, uint32_t blocks_per_sm, cudaS
 template <int D>
 void launch_leafwrite(bool rect, uint32_t grid, cudaStream_t s, const TreeView& t, const float* boxes,
                       const uint2* items, const uint32_t* item_count, uint32_t* work, const HitCache& hc,
-                      const uint64_t* offsets, uint64_t* qcursor, int32_t* out, uint64_t item_cap, uint32_t* qwhist,
+                      const uint32_t* total_ids, const uint64_t* offsets, uint64_t* qcursor, int32_t* out, uint64_t item_cap, uint32_t* qwhist,
                       uint32_t hist_G, uint32_t hist_bits) {
   auto* kern = rect ? k_leafwrite<D, true> : k_leafwrite<D, false>;
-  kern<<<grid, 256, 0, s>>>(t, boxes, items, item_count, work, hc.rec, hc.mask, hc.cursor, (const unsigned long long*)offsets,
+  kern<<<grid, 256, 0, s>>>(t, boxes, items, item_count, work, hc.rec, hc.mask, hc.cursor,
+                            (const unsigned long long*)total_ids, (const unsigned long long*)offsets,
                             (unsigned long long*)qcursor, out, item_cap, qwhist, hist_G, hist_bits);
 }
 
@@ -1208,7 +1218,7 @@ static qcp_status write_items(qcp_index* ix, Workspace* ws, int cur, cudaStream_
   uint32_t* ctr = ws->ctr;
   QCP_DISPATCH_D(ix->dims, launch_leafwrite<DD>(ix->is_rect != 0, grid, s, t, ws->qboxes, ws->items[cur],
                                                 ctr + kCtrFrontier0 + cur, ctr + kCtrWrite, hit_cache_of(ws),
-                                                ws->offsets, ws->qcursor, ws->out_ids, ws->items_cap,
+                                                ctr + kCtrTotal, ws->offsets, ws->qcursor, ws->out_ids, ws->items_cap,
                                                 ws->hist_G ? ws->qwhist : nullptr, ws->hist_G, ws->hist_bits));
   note_launch();
   return check_launch("k_leafwrite");
