@@ -534,8 +534,9 @@ __device__ __forceinline__ Share share_items(const TreeView& t, const float* box
 // of its dependent reads (item, box and MBRs, objects); more CTAs per SM hide it
 // until the registers of a box, its MBRs and four objects spill too much
 // (61,000 8-D points, 7,768 boxes: 110 -> 45 us with three instead of four;
-// MBRs read one group ahead only up to two dimensions: 4 M 4-D rectangles 665 ->
-// 626 us; 3-D points still spill 72 bytes, three CTAs were slower).  1,000 boxes
+// MBRs read one group ahead in one dimension only: 4 M 4-D rectangles 665 -> 626
+// us without, 100,000 2-D points, 15,000 boxes 120 -> 111; 3-D points still spill
+// 60 bytes, three CTAs were slower).  1,000 boxes
 // over 1 M points: 18.9 (a warp per item) -> 12.4 us; 64 boxes over 16 M points
 // 36.7 -> 14.8 us; 3,000 boxes with 34 leaves per item over 4 M 4-D rectangles
 // at fan-out 256, by whole items in turn 900, by need 626.
@@ -590,8 +591,8 @@ __global__ void __launch_bounds__(256, (RECT ? 2 * D : D) > 8 ? 2 : (RECT ? 2 * 
     }
     uint32_t total = 0;  // hits of the unit
     const uint32_t ga = whole ? 0u : u % G, gb = whole ? G : ga + 1;
-    float mlo[D], mhi[D];  // a group's MBRs, with few dimensions loaded one group ahead
-    constexpr bool kMbrAhead = D <= 2;
+    float mlo[D], mhi[D];  // a group's MBRs, in one dimension loaded one group ahead
+    constexpr bool kMbrAhead = D == 1;
     auto load_mbrs = [&](uint32_t g) {
       const uint64_t at = (uint64_t)it.y * F + g * 32 + lane;
 #pragma unroll
