@@ -329,9 +329,17 @@ __global__ void __launch_bounds__(kTinyWarps * 32, kTinyBlocks) k_sort_tiny(cons
   }
 }
 
+// Programmatic dependent launch: the next kernel of the stream may start once
+// every CTA of this one has said so or ended; and the wait for everything
+// before it.
+__device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_for_prerequisites() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // Windows of at most kWinWarpMax ids (listed by k_win_split), one warp
 // each: the window's ids at src + wbase[g] in ascending order to
-// dst + wbase[g].
+// dst + wbase[g].  It may run beside k_win_sort, launched before it, once that
+// one's CTAs are all on the SMs; what it reads is complete before k_win_sort
+// starts, and it ends after k_win_sort, so what follows waits for both.
 __global__ void __launch_bounds__(kTinyWarps * 32, kWinWarpBlocks) k_win_sort_warp(const uint32_t* __restrict__ list,
                                                                    const uint32_t* __restrict__ nlist_p, uint32_t G,
                                                                    uint32_t wbits, const uint32_t* __restrict__ whist,
@@ -354,6 +362,7 @@ __global__ void __launch_bounds__(kTinyWarps * 32, kWinWarpBlocks) k_win_sort_wa
     warp_bucket_sort<kWinWarpMax>(src + off, dst + off, whist[g], lo, bshift, sm.stage[wp], sm.cnt[wp], sm.base[wp],
                                   lane);
   }
+  wait_for_prerequisites();
 }
 
 // The (job, window) pairs into two lists: windows of 1..kWinWarpMax ids for
@@ -825,6 +834,7 @@ __global__ void __launch_bounds__(WinCfg<BITS>::kThreads, WinCfg<BITS>::kBlocks)
   constexpr uint32_t kBmWords = C::kWords;
   constexpr uint32_t kStage = C::kStage;
   constexpr uint32_t kPrefetch = C::kPrefetch;
+  launch_dependents();  // k_win_sort_warp, when all of these CTAs are here
   const uint32_t total = *nlist_p;  // listed (job, window) pairs
   extern __shared__ __align__(16) unsigned char smem_raw[];
   RankSmem<BITS>& s = *reinterpret_cast<RankSmem<BITS>*>(smem_raw);
@@ -1084,8 +1094,12 @@ static void launch_win_sort_t(uint64_t max_pairs, uint32_t sms, const uint32_t* 
 
 // The windows of a call: k_win_split lists them (counts in ctr[kCtrWinBig],
 // ctr[kCtrWinSmall], zeroed by the caller), the bitmap sort takes the large
-// ones and one warp each the small ones, on the second branch (ws->side).  lists holds 2 * max_pairs entries;
-// max_pairs bounds the (job, window) pairs.
+// ones and one warp each the small ones, beside it as soon as all of its CTAs are
+// on the SMs (but not in a call that reports phase times).  On two streams
+// either could come first, and where the small ones' did, CTAs of the bitmap
+// sort waited for them with their full share of windows (10,000 boxes over 16 M
+// points 7.65 ms one time and 9.6 the next; one after the other 7.75).  lists
+// holds 2 * max_pairs entries; max_pairs bounds the (job, window) pairs.
 static qcp_status launch_win_sort(Workspace* ws, uint64_t max_pairs, uint32_t sms, const uint32_t* njobs, uint32_t G,
                                   uint32_t wbits, const uint32_t* whist, const unsigned long long* wbase, uint32_t* lists,
                                   uint32_t* ctr, const int32_t* src, int32_t* out, uint32_t* err, cudaStream_t s,
@@ -1096,19 +1110,24 @@ static qcp_status launch_win_sort(Workspace* ws, uint64_t max_pairs, uint32_t sm
   k_win_split<<<(uint32_t)(split_blocks < (uint64_t)sms * 8 ? split_blocks : (uint64_t)sms * 8), 256, 0, s>>>(
       njobs, G, whist, big, ctr + kCtrWinBig, small, ctr + kCtrWinSmall,
       stats && ws->timing ? ws->d_stats + kStatBitmapIds : nullptr);
-  cudaStream_t warp_s = s;
-  if (!ws->timing) {
-    warp_s = ws->side;
-    QCP_CUDA(ws_branch(ws, 3, s, warp_s));
-  }
   if (wbits >= 18) launch_win_sort_t<18>(max_pairs, sms, big, ctr + kCtrWinBig, G, wbits, whist, wbase, src, out, err, s);
   else if (wbits == 17) launch_win_sort_t<17>(max_pairs, sms, big, ctr + kCtrWinBig, G, wbits, whist, wbase, src, out, err, s);
   else launch_win_sort_t<16>(max_pairs, sms, big, ctr + kCtrWinBig, G, wbits, whist, wbase, src, out, err, s);
   if (stats) mark(ws, kEvSortBitmap, s);
   const uint64_t warp_blocks = (max_pairs + kTinyWarps - 1) / kTinyWarps;
   const uint64_t warp_cap = (uint64_t)sms * kWinWarpBlocks;
-  k_win_sort_warp<<<(uint32_t)(warp_blocks < warp_cap ? warp_blocks : warp_cap), kTinyWarps * 32,
-                    sizeof(TinySmem<kWinWarpMax>), warp_s>>>(small, ctr + kCtrWinSmall, G, wbits, whist, wbase, src, out);
+  cudaLaunchAttribute beside{};
+  beside.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  beside.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((uint32_t)(warp_blocks < warp_cap ? warp_blocks : warp_cap));
+  cfg.blockDim = dim3(kTinyWarps * 32);
+  cfg.dynamicSmemBytes = sizeof(TinySmem<kWinWarpMax>);
+  cfg.stream = s;
+  cfg.attrs = &beside;
+  cfg.numAttrs = ws->timing || max_pairs == 0 ? 0 : 1;  // (no pairs: the kernel before it is not k_win_sort)
+  QCP_CUDA(cudaLaunchKernelEx(&cfg, k_win_sort_warp, (const uint32_t*)small, (const uint32_t*)(ctr + kCtrWinSmall), G,
+                              wbits, whist, wbase, src, out));
   return QCP_OK;
 }
 
@@ -1217,8 +1236,8 @@ qcp_status segmented_sort(qcp_index* ix, Workspace* ws, cudaStream_t s) {
   // call that reports phase times); each leaves much of the chip idle in a
   // batch of some hundred boxes (1,000 over 2 M points 314 -> 261 us) and its
   // tail in large ones (10,000 over 16 M points 8,024 -> 7,954)
-  if (!ws->timing && (nbig || (ntiny && nsmall))) QCP_TRY(ws_reserve_side(ws));
   const bool fork = !ws->timing && (nbig ? ntiny + nsmall : (ntiny && nsmall));
+  if (fork) QCP_TRY(ws_reserve_side(ws));
   cudaStream_t tiny_s = fork ? ws->side : s, small_s = fork && nbig ? ws->side : s;
   if (fork) QCP_CUDA(ws_branch(ws, 2, s, ws->side));
   if (ntiny) {
@@ -1244,7 +1263,7 @@ qcp_status segmented_sort(qcp_index* ix, Workspace* ws, cudaStream_t s) {
   QCP_TRY(ws_reserve_sort(ix, ws, 0, ntiles));
   QCP_TRY(ws_reserve_tables(ws, SortTables(nullptr, nbig, G).bytes));
   QCP_TRY(sort_windows(ix, ws, nbig, ntiles, SortTables(ws->tables, nbig, G), G, wbits, s, true));
-  if (!ws->timing) QCP_CUDA(ws_branch(ws, 4, ws->side, s));
+  if (fork) QCP_CUDA(ws_branch(ws, 4, ws->side, s));
   return QCP_OK;
 }
 
@@ -1275,11 +1294,12 @@ size_t sort_tables_bytes(const qcp_index* ix, const Workspace* ws, uint32_t q) {
 
 // segmented_sort without host readbacks, for at most max_ids ids: job and tile
 // counts stay on the device, every launch has a fixed grid and the kernels
-// read the counts.  The slices and windows that single CTAs and warps sort run
-// on ws->side beside the window partition and the bitmap sort: each of the
-// kernels leaves most of the chip idle on a plan's small batch (a run of 64
-// boxes on 16 M points, 62 us of it sort kernels: 194 -> 153 us with this
-// branch and the tiles numbered by k_classify instead of a scan).
+// read the counts.  The slices that single CTAs and warps sort run on ws->side
+// beside the window partition and the bitmap sort: each of the kernels leaves
+// most of the chip idle on a plan's small batch (a run of 64 boxes on 16 M
+// points, 62 us of it sort kernels: 194 -> 153 us with this branch and the tiles
+// numbered by k_classify instead of a scan; 143 with the small windows behind
+// the bitmap sort's start instead of on the branch).
 // Tables (sort_tables_bytes) and the tile map (at least
 // max_ids / kSortTile + q entries, ws->seg_hist) are the caller's.
 // Stream-capturable.
